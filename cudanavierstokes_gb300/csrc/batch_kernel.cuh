@@ -359,37 +359,45 @@ __global__ void __launch_bounds__(BATCH_THREADS, sizeof(R) == 4 ? 7 : 4)
         if (t < ghost_count(I.g)) {
             const RhsIn<R>& in = I.in[cur];
             const StencilFields<R> f{(R*)in.r, (R*)in.u, (R*)in.v, (R*)in.w, (R*)in.t, (R*)in.p, (R*)in.h,
-                                     (R*)in.m, (float4*)in.qa, (float4*)in.qb};
+                                     (R*)in.m, (float4*)in.qa, (float4*)in.qb, in.fx.gmax, in.fx.gnext};
             ghost_state_cell<R>(I.g, I.ph, f, I.scal, (int)t);
         }
     });
     grid_barrier(bar, nb, err);
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt[0] = 0ULL;
-    // phase 2: dilatation from the packed records (FP32-RHS: the RHS forms the nine gradients
-    // itself) or the nine velocity gradients and the dilatation
+    // phase 2: dilatation from the packed records (FP32-RHS) or the conversion to fixed-point
+    // stencil inputs, the dilatation and (an instance's first unit) the scale factors (FP64)
     sweep(cnt + 1, ctl->unit_off, npu, [&](long long u, int q) {
         const BatchInst<R>& I = tab[q];
         int i, j, k;
         unit_point(I, u - ctl->unit_off[q], tx, ty, i, j, k);
-        if (i < I.g.mx && j < I.g.my) {
-            const RhsIn<R>& in = I.in[cur];
-            if constexpr (sizeof(R) == 4) {
-                dil_point_packed<V>(I.g, I.cf, in.qa, (float*)in.dil, i, j, k);
-            } else {
-                GradOut<R> go;
-                for (int c = 0; c < 9; c++) go.g[c] = (R*)in.g[c];
-                go.dil = (R*)in.dil;
-                grad_point<R, V>(I.g, I.cf, in.u, in.v, in.w, go, i, j, k);
-            }
+        const RhsIn<R>& in = I.in[cur];
+        if constexpr (sizeof(R) == 4) {
+            if (i < I.g.mx && j < I.g.my) dil_point_packed<V>(I.g, I.cf, in.qa, (float*)in.dil, i, j, k);
+        } else {
+            int e[8];
+            fx_exponents(in.fx.gmax, e);
+            if (u == ctl->unit_off[q] && threadIdx.x < FXK_COUNT)
+                in.fx.k[threadIdx.x] =
+                    fx_table(I.cf.fx, in.fx.gmax, I.g.nonuniform_x, I.cf.lam_mu, (int)threadIdx.x);
+            if (i < I.g.mx && j < I.g.my) fx_point<V>(I.g, I.cf.fx, in, e, I.cf.xp, i, j, k);
         }
     });
     grid_barrier(bar, nb, err);
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt[1] = 0ULL;
-    // phase 3: dilatation ghosts
+    // phase 3: dilatation ghosts (FP64: and the conversion of the ghost cells)
     sweep(cnt + 2, ctl->ghost_off, ngu, [&](long long u, int q) {
         const BatchInst<R>& I = tab[q];
         const long long t = (u - ctl->ghost_off[q]) * BATCH_THREADS + threadIdx.x;
-        if (t < ghost_count(I.g)) ghost_scalar_cell<R>(I.g, (R*)I.in[cur].dil, (int)t);
+        if (t >= ghost_count(I.g)) return;
+        if constexpr (sizeof(R) == 4) {
+            ghost_scalar_cell<R>(I.g, (R*)I.in[cur].dil, (int)t);
+        } else {
+            int e[8];
+            fx_exponents(I.in[cur].fx.gmax, e);
+            ghost_scalar_cell<i64>(I.g, I.in[cur].fx.th, (int)t);
+            fx_ghost(I.g, I.in[cur], e, (int)t);
+        }
     });
     grid_barrier(bar, nb, err);
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt[2] = 0ULL;

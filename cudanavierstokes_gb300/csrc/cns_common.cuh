@@ -58,8 +58,26 @@ struct Phys {
 //   c2V[d][k]: second derivative at order 2V (uniform), D2 f = c2V[0] f_0 + sum_k c2V[k](f_{+k}+f_{-k})
 // from the central tables of src/globals.h:69-95 (c1[k] = -coeffF[K-k], c2[k] = coeffS[K-k]).
 // xp / cvsx are the non-uniform x metric tables in type R.
+//
+// FxBase, FP64 mode: the grid's part of the fixed-point scale factors (fx.cuh). Per direction
+// d: the inverse spacing over the common denominator of the first-derivative weights, times
+// their scaling (b1V at the viscous order, b1S at the advective one), and the second
+// derivative's; on a stretched x the latter is the scale of the integer metrics xx, and the
+// first derivatives carry that of xpk.
+struct FxBase {
+    double b1V[3], b1S[3], b2[3], b1V3[3];   // b1V3 = b1V / 3
+    double th[3], thmax;                     // b1V without the metric; th[0] at the largest 1/x'
+    const longlong2* xx;    // [mx] factors of f'' and f' (index derivatives) in the second derivative
+    const long long* xpk;   // [mx] 1/x' as a factor (low word, balanced high half), the largest 2^63 (1 - 2^-20)
+};
 template <typename R>
-struct CoefT {
+struct CoefFx {};
+template <>
+struct CoefFx<double> {
+    FxBase fx;
+};
+template <typename R>
+struct CoefT : CoefFx<R> {
     R c1S[3][5];
     R c1V[3][5];
     R c2V[3][5];

@@ -26,6 +26,7 @@ struct StateOut {
 // neighbour costs two vector loads (and one address each) instead of eight scalar loads.
 template <typename R>
 struct DerivedOut {
+    unsigned* gmax;     // FP64 mode: the fields' maxima (fx_track, fx.cuh)
     R *h, *t, *p, *m;   // FP64 mode
     R *r, *u, *v, *w;   // pair mode: the state's rho, u, v, w as pairs
     float4 *qa, *qb;    // FP32-RHS mode
@@ -36,6 +37,23 @@ template <typename R>
 struct StencilFields {
     R *r, *u, *v, *w, *t, *p, *h, *m;   // FP64 mode
     float4 *qa, *qb;                    // FP32-RHS mode (packed, see DerivedOut)
+    unsigned *gmax, *gnext;             // FP64 mode: maxima of these fields; of the next state
+};
+
+// per stage: the integer factors of the sums, 16 per direction (velocity gradients, grad mu,
+// grad T, grad theta / 3, grad p, second derivatives of u, v, w, T, mass flux, fluxes of u, v,
+// w, H); of the centre terms; units as doubles (fx_table)
+enum { FXK_U = 0, FXK_MU = 3, FXK_T = 4, FXK_TH = 5, FXK_P = 6, FXK_L = 7, FXK_LT = 10, FXK_F0 = 11, FXK_F = 12,
+       FXK_DIR = 16, FXK_CTR = 48, FXK_A = 52, FXK_UL = 57, FXK_UD = 61, FXK_UC = 62, FXK_UE = 63, FXK_TG = 64,
+       FXK_COUNT = 65 };
+
+// FP64 mode: the ghosted stencil inputs as pairs of 64-bit fixed-point values, (rho, u),
+// (v, w), (T, p), (H, mu), theta, and the stage's scale factors
+struct FxFields {
+    longlong2* f[4];
+    long long* th;
+    long long* k;
+    unsigned *gmax, *gnext;   // maxima of this state's fields; of the next state's
 };
 
 template <typename R>
@@ -51,6 +69,7 @@ struct RhsIn {
     const R *r, *u, *v, *w, *t, *p, *h, *m, *dil;
     const R* g[9];
     const float4 *qa, *qb;
+    FxFields fx;   // FP64 mode
 };
 
 // time-scheme stage kinds
@@ -118,6 +137,9 @@ int check_reduce_args(const char* who, int mx, int my, int mz, const void* const
 // the RHS + stage kernel over the interior; returns the number of launches (band groups)
 int launch_rhs_fp64(int S, int V, const Geom& g, const Phys& ph, const CoefT<double>& cf, const RhsIn<double>& in,
                     const Update<double>& up, double* scal, int quirk, cudaStream_t s);
+// FP64 mode: the stencil inputs as fixed-point values, theta (with its ghost images with
+// own) and the stage's scale factors
+void launch_fx(int V, const Geom& g, const CoefT<double>& cf, const RhsIn<double>& in, int own, cudaStream_t s);
 int launch_rhs_fp32(int S, int V, const Geom& g, const Phys& ph, const CoefT<float>& cf, const RhsIn<float>& in,
                     const Update<float>& up, double* scal, int quirk, cudaStream_t s);
 int launch_rhs_pair(int S, int V, const Geom& g, const Phys& ph, const CoefT<ff>& cf, const RhsIn<ff>& in,

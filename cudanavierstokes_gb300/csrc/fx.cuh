@@ -1,0 +1,135 @@
+// fx.cuh -- 64-bit fixed-point arithmetic of the FP64 mode's stencil sums.
+//
+// On this GPU an FP64 instruction issues to 2 lanes per SM per cycle, a 32 x 32 + 64-bit
+// integer multiply-add to 64 and a 32-bit addition to ~104 (measured), so a stencil sum of
+// FP64 values is ~20 times cheaper on the integer units. A field f with |f| < 2^e over the
+// whole grid, ghosts included, is held as F = f 2^(62 - e), truncated: exact wherever |f| >=
+// 2^(e - 10) (an FP64 value has 53 bits, the format 62), elsewhere within 2^(e - 62), 2^-9 of
+// the rounding of the field's large values. Sums and differences of fields are exact; the
+// central-difference weights are rationals with a common denominator, so a weighted
+// difference is exact up to one truncation at 2^-62 of its range. The field's exponent e
+// comes from its maximum, which the kernels that write the field track (fx_track).
+//
+// Ranges. |F| < 2^62 (1 - 2^-21) (fx_exponent), so the sum or difference of two fields fits
+// 63 bits and its balanced high half (below) 31 bits; every 64-bit accumulator's bound is
+// noted where it is formed.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace cns {
+
+typedef long long i64;
+
+// ---- a value as h 2^32 + l with both halves signed: l the low word, h the high word plus
+// the low word's sign ----
+__device__ __forceinline__ int fx_lo(i64 v) { return (int)(unsigned)v; }
+__device__ __forceinline__ int fx_word1(i64 v) { return (int)(v >> 32); }
+__device__ __forceinline__ int fx_hi(i64 v) { return fx_word1(v) + (int)((unsigned)v >> 31); }
+
+// a b + c: the carry pair below assembles to one 32 x 32 + 64-bit multiply-add. (mad.wide
+// becomes a multiplication and a 64-bit addition, three instructions; from a 64-bit C
+// expression the compiler splits constant factors into shifts.)
+__device__ __forceinline__ i64 fx_mad(int a, int b, i64 c) {
+    i64 r;
+    asm("{\n\t.reg .s32 l, h;\n\tmov.b64 {l, h}, %3;\n\tmad.lo.cc.s32 l, %1, %2, l;\n\t"
+        "madc.hi.s32 h, %1, %2, h;\n\tmov.b64 %0, {l, h};\n\t}"
+        : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+}
+
+constexpr i64 FX_HALF = 0x80000000LL;   // rounds the division by 2^32
+
+// a b / 2^64, |a|, |b| < 2^63 (1 - 2^-21): the product of the high halves plus the two cross
+// products, rounded; the product of the low halves (below a quarter of the last bit) is left
+// out. Within 0.75 of the last bit, unbiased (truncation would add up over a stencil's sums). The cross sum stays below 2^63 (1 - 2^-21) + 2^32.
+__device__ __forceinline__ i64 fx_mul(i64 a, i64 b) {
+    const int ah = fx_hi(a), al = fx_lo(a), bh = fx_hi(b), bl = fx_lo(b);
+    const i64 m = fx_mad(ah, bl, fx_mad(al, bh, FX_HALF));
+    return fx_mad(ah, bh, (i64)fx_word1(m));
+}
+
+// sum of products a_k w_k / 2^32 with small-integer weights: two accumulators, the high
+// halves' and the low halves'. With |a| < 2^63 and sum |w| <= 2^30.8 both stay below 2^61.8.
+struct FxSum {
+    i64 h, l;
+    __device__ __forceinline__ FxSum() : h(0), l(0) {}
+    __device__ __forceinline__ void add(i64 a, int w) {
+        h = fx_mad(fx_hi(a), w, h);
+        l = fx_mad(fx_lo(a), w, l);
+    }
+    __device__ __forceinline__ i64 value() const { return h + (i64)fx_word1(l + FX_HALF); }
+    __device__ __forceinline__ i64 twice() const { return (h << 1) + ((l + FX_HALF / 2) >> 31); }
+};
+
+// ---- central-difference weights as integers: c1[k] = fxw1(K, k) / fxn1(K) etc., scaled by
+// 2^s so that the sum of the magnitudes (both sides of a first derivative; one side and half
+// the centre weight of a second one) stays below 2^30.8 ----
+__host__ __device__ constexpr int fxs1(int K) { return K == 1 ? 30 : K == 2 ? 27 : K == 3 ? 25 : 21; }
+__host__ __device__ constexpr int fxn1(int K) { return K == 1 ? 2 : K == 2 ? 12 : K == 3 ? 60 : 840; }
+__host__ __device__ constexpr int fxw1(int K, int k) {
+    return (K == 1 ? 1
+            : K == 2 ? (k == 1 ? 8 : -1)
+            : K == 3 ? (k == 1 ? 45 : k == 2 ? -9 : 1)
+                     : (k == 1 ? 672 : k == 2 ? -168 : k == 3 ? 32 : -3)) * (1 << fxs1(K));
+}
+__host__ __device__ constexpr int fxs2(int K) { return K == 1 ? 29 : K == 2 ? 25 : K == 3 ? 21 : 16; }
+__host__ __device__ constexpr int fxn2(int K) { return K == 1 ? 1 : K == 2 ? 12 : K == 3 ? 180 : 5040; }
+__host__ __device__ constexpr int fxw2(int K, int k) {
+    return (K == 1 ? (k == 0 ? -2 : 1)
+            : K == 2 ? (k == 0 ? -30 : k == 1 ? 16 : -1)
+            : K == 3 ? (k == 0 ? -490 : k == 1 ? 270 : k == 2 ? -27 : 2)
+                     : (k == 0 ? -14350 : k == 1 ? 8064 : k == 2 ? -1008 : k == 3 ? 128 : -9)) * (1 << fxs2(K));
+}
+
+// ---- exponents ----
+// e with |f| < 2^e (1 - 2^-21) from the largest high word (sign cleared) of a field's
+// values. Magnitudes below 2^-300 count as 2^-300; above 2^300, infinities and NaN make the
+// state invalid (fx_valid), as they make the FP64 arithmetic overflow.
+constexpr int FX_EMAX = 300;
+__device__ __forceinline__ int fx_exponent(unsigned hw) {
+    const int e = (int)(hw >> 20) - 1022 + ((hw & 0xfffffu) == 0xfffffu ? 1 : 0);
+    return e < -FX_EMAX ? -FX_EMAX : e;
+}
+__device__ __forceinline__ bool fx_valid(int e) { return e <= FX_EMAX; }
+
+// x 2^(62 - e), |x| < 2^e, truncated towards zero, on the integer units
+__device__ __forceinline__ i64 fx_from(double x, int e) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int ex = (int)((hi >> 20) & 0x7ffu);
+    // the significand with its leading bit at 2^61, then right by e - (ex - 1022) >= 0
+    const unsigned mh = (__funnelshift_l(lo, hi, 9) & 0x1fffffffu) | 0x20000000u;
+    const unsigned ml = lo << 9;
+    i64 m;
+    asm("shr.u64 %0, %1, %2;" : "=l"(m) : "l"(((i64)mh << 32) | (i64)ml), "r"(e - (ex - 1022)));   // 0 beyond 63
+    const i64 s = (i64)((int)hi >> 31);
+    return (m ^ s) - s;
+}
+
+// 2^a, a clamped to the range of normal numbers
+__device__ __forceinline__ double fx_pow2(int a) {
+    return __hiloint2double((min(max(a, -1022), 1023) + 1023) << 20, 0);
+}
+
+// ---- maxima: slots of the eight fields (rho, u, v, w, T, p, H, mu), the largest high words
+// seen. Reads first: a warp issues atomics only while it raises a slot. ----
+__device__ __forceinline__ void fx_track(unsigned* slots, const double (&f)[8]) {
+    const unsigned mask = __activemask();
+    const uint4 a = __ldcg((const uint4*)slots), b = __ldcg((const uint4*)slots + 1);
+    const unsigned cur[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    unsigned h[8];
+    bool up = false;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        h[q] = (unsigned)__double2hiint(f[q]) & 0x7fffffffu;
+        up |= h[q] > cur[q];
+    }
+    if (!__any_sync(mask, up)) return;
+    const bool first = (threadIdx.y * blockDim.x + threadIdx.x) % 32 == __ffs(mask) - 1;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const unsigned m = __reduce_max_sync(mask, h[q]);
+        if (first && m > cur[q]) atomicMax(slots + q, m);
+    }
+}
+
+}  // namespace cns

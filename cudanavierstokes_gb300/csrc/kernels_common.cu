@@ -2,6 +2,7 @@
 // layout conversion. The RHS/stage kernel lives in kernels_rhs.cuh.
 #include "cns_common.cuh"
 #include "cns_internal.h"
+#include "kernels_fx.cuh"
 #include "kernels_point.cuh"
 
 namespace cns {
@@ -50,6 +51,31 @@ __global__ void __launch_bounds__(DIL_TX * DIL_TY) k_dil_march(Geom g, CoefT<flo
     const int k0 = blockIdx.z * DIL_NZ;
     dil_column_packed<V, DIL_TY>(g, cf, qa, dil, blockIdx.x * DIL_TX, blockIdx.y * DIL_TY, k0,
                                  min(k0 + DIL_NZ, g.mz), own != 0, (int)threadIdx.x, (int)threadIdx.y, su, sv);
+}
+
+// FP64 mode: fixed-point conversion and theta. Blocks of 32 x 8 threads: the first `tiles`
+// march nz planes of a 32 x 8 tile each (fx_column), the others convert 256 ghost cells each;
+// the first block also writes the stage's scale factors.
+template <int V>
+__global__ void __launch_bounds__(DIL_TX * DIL_TY, 4) k_fx(Geom g, const __grid_constant__ FxBase b,
+                                                           const __grid_constant__ RhsIn<double> in,
+                                                           const double* __restrict__ xp, double lam_mu, int own,
+                                                           int tiles, int nbx, int nby, int nz) {
+    __shared__ i64 su[DIL_TY][DIL_TX + 2 * V];   // u of the tile rows, x halo V on each side
+    __shared__ i64 sv[DIL_TY + 2 * V][DIL_TX];   // v of the tile columns, y halo V on each side
+    const int tid = threadIdx.y * DIL_TX + threadIdx.x;
+    int e[8];
+    fx_exponents(in.fx.gmax, e);   // out of range: the factors are NaN
+    int t = (int)blockIdx.x;
+    if (t == 0 && tid < FXK_COUNT) in.fx.k[tid] = fx_table(b, in.fx.gmax, g.nonuniform_x, lam_mu, tid);
+    if (t >= tiles) {
+        t = (t - tiles) * DIL_TX * DIL_TY + tid;
+        if (t < ghost_count(g)) fx_ghost(g, in, e, t);
+        return;
+    }
+    const int r = t / nbx, bz = r / nby, k0 = bz * nz;
+    fx_column<V, DIL_TY>(g, b, in, e, xp, (t - r * nbx) * DIL_TX, (r - bz * nby) * DIL_TY, k0, min(k0 + nz, g.mz),
+                         own != 0, (int)threadIdx.x, (int)threadIdx.y, su, sv);
 }
 
 template <typename R>
@@ -238,6 +264,22 @@ void launch_dil_packed(int V, const Geom& g, const CoefT<float>& cf, const float
     default: k_dil_march<4><<<grid, block, 0, s>>>(g, cf, qa, dil, own); break;
     }
 }
+// Planes per block: 8, halved while the tiles would not fill the GPU's four blocks per SM
+// (small boxes: a plane is a dependent step of a block).
+void launch_fx(int V, const Geom& g, const CoefT<double>& cf, const RhsIn<double>& in, int own, cudaStream_t s) {
+    const int nbx = (g.mx + DIL_TX - 1) / DIL_TX, nby = (g.my + DIL_TY - 1) / DIL_TY;
+    int nz = DIL_NZ;
+    while (nz > 1 && (long long)nbx * nby * ((g.mz + nz - 1) / nz) < 4 * 152) nz /= 2;
+    const int tiles = nbx * nby * ((g.mz + nz - 1) / nz);
+    const unsigned grid = (unsigned)tiles + ghost_blocks(g);
+    const dim3 block(DIL_TX, DIL_TY, 1);
+    switch (V) {
+    case 1: k_fx<1><<<grid, block, 0, s>>>(g, cf.fx, in, cf.xp, cf.lam_mu, own, tiles, nbx, nby, nz); break;
+    case 2: k_fx<2><<<grid, block, 0, s>>>(g, cf.fx, in, cf.xp, cf.lam_mu, own, tiles, nbx, nby, nz); break;
+    case 3: k_fx<3><<<grid, block, 0, s>>>(g, cf.fx, in, cf.xp, cf.lam_mu, own, tiles, nbx, nby, nz); break;
+    default: k_fx<4><<<grid, block, 0, s>>>(g, cf.fx, in, cf.xp, cf.lam_mu, own, tiles, nbx, nby, nz); break;
+    }
+}
 template <typename R>
 int launch_reduce(const Geom& g, const Phys& ph, const StateIn& q, const R* mu, int mstride, double* part, int want,
                   double* scal, double* diag, cudaStream_t s) {
@@ -269,8 +311,7 @@ void launch_pack(const Geom& g, const T* src, double* dst, cudaStream_t s) {
     template void launch_pack<R>(const Geom&, const R*, double*, cudaStream_t);
 CNS_INST(double)
 CNS_INST(float)
-template void launch_grad<double>(int, const Geom&, const CoefT<double>&, const double*, const double*, const double*,
-                                  const GradOut<double>&, int, cudaStream_t);
+template void launch_ghost_scalar<long long>(const Geom&, long long*, cudaStream_t);
 // pair mode (FP32-pair RHS arithmetic): the stencil-input kernels and the RHS output
 template void launch_state<ff>(const Geom&, const Phys&, const StateIn&, const DerivedOut<ff>&, double*, int, double*,
                                long long, cudaStream_t);

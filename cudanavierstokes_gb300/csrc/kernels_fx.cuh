@@ -1,0 +1,444 @@
+// kernels_fx.cuh -- FP64 mode: fixed-point stencil inputs, dilatation and the RHS of one
+// point (fx.cuh explains the number format).
+//
+// Per stage, from the ghosted FP64 fields and their maxima:
+//   fx_column   the eight fields of a column of points as integers, and theta from the
+//               integers of u, v, w (fx_point: of one point)
+//   fx_ghost    the same conversion of a ghost cell
+//   fx_table    the stage's scale factors (one thread each)
+//   rhs_acc_fx  the RHS of a point on the integer units; the five sums are converted once
+#pragma once
+#include "cns_common.cuh"
+#include "cns_internal.h"
+#include "fx.cuh"
+#include "kernels_point.cuh"
+
+namespace cns {
+
+// exponents of the eight fields from their maxima; false: a field is out of range
+__device__ __forceinline__ bool fx_exponents(const unsigned* gmax, int (&e)[8]) {
+    const uint4 a = __ldcg((const uint4*)gmax), b = __ldcg((const uint4*)gmax + 1);
+    const unsigned m[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        e[q] = fx_exponent(m[q]);
+        ok = ok && fx_valid(e[q]);
+    }
+    return ok;
+}
+
+// Units. Each sum of the RHS that joins several integer sums has a unit U of its own: the
+// factor K of a term becomes the integer K / U 2^64 <= 2^63 (1 - 2^-20) (equal for the largest
+// K of the sum) and fx_mul of the two gives the term. The gradients and theta have a power of
+// two, 2^G, with factors below 2^62. So every sum is kept to 2^-59 or finer of the largest
+// value that its terms can take; the conversion to FP64 is relative to the value itself.
+constexpr double FX_FULL = 0x1p63 * (1.0 - 0x1p-20);
+
+// x 2^n of a positive normal number on the integer units, kept within the normal range
+__device__ __forceinline__ double fx_scaled(double x, int n) {
+    const int hi = __double2hiint(x);
+    const int ex = min(max((hi >> 20) + n, 1), 2046);
+    return __hiloint2double((ex << 20) | (hi & 0xfffff), __double2loint(x));
+}
+__device__ __forceinline__ double fx_larger(double x, double y) {   // of positive numbers
+    const i64 a = __double_as_longlong(x), b = __double_as_longlong(y);
+    return a > b ? x : y;
+}
+__device__ __forceinline__ int fx_log2(double x) { return (__double2hiint(x) >> 20) - 1023; }   // floor
+
+// unit of theta, 2^x: the largest of its three factors in [2^61, 2^62), theta < 2^61.4
+__device__ __forceinline__ int fx_unit_theta(const FxBase& b, const int (&e)[8]) {
+    return fx_log2(fx_larger(fx_scaled(b.thmax, e[1] - 62),
+                             fx_larger(fx_scaled(b.th[1], e[2] - 62), fx_scaled(b.th[2], e[3] - 62)))) + 3;
+}
+
+// the factors of theta = sum_d (weighted difference of the d-th velocity)_d k_d; xp: 1/x' of
+// the point on a stretched x
+__device__ __forceinline__ void fx_theta_factors(const FxBase& b, const int (&e)[8], int nonuniform_x, double xp,
+                                                 i64& kx, i64& ky, i64& kz) {
+    const int n = fx_unit_theta(b, e);   // K 2^(64 - n) = (K 2^(62 - m)) with m = n - 2
+    kx = fx_from(fx_scaled(nonuniform_x ? b.th[0] * xp : b.th[0], e[1] - 62), n - 2);
+    ky = fx_from(fx_scaled(b.th[1], e[2] - 62), n - 2);
+    kz = fx_from(fx_scaled(b.th[2], e[3] - 62), n - 2);
+}
+
+// the factor of sum q (FXK_*) in direction d; xth: the exponent of theta's unit. Mass flux: Q
+// in units of 2^(e_rho + e_g - 60), weight 1/2; cubic fluxes: Q phi in units of 2^(e_rho + e_g
+// + e_phi - 58), doubled, weight 1/4. On a stretched x the first derivatives' sums are
+// multiplied by x'^-1 / xpmax 2^63 (1 - 2^-20) / 2^64 beforehand (in the base factors).
+__device__ __forceinline__ double fx_factor(const FxBase& b, const int (&e)[8], int xth, int d, int q) {
+    const auto pick = [&](const double (&a)[3]) { return d == 0 ? a[0] : d == 1 ? a[1] : a[2]; };
+    const auto ev = [&](int n) { return n == 0 ? e[1] : n == 1 ? e[2] : e[3]; };   // u, v, w
+    if (q < FXK_MU) return fx_scaled(pick(b.b1V), ev(q) - 62);
+    if (q == FXK_MU) return fx_scaled(pick(b.b1V), e[7] - 62);
+    if (q == FXK_T) return fx_scaled(pick(b.b1V), e[4] - 62);
+    if (q == FXK_TH) return fx_scaled(pick(b.b1V3), xth);
+    if (q == FXK_P) return fx_scaled(pick(b.b1S), e[5] - 62);
+    if (q < FXK_LT) return fx_scaled(pick(b.b2), ev(q - FXK_L) - 62);
+    if (q == FXK_LT) return fx_scaled(pick(b.b2), e[4] - 62);
+    const int er = e[0] + ev(d);
+    if (q == FXK_F0) return fx_scaled(pick(b.b1S), er - 61);
+    return fx_scaled(pick(b.b1S), er + (q == FXK_F + 3 ? e[6] : ev(q - FXK_F)) - 61);
+}
+
+// entry t of the stage's table (FXK_*). The factors from the RHS integers to real values are
+// NaN if a field is out of range, so that the state becomes NaN and is reported as every
+// other non-finite state.
+__device__ __forceinline__ i64 fx_table(const FxBase& b, const unsigned* gmax, int nonuniform_x, double lam_mu, int t) {
+    int e[8];
+    if (!fx_exponents(gmax, e)) return 0x7ff8000000000000LL;
+    const int xth = fx_unit_theta(b, e);
+    const auto K = [&](int d, int q) { return fx_factor(b, e, xth, d, q); };
+    const auto ev = [&](int q) { return q == 1 ? e[1] : q == 2 ? e[2] : q == 3 ? e[3] : e[6]; };   // u, v, w, H
+    const auto big = [&](int q) { return fx_larger(K(0, q), fx_larger(K(1, q), K(2, q))); };
+    // units (2^64 / FX_FULL of the largest factor): the gradients' power of two, above 4 times
+    // their largest factor; the mass sum; the sum of equation q with its centre term's factor;
+    // second derivatives of component q (with grad theta / 3)
+    const int xg = fx_log2(fx_larger(big(FXK_U), fx_larger(big(FXK_U + 1), big(FXK_U + 2)))) + 3;
+    const double U0 = big(FXK_F0) * (0x1p64 / FX_FULL);
+    const auto ctr = [&](int q) { return fx_scaled(U0, ev(q) - 1); };
+    const auto UA = [&](int q) {
+        if (q == 0) return U0;
+        double m = fx_larger(big(FXK_F0 + q), ctr(q));
+        if (q < 4) m = fx_larger(m, K(q - 1, FXK_P));
+        return m * (0x1p64 / FX_FULL);
+    };
+    const auto UL = [&](int q) {
+        double m = big(FXK_L + q);
+        if (q < 3) m = fx_larger(m, K(q, FXK_TH));
+        return m * (0x1p64 / FX_FULL);
+    };
+    const double UM = big(FXK_MU) * (0x1p64 / FX_FULL), UT = big(FXK_T) * (0x1p64 / FX_FULL);
+    const auto factor = [&](double k, double unit) {   // low word, balanced high half
+        const i64 v = __double2ll_rn(k / unit * 0x1p64);
+        return (i64)(((unsigned long long)(unsigned)fx_hi(v) << 32) | (unsigned)fx_lo(v));
+    };
+    if (t < 3 * FXK_DIR) {
+        const int d = t / FXK_DIR, q = t % FXK_DIR;
+        const double u = q < FXK_MU ? fx_pow2(xg) : q == FXK_MU ? UM : q == FXK_T ? UT : q == FXK_TH ? UL(d)
+                         : q == FXK_P ? UA(1 + d) : q <= FXK_LT ? UL(q - FXK_L) : UA(q - FXK_F0);
+        return factor(K(d, q), u);
+    }
+    if (t == FXK_TG) return factor(fx_scaled(1.0 / 3.0, xth), fx_pow2(xg));
+    if (t < FXK_A) return factor(ctr(1 + t - FXK_CTR), UA(1 + t - FXK_CTR));
+    // units as doubles: the five sums; mu times the second derivatives (of T: with lambda/mu);
+    // stress . grad mu, grad T . grad mu (with lambda/mu), the dissipation
+    const double um = fx_pow2(e[7] + 2);
+    return __double_as_longlong(t < FXK_UL ? UA(t - FXK_A) : t < FXK_UL + 3 ? um * UL(t - FXK_UL)
+                                : t == FXK_UL + 3 ? lam_mu * um * UL(3) : t == FXK_UD ? fx_pow2(xg + 64) * UM
+                                : t == FXK_UC ? lam_mu * 0x1p64 * UT * UM : fx_pow2(2 * xg + 64));
+}
+
+// a0 b0 + a1 b1, / 2^62: the second derivative on a stretched x, 1/x'^2 f'' - x''/x'^3 f' of
+// the index derivatives' sums b0 < 2^61, b1 < 2^61.8 with |a0| / 2 + 0.87 |a1| <= 2^62 (1 -
+// 2^-19): the cross sum < 2^62.9, the value < 2^62
+__device__ __forceinline__ i64 fx_mul2(i64 a0, i64 b0, i64 a1, i64 b1) {
+    const int a0h = fx_hi(a0), a0l = fx_lo(a0), a1h = fx_hi(a1), a1l = fx_lo(a1);
+    const int b0h = fx_hi(b0), b0l = fx_lo(b0), b1h = fx_hi(b1), b1l = fx_lo(b1);
+    const i64 m = fx_mad(a0h, b0l, fx_mad(a0l, b0h, fx_mad(a1h, b1l, fx_mad(a1l, b1h, FX_HALF / 4))));
+    return (fx_mad(a0h, b0h, fx_mad(a1h, b1h, 0)) << 2) + (m >> 30);
+}
+
+// the eight fields of element c as integers; u and v given if the caller has them
+__device__ __forceinline__ void fx_store(const FxFields& o, const RhsIn<double>& in, const int (&e)[8], int c, i64 u,
+                                         i64 v, i64 w) {
+    o.f[0][c] = make_longlong2(u, v);
+    o.f[1][c] = make_longlong2(w, fx_from(in.p[c], e[5]));
+    o.f[2][c] = make_longlong2(fx_from(in.t[c], e[4]), fx_from(in.m[c], e[7]));
+    o.f[3][c] = make_longlong2(fx_from(in.r[c], e[0]), fx_from(in.h[c], e[6]));
+}
+
+// the conversion of ghost cell t
+__device__ __forceinline__ void fx_ghost(const Geom& g, const RhsIn<double>& in, const int (&e)[8], int t) {
+    const GhostCell gc = ghost_cell_of(g, t);
+    const int off = gc.side == 0 ? -gc.m : gc.m - 1;
+    const int c = (int)(gc.face == 0   ? g.at(gc.side == 0 ? off : g.mx + off, gc.j, gc.k)
+                        : gc.face == 1 ? g.at(gc.i, gc.side == 0 ? off : g.my + off, gc.k)
+                                       : g.at(gc.i, gc.j, gc.side == 0 ? off : g.mz + off));
+    fx_store(in.fx, in, e, c, fx_from(in.u[c], e[1]), fx_from(in.v[c], e[2]), fx_from(in.w[c], e[3]));
+}
+
+// Conversion of a column of points and its theta. The threads (tx, ty), tx < 32, ty < TY, own
+// the x-y tile at (i0, j0) and march the planes [k0, k1): u of the tile rows with V halo
+// points on either side and v of the tile columns in shared memory, w of the planes k - V ..
+// k + V in a register ring, so that a point converts ~9.4 values instead of the 8 + 6V of
+// fx_point (a conversion is ~20 instructions: 8.6 against 32 made the kernel ALU bound); the
+// next plane's loads are issued before the current plane is computed. Tile slots beyond [-V,
+// mx + V) x [-V, my + V) are read by no interior point and not loaded. All threads of the
+// block call it.
+template <int V, int TY>
+__device__ __forceinline__ void fx_column(const Geom& g, const FxBase& b, const RhsIn<double>& in, const int (&e)[8],
+                                          const double* __restrict__ xp, int i0, int j0, int k0, int k1, bool own,
+                                          int tx, int ty, i64 (*su)[32 + 2 * V], i64 (*sv)[32]) {
+    static_assert(V <= TY, "the y halo rows are loaded by the first and last V tile rows");
+    const int i = i0 + tx, j = j0 + ty;
+    const bool inside = i < g.mx && j < g.my;
+    const bool ghosted = i < g.mx + V && j < g.my + V;   // own slot of the tiles is read by someone
+    const int P = (int)g.P, PS = (int)g.PS;
+    const int c0 = (int)g.at(i, j, 0);
+    i64 kx, ky, kz;
+    fx_theta_factors(b, e, g.nonuniform_x, inside ? xp[i] : 0.0, kx, ky, kz);
+    i64 ring[2 * V + 1];
+#pragma unroll
+    for (int l = 0; l < 2 * V; l++) ring[l] = inside ? fx_from(__ldg(in.w + c0 + (k0 - V + l) * PS), e[3]) : 0;
+    double nw = 0., nu = 0., nv = 0., hx = 0., hy = 0.;
+    const bool xl = tx < V, xr = tx >= 32 - V, yl = ty < V, yr = ty >= TY - V;
+    const auto fetch = [&](int k) {
+        const int ck = c0 + k * PS;
+        nw = inside ? __ldg(in.w + ck + V * PS) : 0.0;
+        if (ghosted) {
+            nu = __ldg(in.u + ck);
+            nv = __ldg(in.v + ck);
+        }
+        // the halos: a thread fills at most one of the two x halos (V <= 16); with V > TY / 2
+        // the rows of the two y halos overlap, the upper one is then fetched at the store
+        if (xl && j < g.my) hx = __ldg(in.u + ck - V);
+        if (xr && i < g.mx && j < g.my) hx = __ldg(in.u + ck + V);
+        if (yl && i < g.mx) hy = __ldg(in.v + ck - V * P);
+        if (yr && j < g.my && i < g.mx && !yl) hy = __ldg(in.v + ck + V * P);
+    };
+    if (k0 < k1) fetch(k0);
+    for (int k = k0; k < k1; k++) {
+        const int ck = c0 + k * PS;
+        double q[5] = {0, 0, 0, 0, 0};
+        if (inside) { q[0] = __ldg(in.p + ck); q[1] = __ldg(in.t + ck); q[2] = __ldg(in.m + ck); q[3] = __ldg(in.r + ck); q[4] = __ldg(in.h + ck); }
+        const i64 cu = fx_from(nu, e[1]), cv = fx_from(nv, e[2]);
+        ring[2 * V] = fx_from(nw, e[3]);
+        const i64 cx = xl || xr ? fx_from(hx, e[1]) : 0, cy = yl || yr ? fx_from(hy, e[2]) : 0;
+        if (k + 1 < k1) fetch(k + 1);
+        __syncthreads();   // the previous plane's tiles are no longer read
+        su[ty][tx + V] = cu;
+        sv[ty + V][tx] = cv;
+        if (xl) su[ty][tx] = cx;
+        if (xr) su[ty][tx + 2 * V] = cx;
+        if (yl) sv[ty][tx] = cy;
+        if (yr && !yl) sv[ty + 2 * V][tx] = cy;
+        if (2 * V > TY && yr && yl && j < g.my && i < g.mx) sv[ty + 2 * V][tx] = fx_from(__ldg(in.v + ck + V * P), e[2]);
+        __syncthreads();
+        if (inside) {
+            FxSum sx, sy, sz;
+#pragma unroll
+            for (int l = 1; l <= V; l++) {
+                sx.add(su[ty][tx + V + l] - su[ty][tx + V - l], fxw1(V, l));
+                sy.add(sv[ty + V + l][tx] - sv[ty + V - l][tx], fxw1(V, l));
+                sz.add(ring[V + l] - ring[V - l], fxw1(V, l));
+            }
+            const i64 th = fx_mul(sx.value(), kx) + fx_mul(sy.value(), ky) + fx_mul(sz.value(), kz);
+            in.fx.th[ck] = th;
+            if (own) dil_ghost_owner<i64>(g, in.fx.th, ck, i, j, k, th);
+            in.fx.f[0][ck] = make_longlong2(cu, cv);
+            in.fx.f[1][ck] = make_longlong2(ring[V], fx_from(q[0], e[5]));
+            in.fx.f[2][ck] = make_longlong2(fx_from(q[1], e[4]), fx_from(q[2], e[7]));
+            in.fx.f[3][ck] = make_longlong2(fx_from(q[3], e[0]), fx_from(q[4], e[6]));
+        }
+#pragma unroll
+        for (int l = 0; l < 2 * V; l++) ring[l] = ring[l + 1];
+    }
+}
+
+// The conversion and theta of one point, every neighbour from global memory (the batched
+// stage kernel's form; the same integers)
+template <int V>
+__device__ __forceinline__ void fx_point(const Geom& g, const FxBase& b, const RhsIn<double>& in, const int (&e)[8],
+                                         const double* __restrict__ xp, int i, int j, int k) {
+    const int c = (int)g.at(i, j, k), P = (int)g.P, PS = (int)g.PS;
+    i64 kx, ky, kz;
+    fx_theta_factors(b, e, g.nonuniform_x, xp[i], kx, ky, kz);
+    FxSum sx, sy, sz;
+#pragma unroll
+    for (int l = 1; l <= V; l++) {
+        sx.add(fx_from(in.u[c + l], e[1]) - fx_from(in.u[c - l], e[1]), fxw1(V, l));
+        sy.add(fx_from(in.v[c + l * P], e[2]) - fx_from(in.v[c - l * P], e[2]), fxw1(V, l));
+        sz.add(fx_from(in.w[c + l * PS], e[3]) - fx_from(in.w[c - l * PS], e[3]), fxw1(V, l));
+    }
+    const i64 th = fx_mul(sx.value(), kx) + fx_mul(sy.value(), ky) + fx_mul(sz.value(), kz);
+    in.fx.th[c] = th;
+    fx_store(in.fx, in, e, c, fx_from(in.u[c], e[1]), fx_from(in.v[c], e[2]), fx_from(in.w[c], e[3]));
+}
+
+// The sums of one direction at a point, in two passes over the neighbour pairs (-l, l), each of
+// which loads a pair once and feeds every sum that needs it:
+//   fx_visc  first derivatives of u, v, w, mu, T, theta and second ones of u, v, w, T (viscous
+//            order)
+//   fx_conv  first derivative of p and the telescoped split-form fluxes (advective order)
+//              sum_l a_l (Q- - Q+)  and  sum_l a_l (Q- phi_{-l} - Q+ phi_l),
+//              Q+- = (rho_0 + rho_{+-l}) (g_0 + g_{+-l}),  g the velocity along the direction
+// Bounds (F: a field, |F| < 2^62): differences and sums of two fields < 2^63; Q < 2^62; a
+// flux term's two sides together < 2^61, their cross products < 2^63 (1 - 2^-21) + 2^33.
+struct FxVisc {
+    i64 d[6], L[4];   // u, v, w, mu, T, theta; u, v, w, T
+};
+struct FxConv {
+    i64 p, F[5];   // mass flux; u, v, w, H fluxes, doubled
+};
+
+template <int V>
+__device__ __forceinline__ FxVisc fx_visc(const FxFields& in, int c, int st, const i64 (&ctr)[4]) {
+    FxSum D[6], L[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) L[q].add(ctr[q], fxw2(V, 0));
+#pragma unroll
+    for (int l = 1; l <= V; l++) {
+        const longlong2 am = __ldg(in.f[0] + c - l * st), ap = __ldg(in.f[0] + c + l * st);
+        const longlong2 bm = __ldg(in.f[1] + c - l * st), bp = __ldg(in.f[1] + c + l * st);
+        const longlong2 tm = __ldg(in.f[2] + c - l * st), tp = __ldg(in.f[2] + c + l * st);
+        D[0].add(ap.x - am.x, fxw1(V, l));
+        D[1].add(ap.y - am.y, fxw1(V, l));
+        D[2].add(bp.x - bm.x, fxw1(V, l));
+        D[3].add(tp.y - tm.y, fxw1(V, l));
+        D[4].add(tp.x - tm.x, fxw1(V, l));
+        D[5].add(__ldg(in.th + c + l * st) - __ldg(in.th + c - l * st), fxw1(V, l));
+        L[0].add(ap.x + am.x, fxw2(V, l));
+        L[1].add(ap.y + am.y, fxw2(V, l));
+        L[2].add(bp.x + bm.x, fxw2(V, l));
+        L[3].add(tp.x + tm.x, fxw2(V, l));
+    }
+    FxVisc o;
+#pragma unroll
+    for (int q = 0; q < 6; q++) o.d[q] = D[q].value();
+#pragma unroll
+    for (int q = 0; q < 4; q++) o.L[q] = L[q].value();
+    return o;
+}
+
+template <int S, int DIR>
+__device__ __forceinline__ FxConv fx_conv(const FxFields& in, int c, int st, i64 r0, i64 g0) {
+    FxSum P, F[5];
+#pragma unroll 1
+    for (int l = 1; l <= S; l++) {
+        const longlong2 am = __ldg(in.f[0] + c - l * st), ap = __ldg(in.f[0] + c + l * st);
+        const longlong2 bm = __ldg(in.f[1] + c - l * st), bp = __ldg(in.f[1] + c + l * st);
+        const longlong2 hm = __ldg(in.f[3] + c - l * st), hp = __ldg(in.f[3] + c + l * st);
+        P.add(bp.y - bm.y, fxw1(S, l));
+        const i64 gm = DIR == 0 ? am.x : DIR == 1 ? am.y : bm.x;
+        const i64 gp = DIR == 0 ? ap.x : DIR == 1 ? ap.y : bp.x;
+        const i64 qm = fx_mul(hm.x + r0, gm + g0), qp = -fx_mul(hp.x + r0, gp + g0);
+        F[0].add(qm + qp, fxw1(S, l));
+        const int qmh = fx_hi(qm), qml = fx_lo(qm), qph = fx_hi(qp), qpl = fx_lo(qp);
+        const i64 phm[4] = {am.x, am.y, bm.x, hm.y}, php[4] = {ap.x, ap.y, bp.x, hp.y};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int mh = fx_hi(phm[q]), ml = fx_lo(phm[q]), ph = fx_hi(php[q]), pl = fx_lo(php[q]);
+            const i64 m = fx_mad(qmh, ml, fx_mad(qml, mh, fx_mad(qph, pl, fx_mad(qpl, ph, FX_HALF))));
+            F[1 + q].add(fx_mad(qmh, mh, fx_mad(qph, ph, (i64)fx_word1(m))), fxw1(S, l));
+        }
+    }
+    FxConv o;
+    o.p = P.value();
+#pragma unroll
+    for (int q = 0; q < 5; q++) o.F[q] = q == 0 ? F[q].value() : F[q].twice();
+    return o;
+}
+
+// fx_mul with a table factor (low word, balanced high half)
+__device__ __forceinline__ i64 fx_mulk(i64 v, i64 k) {
+    const int vh = fx_hi(v), vl = fx_lo(v), kh = fx_word1(k), kl = fx_lo(k);
+    const i64 m = fx_mad(vh, kl, fx_mad(vl, kh, FX_HALF));
+    return fx_mad(vh, kh, (i64)fx_word1(m));
+}
+
+// a b / 2^62, |a b| < 2^124.6
+__device__ __forceinline__ i64 fx_mul_by4(i64 a, i64 b) {
+    const int ah = fx_hi(a), al = fx_lo(a), bh = fx_hi(b), bl = fx_lo(b);
+    const i64 m = fx_mad(ah, bl, fx_mad(al, bh, FX_HALF / 4));
+    return (fx_mad(ah, bh, 0) << 2) + (m >> 30);
+}
+
+// sum of three products / 2^64, the low halves' products (below a quarter each) left out;
+// factors below 2^62 and 2^62: the cross sums < 2^62.6 in pairs of products
+__device__ __forceinline__ i64 fx_dot3(i64 a0, i64 b0, i64 a1, i64 b1, i64 a2, i64 b2) {
+    const int a0h = fx_hi(a0), a1h = fx_hi(a1), a2h = fx_hi(a2), b0h = fx_hi(b0), b1h = fx_hi(b1), b2h = fx_hi(b2);
+    const i64 m = fx_mad(a0h, fx_lo(b0), fx_mad(fx_lo(a0), b0h, FX_HALF));
+    const i64 n = fx_mad(a1h, fx_lo(b1), fx_mad(fx_lo(a1), b1h, FX_HALF));
+    const i64 o = fx_mad(a2h, fx_lo(b2), fx_mad(fx_lo(a2), b2h, FX_HALF));
+    return fx_mad(a0h, b0h, fx_mad(a1h, b1h, fx_mad(a2h, b2h, (i64)fx_word1(m) + fx_word1(n) + fx_word1(o))));
+}
+// magnitude bits of the high word, and the left shift that brings the largest of several
+// values (the OR of their bits) to [2^61, 2^62)
+__device__ __forceinline__ int fx_bits(i64 v) { return fx_word1(v) ^ (fx_word1(v) >> 31); }
+__device__ __forceinline__ int fx_room(int bits) { return max(__clz(bits) - 2, 0); }
+
+// RHS of one interior point at element c into out (without body force and sponge). Bounds in
+// the units of fx_table: gradients < 2^59.8, theta, stress < 2^61.8, grad mu, grad T < 2^60.8,
+// second derivatives < 2^62.3, RHS sums < 2^62.4.
+template <int S, int V>
+__device__ __forceinline__ void rhs_acc_fx(const Geom& g, const FxBase& b, const RhsIn<double>& in, int quirk, int i,
+                                           int c, double u0, double v0, double w0, double (&out)[5]) {
+    const FxFields& x = in.fx;
+    const i64* __restrict__ K = x.k;
+    i64 acc[5] = {0, 0, 0, 0, 0};
+    const bool nux = g.nonuniform_x;
+    const i64 xp = nux ? __ldg(b.xpk + i) : 0;
+    const longlong2 A = __ldg(x.f[0] + c), B = __ldg(x.f[1] + c), H = __ldg(x.f[3] + c);
+    const auto conv = [&](const FxConv& o, int d, bool sx) {
+        const i64* k = K + d * FXK_DIR;
+        const auto f = [&](i64 v, int q) { return fx_mulk(sx ? fx_mulk(v, xp) : v, k[q]); };
+        acc[1 + d] -= f(o.p, FXK_P);
+#pragma unroll
+        for (int q = 0; q < 5; q++) acc[q] += f(o.F[q], FXK_F0 + q);
+    };
+    conv(fx_conv<S, 0>(x, c, 1, H.x, A.x), 0, nux);
+    conv(fx_conv<S, 1>(x, c, (int)g.P, H.x, A.y), 1, false);
+    conv(fx_conv<S, 2>(x, c, (int)g.PS, H.x, B.x), 2, false);
+    // the cubic fluxes' centre values: phi_0 times half the mass flux
+    const i64 phi[4] = {A.x, A.y, B.x, H.y};
+#pragma unroll
+    for (int q = 0; q < 4; q++) acc[1 + q] += fx_mulk(fx_mul_by4(phi[q], acc[0]), K[FXK_CTR + q]);
+    const longlong2 T = __ldg(x.f[2] + c);
+    const i64 ctr[4] = {A.x, A.y, B.x, T.x};
+    const longlong2 xx = nux ? __ldg(b.xx + i) : make_longlong2(0, 0);
+    i64 G[9], dmu[3], dT[3], L[4] = {0, 0, 0, 0};
+    const auto visc = [&](const FxVisc& o, int d, bool sx) {
+        const i64* k = K + d * FXK_DIR;
+        const auto f = [&](i64 v, int q) { return fx_mulk(sx ? fx_mulk(v, xp) : v, k[q]); };
+#pragma unroll
+        for (int q = 0; q < 3; q++) G[3 * d + q] = f(o.d[q], FXK_U + q);
+        dmu[d] = f(o.d[3], FXK_MU);
+        dT[d] = f(o.d[4], FXK_T);
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            L[q] += fx_mulk(sx ? fx_mul2(xx.x, o.L[q], xx.y, o.d[q < 3 ? q : 4]) : o.L[q], k[FXK_L + q]);
+        L[d] += f(o.d[5], FXK_TH);
+    };
+    visc(fx_visc<V>(x, c, 1, ctr), 0, nux);
+    visc(fx_visc<V>(x, c, (int)g.P, ctr), 1, false);
+    visc(fx_visc<V>(x, c, (int)g.PS, ctr), 2, false);
+    const auto unit = [&](int q, int s) {   // table unit times 2^-s
+        const double k = __longlong_as_double(K[q]);
+        return __hiloint2double(__double2hiint(k) - (s << 20), __double2loint(k));
+    };
+    // grad mu and the stress tensor tau / mu, each scaled to the full range
+    const int sm = fx_room(fx_bits(dmu[0]) | fx_bits(dmu[1]) | fx_bits(dmu[2]));
+#pragma unroll
+    for (int q = 0; q < 3; q++) dmu[q] <<= sm;
+    const i64 th3 = fx_mulk(__ldg(x.th + c), K[FXK_TG]);   // theta / 3
+    i64 t[6] = {2 * (G[0] - th3), 2 * (G[4] - th3), 2 * (G[8] - th3), G[1] + G[3], G[2] + G[6], G[5] + G[7]};
+    // y-z dissipation with the quirk: tau_yz dv/dz in the y sum as in the z sum (src/cuda_rhs.cu:175)
+    i64 q12 = quirk ? 2 * G[7] : t[5];
+    const int st = fx_room(fx_bits(t[0]) | fx_bits(t[1]) | fx_bits(t[2]) | fx_bits(t[3]) | fx_bits(t[4]) |
+                           fx_bits(t[5]) | fx_bits(q12));
+#pragma unroll
+    for (int q = 0; q < 6; q++) t[q] <<= st;
+    q12 <<= st;
+    // dissipation / mu: tau_ab du_b/dx_a = sum t_aa^2 / 2 (the trace of t is zero) + sum t_ab^2
+    const i64 diss = (fx_dot3(t[0], t[0], t[1], t[1], t[2], t[2]) >> 1) + fx_dot3(t[3], t[3], t[4], t[4], t[5], q12);
+    const double ud = unit(FXK_UD, sm + st);
+    const double W[3] = {fma((double)fx_mul(T.y, L[0]), unit(FXK_UL, 0),
+                             (double)fx_dot3(t[0], dmu[0], t[3], dmu[1], t[4], dmu[2]) * ud),
+                         fma((double)fx_mul(T.y, L[1]), unit(FXK_UL + 1, 0),
+                             (double)fx_dot3(t[3], dmu[0], t[1], dmu[1], t[5], dmu[2]) * ud),
+                         fma((double)fx_mul(T.y, L[2]), unit(FXK_UL + 2, 0),
+                             (double)fx_dot3(t[4], dmu[0], t[5], dmu[1], t[2], dmu[2]) * ud)};
+    double en = (double)acc[4] * unit(FXK_A + 4, 0);
+    en = fma((double)fx_mul(T.y, L[3]), unit(FXK_UL + 3, 0), en);
+    en = fma((double)fx_dot3(dT[0], dmu[0], dT[1], dmu[1], dT[2], dmu[2]), unit(FXK_UC, sm), en);
+    en = fma(in.m[c], (double)diss * unit(FXK_UE, 2 * st), en);
+    out[0] = (double)acc[0] * unit(FXK_A, 0);
+    out[1] = fma((double)acc[1], unit(FXK_A + 1, 0), W[0]);
+    out[2] = fma((double)acc[2], unit(FXK_A + 2, 0), W[1]);
+    out[3] = fma((double)acc[3], unit(FXK_A + 3, 0), W[2]);
+    out[4] = en + fma(u0, W[0], fma(v0, W[1], w0 * W[2]));
+}
+
+}  // namespace cns

@@ -4,6 +4,7 @@
 #pragma once
 #include "cns_common.cuh"
 #include "cns_internal.h"
+#include "fx.cuh"
 
 namespace cns {
 
@@ -52,6 +53,7 @@ __device__ __forceinline__ void state_store(const Phys& ph, const DerivedOut<R>&
         o.p[c] = to_r<R>(pr);
         o.h[c] = to_r<R>(hh);
         o.m[c] = to_r<R>(suth * ph.invRe);
+        if constexpr (!is_ff<R>) fx_track(o.gmax, {rr, uu, vv, ww, T, pr, hh, suth * ph.invRe});
         if (!positive_bits(T) || !positive_bits(rr)) scal[SC_NONFINITE] = 1.0;   // racy flag write, any writer is fine
     }
 }
@@ -203,6 +205,10 @@ __device__ __forceinline__ void ghost_state_cell(const Geom& g, const Phys& ph, 
         return;
     }
     R* F[8] = {f.r, f.u, f.v, f.w, f.t, f.p, f.h, f.m};
+    // FP64 mode: ghosts that are no copies of interior values join the maxima; the next
+    // state's slots start at zero (its writer runs after this phase)
+    constexpr bool FX = !is_ff<R> && sizeof(R) == 8;
+    if (FX && t < 8) f.gnext[t] = 0u;
     const GhostCell gc = ghost_cell_of(g, t);
     const int m = gc.m, side = gc.side;
     long long cg, cs;
@@ -240,6 +246,9 @@ __device__ __forceinline__ void ghost_state_cell(const Geom& g, const Phys& ph, 
             f.m[cg] = to_r<R>(suth * ph.invRe);
             f.h[cg] = to_r<R>(Tg * ph.hcoef + 0.5 * (ug * ug + vg * vg + wg * wg));
             f.r[cg] = to_r<R>(pg / (ph.Rgas * Tg));
+            if constexpr (FX)
+                fx_track(f.gmax, {pg / (ph.Rgas * Tg), ug, vg, wg, Tg, pg,
+                                  Tg * ph.hcoef + 0.5 * (ug * ug + vg * vg + wg * wg), suth * ph.invRe});
             return;
         }
         cs = g.at(side == 0 ? g.mx - m : m - 1, j, k);
@@ -255,7 +264,8 @@ __device__ __forceinline__ void ghost_state_cell(const Geom& g, const Phys& ph, 
 #pragma unroll
             for (int q = 0; q < 8; q++) { a[q] = F[q][c0]; b[q] = F[q][cm]; }
 #pragma unroll
-            for (int q = 0; q < 8; q++) F[q][cg] = (R)2.0 * a[q] - b[q];
+            for (int q = 0; q < 8; q++) { a[q] = (R)2.0 * a[q] - b[q]; F[q][cg] = a[q]; }
+            if constexpr (FX) fx_track(f.gmax, a);
             return;
         }
         cs = g.at(gc.i, gc.j, side == 0 ? g.mz - m : m - 1);

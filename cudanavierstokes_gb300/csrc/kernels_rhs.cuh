@@ -19,6 +19,7 @@
 #pragma once
 #include "cns_common.cuh"
 #include "cns_internal.h"
+#include "kernels_fx.cuh"
 #include "kernels_point.cuh"
 
 namespace cns {
@@ -639,6 +640,12 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
                                           double* __restrict__ scal, int quirk, int i, int j, int k) {
     if constexpr (sizeof(R) == 4) {
         rhs_point_packed<S, V, CW>(g, cf, in, up, scal, quirk, i, j, k);
+    } else if constexpr (!is_ff<R>) {
+        const int c = (int)g.at(i, j, k);
+        const double u0 = up.qin.u[c], v0 = up.qin.v[c], w0 = up.qin.w[c];
+        double acc[5];
+        rhs_acc_fx<S, V>(g, cf.fx, in, quirk, i, c, u0, v0, w0, acc);
+        stage_tail<double>(g, up, scal, i, k, c, acc, u0, v0, w0, up.qin.r[c]);
     } else {
         const int c = (int)g.at(i, j, k);
         const R th0 = ld(in.dil, c), m0 = ld(in.m, c);
@@ -659,7 +666,7 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
 // group's blocks sweep them (one launch over whole planes would cycle ~2S planes of the
 // inputs through L2 between their uses).
 template <typename R, int S, int V>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 4) k_rhs(Geom g, const __grid_constant__ CoefT<R> cf,
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : is_ff<R> ? 4 : 5) k_rhs(Geom g, const __grid_constant__ CoefT<R> cf,
                                                                                    const __grid_constant__ RhsIn<R> in, Update<R> up,
                                              double* __restrict__ scal, int quirk, int band0) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -13,6 +13,7 @@
 // host and MPI every check_cfl steps: src/cuda_main.cu:249-265).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -23,6 +24,7 @@
 
 #include "../../include/cns.h"
 #include "cns_internal.h"
+#include "fx.cuh"
 #include "grid.h"
 #include "solver_internal.h"
 
@@ -122,6 +124,8 @@ RhsIn<R> rhs_in(cns_solver* h, int c) {
         for (int q = 0; q < 9; q++) in.g[q] = (const R*)h->grad[q];
     }
     in.dil = (const R*)h->dil;
+    in.fx = h->fx;
+    in.fx.gmax = h->gmax[c]; in.fx.gnext = h->gmax[1 - c];
     return in;
 }
 
@@ -137,6 +141,7 @@ DerivedOut<R> derived_out(cns_solver* h, int b) {
         o.qa = (float4*)h->der[b][0];
         o.qb = (float4*)h->der[b][1];
     } else {
+        o.gmax = h->gmax[b];
         o.h = (R*)h->der[b][0]; o.t = (R*)h->der[b][1]; o.p = (R*)h->der[b][2]; o.m = (R*)h->der[b][3];
         if constexpr (is_ff<R>) {
             o.r = (R*)h->der[b][4]; o.u = (R*)h->der[b][5]; o.v = (R*)h->der[b][6]; o.w = (R*)h->der[b][7];
@@ -148,6 +153,7 @@ DerivedOut<R> derived_out(cns_solver* h, int b) {
 // calcState of the current state (when the RHS kernel has not recovered it already)
 template <typename R>
 int state_phase(cns_solver* h) {
+    if (h->gmax[0]) CK(cudaMemsetAsync(h->gmax[h->cur], 0, 8 * sizeof(unsigned), h->stream));
     launch_state<R>(h->geom, h->phys, state_in(h, h->cur), derived_out<R>(h, h->cur), h->scal, 0, nullptr, 0,
                     h->stream);
     h->launches += 1;
@@ -171,6 +177,7 @@ int ghost_phase(cns_solver* h) {
     } else {
         f.r = (R*)h->q[c][0]; f.u = (R*)h->q[c][1]; f.v = (R*)h->q[c][2]; f.w = (R*)h->q[c][3];
         f.t = o.t; f.p = o.p; f.h = o.h; f.m = o.m;
+        f.gmax = h->gmax[c]; f.gnext = h->gmax[1 - c];
     }
     launch_ghost_state<R>(h->geom, h->phys, f, h->scal, h->stream);
     h->launches += 1;
@@ -186,19 +193,19 @@ int grad_phase(cns_solver* h) {
     if constexpr (std::is_same<R, float>::value) {   // FP32-RHS: theta alone, from the packed records
         launch_dil_packed(h->p.stencil_visc, h->geom, h->cf32, (const float4*)h->der[h->cur][0], (float*)h->dil,
                           own ? 1 : 0, h->stream);
-    } else {
+    } else if constexpr (is_ff<R>) {
         GradOut<R> o;
         for (int q = 0; q < 9; q++) o.g[q] = (R*)h->grad[q];
         o.dil = (R*)h->dil;
         const RhsIn<R> in = rhs_in<R>(h, h->cur);
-        if constexpr (is_ff<R>)
-            launch_grad<R>(h->p.stencil_visc, h->geom, h->cfp, in.u, in.v, in.w, o, own ? 1 : 0, h->stream);
-        else
-            launch_grad<R>(h->p.stencil_visc, h->geom, h->cf64, in.u, in.v, in.w, o, own ? 1 : 0, h->stream);
+        launch_grad<R>(h->p.stencil_visc, h->geom, h->cfp, in.u, in.v, in.w, o, own ? 1 : 0, h->stream);
+    } else {   // FP64: the stencil inputs as fixed-point values, and theta
+        launch_fx(h->p.stencil_visc, h->geom, h->cf64, rhs_in<R>(h, h->cur), own ? 1 : 0, h->stream);
     }
     h->launches += 1;
     if (!own) {
-        launch_ghost_scalar<R>(h->geom, (R*)h->dil, h->stream);
+        if constexpr (std::is_same<R, double>::value) launch_ghost_scalar<long long>(h->geom, h->fx.th, h->stream);
+        else launch_ghost_scalar<R>(h->geom, (R*)h->dil, h->stream);
         h->launches += 1;
     }
     CKL();
@@ -400,6 +407,60 @@ int upload_grid_tables(cns_solver* h) {
     return CNS_OK;
 }
 
+// FP64 mode: the grid's part of the fixed-point scale factors, and the integer metrics of a
+// stretched x: 1/x' (xpk) and, of f'' and f' in the second derivative 1/x'^2 f'' - x''/x'^3 f',
+// the factors xx, |xx.x| / 2 + 0.87 |xx.y| <= 2^62 (1 - 2^-19) at every i
+int set_fx_base(cns_solver* h) {
+    const int mx = h->p.mx, S = h->p.stencil_size, V = h->p.stencil_visc;
+    const HostGrid& g = h->hg;
+    FxBase& b = h->cf64.fx;
+    const double inv[3] = {g.dx, g.dy, g.dz}, inv2[3] = {g.d2x, g.d2y, g.d2z};
+    for (int d = 0; d < 3; d++) {
+        b.b1V[d] = ldexp(inv[d] / fxn1(V), 32 - fxs1(V));
+        b.b1S[d] = ldexp(inv[d] / fxn1(S), 32 - fxs1(S));
+        b.b2[d] = ldexp(inv2[d] / fxn2(V), 32 - fxs2(V));
+    }
+    const auto derived = [&] {
+        for (int d = 0; d < 3; d++) b.b1V3[d] = b.b1V[d] / 3.0;
+    };
+    for (int d = 0; d < 3; d++) b.th[d] = b.b1V[d];
+    b.thmax = b.th[0];
+    b.xx = nullptr;
+    b.xpk = nullptr;
+    derived();
+    if (!h->geom.nonuniform_x) return CNS_OK;
+    double big = 0.0, xpmax = 0.0;
+    std::vector<double> f2(mx), f1(mx);
+    for (int i = 0; i < mx; i++) {
+        const double xp = g.xp[i];
+        f2[i] = b.b2[0] * (xp * xp);
+        f1[i] = -b.b1V[0] * (g.xpp[i] * (xp * xp * xp));
+        big = std::max(big, 0.5 * fabs(f2[i]) + 0.87 * fabs(f1[i]));
+        xpmax = std::max(xpmax, fabs(xp));
+    }
+    const double scale = ldexp(1.0 - 0x1p-19, 62) / big;
+    std::vector<longlong2> xx(mx);
+    std::vector<long long> xk(mx);
+    for (int i = 0; i < mx; i++) {
+        xx[i] = make_longlong2(llrint(f2[i] * scale), llrint(f1[i] * scale));
+        const long long v = llrint(ldexp(g.xp[i] / xpmax, 63) * (1.0 - 0x1p-20));
+        const long long lo = (long long)(int)(unsigned)v, hi = (v - lo) >> 32;   // balanced halves
+        xk[i] = (long long)(((unsigned long long)(unsigned)hi << 32) | (unsigned)lo);
+    }
+    int rc;
+    if ((rc = h->alloc(&h->xx, xx.size())) || (rc = h->alloc(&h->xpk, xk.size()))) return rc;
+    CK(cudaMemcpy(h->xx, xx.data(), xx.size() * sizeof(longlong2), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(h->xpk, xk.data(), xk.size() * sizeof(long long), cudaMemcpyHostToDevice));
+    b.xx = h->xx;
+    b.xpk = h->xpk;
+    b.b2[0] = 0x1p62 / scale;
+    b.thmax = b.th[0] * xpmax;
+    b.b1V[0] *= xpmax * 2.0 / (1.0 - 0x1p-20);
+    b.b1S[0] *= xpmax * 2.0 / (1.0 - 0x1p-20);
+    derived();
+    return CNS_OK;
+}
+
 int sync_and_check(cns_solver* h) {
     CK(cudaStreamSynchronize(h->stream));
     double sc[SC_COUNT];
@@ -550,8 +611,15 @@ int cns_create(const cns_params* pin, int device, cns_solver** out) {
             for (int f = 0; f < (h->pair ? 8 : 4) && !rc; f++) rc = h->alloc_field(&h->der[b][f], rs);
     }
     if (!rc) rc = h->alloc_field(&h->dil, rs);
-    if (!h->fp32)   // FP32-RHS: the RHS kernel forms the velocity gradients itself
+    if (h->pair) {
         for (int f = 0; f < 9 && !rc; f++) rc = h->alloc_field(&h->grad[f], rs);
+    } else if (!h->fp32) {
+        for (int f = 0; f < 4 && !rc; f++) rc = h->alloc_field((void**)&h->fx.f[f], sizeof(longlong2));
+        h->fx.th = (long long*)h->dil;
+        if (!rc) rc = h->alloc(&h->fx.k, FXK_COUNT);
+        for (int b = 0; b < 2 && !rc; b++) rc = h->alloc(&h->gmax[b], 8);
+        if (!rc) rc = set_fx_base(h);
+    }
     if (!rc) rc = h->alloc_fields(h->rb, 5, rs);
     if (!rc && p.scheme != CNS_RK3_LOWSTORAGE) {
         for (int f = 0; f < 5 && !rc; f++) rc = h->alloc_field(&h->k2[f], rs);

@@ -43,11 +43,17 @@ struct cns_solver {
     // q[cur] and writes those of the new state q[1 - cur] (fused state recovery). Pair mode:
     // der[b][0..3] = h, t, p, mu and der[b][4..7] = rho, u, v, w, all as pairs
     void* der[2][8] = {};
+    // FP64 mode: fixed-point stencil inputs of the current stage (kernels_fx.cuh), the
+    // stage's scale factors, and the maxima of the fields of each state buffer
+    cns::FxFields fx{};
+    unsigned* gmax[2] = {};
+    longlong2* xx = nullptr;     // integer metrics of a stretched x
+    long long* xpk = nullptr;
     bool der_ok[2] = {false, false};   // der[b] holds the recovery of q[b]
     int mu_buf = 0;                    // buffer of the latest state recovery in program order of
                                        // the reference (its mu sets the CFL time step)
     void* dil = nullptr;         // (R)
-    void* grad[9] = {};          // (R)
+    void* grad[9] = {};          // pair mode (R)
     void* rb[5] = {};            // RHS register (R)
     void* k2[5] = {};            // classic RK3 k2 / RK4 accumulator (R)
     double* q0[5] = {};          // classic schemes: conserved state at the step start
@@ -139,6 +145,7 @@ inline void solver_set_parity(cns_solver* h, int want) {
     for (int f = 0; f < 8; f++) {
         void* a = h->der[0][f]; h->der[0][f] = h->der[1][f]; h->der[1][f] = a;
     }
+    unsigned* gm = h->gmax[0]; h->gmax[0] = h->gmax[1]; h->gmax[1] = gm;
     const bool ok0 = h->der_ok[0];
     h->der_ok[0] = h->der_ok[1];
     h->der_ok[1] = ok0;
