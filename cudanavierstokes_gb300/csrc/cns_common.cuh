@@ -11,7 +11,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "ff.cuh"
 #include "pow_tables.h"
 
 namespace cns {
@@ -161,13 +160,11 @@ __device__ __forceinline__ double f2d(float f) {
 template <typename R>
 __device__ __forceinline__ R to_r(double x) {
     if constexpr (sizeof(R) == 4) return d2f(x);
-    else if constexpr (is_ff<R>) return d_to_ff(x);
     else return x;
 }
 template <typename R>
 __device__ __forceinline__ double to_d(R x) {
     if constexpr (sizeof(R) == 4) return f2d(x);
-    else if constexpr (is_ff<R>) return ff_to_d(x);
     else return x;
 }
 

@@ -28,7 +28,6 @@ template <typename R>
 struct DerivedOut {
     unsigned* gmax;     // FP64 mode: the fields' maxima (fx_track, fx.cuh)
     R *h, *t, *p, *m;   // FP64 mode
-    R *r, *u, *v, *w;   // pair mode: the state's rho, u, v, w as pairs
     float4 *qa, *qb;    // FP32-RHS mode
 };
 
@@ -56,18 +55,11 @@ struct FxFields {
     unsigned *gmax, *gnext;   // maxima of this state's fields; of the next state's
 };
 
-template <typename R>
-struct GradOut {
-    R* g[9];
-    R* dil;
-};
-
-// RHS stage kernel inputs (FP64: separate fields and the nine velocity gradients; FP32-RHS:
-// the packed records qa, qb and theta, the RHS kernel forms the gradients itself)
+// RHS stage kernel inputs (FP64: separate fields and their fixed-point form; FP32-RHS: the
+// packed records qa, qb and theta)
 template <typename R>
 struct RhsIn {
     const R *r, *u, *v, *w, *t, *p, *h, *m, *dil;
-    const R* g[9];
     const float4 *qa, *qb;
     FxFields fx;   // FP64 mode
 };
@@ -112,9 +104,6 @@ template <typename R>
 void launch_ghost_state(const Geom& g, const Phys& ph, const StencilFields<R>& f, const double* scal, cudaStream_t s);
 template <typename R>
 void launch_ghost_scalar(const Geom& g, R* f, cudaStream_t s);
-template <typename R>
-void launch_grad(int V, const Geom& g, const CoefT<R>& cf, const R* u, const R* v, const R* w, const GradOut<R>& o,
-                 int own, cudaStream_t s);
 // FP32-RHS dilatation (and its ghost images with own) from the packed records (rho, u, v, w)
 void launch_dil_packed(int V, const Geom& g, const CoefT<float>& cf, const float4* qa, float* dil, int own,
                        cudaStream_t s);
@@ -142,7 +131,4 @@ int launch_rhs_fp64(int S, int V, const Geom& g, const Phys& ph, const CoefT<dou
 void launch_fx(int V, const Geom& g, const CoefT<double>& cf, const RhsIn<double>& in, int own, cudaStream_t s);
 int launch_rhs_fp32(int S, int V, const Geom& g, const Phys& ph, const CoefT<float>& cf, const RhsIn<float>& in,
                     const Update<float>& up, double* scal, int quirk, cudaStream_t s);
-int launch_rhs_pair(int S, int V, const Geom& g, const Phys& ph, const CoefT<ff>& cf, const RhsIn<ff>& in,
-                    const Update<ff>& up, double* scal, int quirk, cudaStream_t s);
-
 }  // namespace cns

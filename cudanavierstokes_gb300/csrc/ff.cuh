@@ -14,8 +14,8 @@
 // Every step uses the _rn intrinsics, which the compiler neither contracts into FMAs nor
 // reassociates: the error-free transforms rely on each rounding happening as written.
 //
-// On this GPU an FP64 operation issues to 2 lanes per SM per cycle and an FP32 one to 128,
-// so a pair operation of 9-20 FP32 instructions still has several times the FP64 rate.
+// Behind cns_selftest_pair. (The solver's RHS ran in this type under CNS_PREC_PAIR_RHS at 3.3x
+// the rate of FP64 arithmetic; the fixed-point sums of fx.cuh are faster and more accurate.)
 #pragma once
 #include <cuda_runtime.h>
 

@@ -1,5 +1,5 @@
-// kernels_common.cu -- state recovery, ghost fills, velocity gradients, reductions and
-// layout conversion. The RHS/stage kernel lives in kernels_rhs.cuh.
+// kernels_common.cu -- state recovery, ghost fills, fixed-point conversion, dilatation,
+// reductions and layout conversion. The RHS/stage kernel lives in kernels_rhs.cuh.
 #include "cns_common.cuh"
 #include "cns_internal.h"
 #include "kernels_fx.cuh"
@@ -28,15 +28,6 @@ template <typename R>
 __global__ void __launch_bounds__(256) k_ghost_state(Geom g, Phys ph, StencilFields<R> f, const double* scal) {
     const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (t < ghost_count(g)) ghost_state_cell<R>(g, ph, f, scal, t);
-}
-
-template <typename R, int V>
-__global__ void __launch_bounds__(128) k_grad(Geom g, CoefT<R> cf, const R* __restrict__ u, const R* __restrict__ v,
-                                              const R* __restrict__ w, GradOut<R> o, int own) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.mx || j >= g.my) return;
-    grad_point<R, V, sizeof(R) == 4>(g, cf, u, v, w, o, i, j, (int)blockIdx.z, own != 0);
 }
 
 // FP32-RHS dilatation from the packed records (rho, u, v, w), marching in z: blocks of
@@ -215,8 +206,7 @@ __global__ void __launch_bounds__(256) k_pack(Geom g, const T* __restrict__ src,
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         const unsigned tt = (unsigned)t, jk = tt / mx;
         const T x = src[g.at((int)(tt - jk * mx), (int)(jk % my), (int)(jk / my))];
-        if constexpr (is_ff<T>) dst[t] = ff_to_d(x);
-        else dst[t] = (double)x;
+        dst[t] = (double)x;
     }
 }
 
@@ -242,16 +232,6 @@ void launch_ghost_state(const Geom& g, const Phys& ph, const StencilFields<R>& f
 template <typename R>
 void launch_ghost_scalar(const Geom& g, R* f, cudaStream_t s) {
     k_ghost_scalar<R><<<ghost_blocks(g), 256, 0, s>>>(g, f);
-}
-template <typename R>
-void launch_grad(int V, const Geom& g, const CoefT<R>& cf, const R* u, const R* v, const R* w, const GradOut<R>& o,
-                 int own, cudaStream_t s) {
-    switch (V) {
-    case 1: k_grad<R, 1><<<point_grid(g), point_block(), 0, s>>>(g, cf, u, v, w, o, own); break;
-    case 2: k_grad<R, 2><<<point_grid(g), point_block(), 0, s>>>(g, cf, u, v, w, o, own); break;
-    case 3: k_grad<R, 3><<<point_grid(g), point_block(), 0, s>>>(g, cf, u, v, w, o, own); break;
-    default: k_grad<R, 4><<<point_grid(g), point_block(), 0, s>>>(g, cf, u, v, w, o, own); break;
-    }
 }
 void launch_dil_packed(int V, const Geom& g, const CoefT<float>& cf, const float4* qa, float* dil, int own,
                        cudaStream_t s) {
@@ -312,15 +292,5 @@ void launch_pack(const Geom& g, const T* src, double* dst, cudaStream_t s) {
 CNS_INST(double)
 CNS_INST(float)
 template void launch_ghost_scalar<long long>(const Geom&, long long*, cudaStream_t);
-// pair mode (FP32-pair RHS arithmetic): the stencil-input kernels and the RHS output
-template void launch_state<ff>(const Geom&, const Phys&, const StateIn&, const DerivedOut<ff>&, double*, int, double*,
-                               long long, cudaStream_t);
-template void launch_ghost_state<ff>(const Geom&, const Phys&, const StencilFields<ff>&, const double*, cudaStream_t);
-template void launch_ghost_scalar<ff>(const Geom&, ff*, cudaStream_t);
-template int launch_reduce<ff>(const Geom&, const Phys&, const StateIn&, const ff*, int, double*, int, double*, double*,
-                               cudaStream_t);
-template void launch_pack<ff>(const Geom&, const ff*, double*, cudaStream_t);
-template void launch_grad<ff>(int, const Geom&, const CoefT<ff>&, const ff*, const ff*, const ff*, const GradOut<ff>&,
-                              int, cudaStream_t);
 
 }  // namespace cns

@@ -43,17 +43,11 @@ __device__ __forceinline__ void state_store(const Phys& ph, const DerivedOut<R>&
         const double pr = rr * RT;
         const double hh = er + RT;
         const double suth = ph.vexp_is_one ? T : pow_visc(T, ph.vexp);
-        if constexpr (is_ff<R>) {   // the pair mode's stencil inputs include rho, u, v, w
-            o.r[c] = d_to_ff(rr);
-            o.u[c] = d_to_ff(uu);
-            o.v[c] = d_to_ff(vv);
-            o.w[c] = d_to_ff(ww);
-        }
-        o.t[c] = to_r<R>(T);
-        o.p[c] = to_r<R>(pr);
-        o.h[c] = to_r<R>(hh);
-        o.m[c] = to_r<R>(suth * ph.invRe);
-        if constexpr (!is_ff<R>) fx_track(o.gmax, {rr, uu, vv, ww, T, pr, hh, suth * ph.invRe});
+        o.t[c] = T;
+        o.p[c] = pr;
+        o.h[c] = hh;
+        o.m[c] = suth * ph.invRe;
+        fx_track(o.gmax, {rr, uu, vv, ww, T, pr, hh, suth * ph.invRe});
         if (!positive_bits(T) || !positive_bits(rr)) scal[SC_NONFINITE] = 1.0;   // racy flag write, any writer is fine
     }
 }
@@ -205,9 +199,9 @@ __device__ __forceinline__ void ghost_state_cell(const Geom& g, const Phys& ph, 
         return;
     }
     R* F[8] = {f.r, f.u, f.v, f.w, f.t, f.p, f.h, f.m};
-    // FP64 mode: ghosts that are no copies of interior values join the maxima; the next
-    // state's slots start at zero (its writer runs after this phase)
-    constexpr bool FX = !is_ff<R> && sizeof(R) == 8;
+    // ghosts that are no copies of interior values join the maxima; the next state's slots
+    // start at zero (its writer runs after this phase)
+    constexpr bool FX = sizeof(R) == 8;
     if (FX && t < 8) f.gnext[t] = 0u;
     const GhostCell gc = ghost_cell_of(g, t);
     const int m = gc.m, side = gc.side;
@@ -216,7 +210,6 @@ __device__ __forceinline__ void ghost_state_cell(const Geom& g, const Phys& ph, 
         const int j = gc.j, k = gc.k;
         cg = g.at(side == 0 ? -m : g.mx - 1 + m, j, k);
         if (g.xbc != XBC_PER) {
-            // in FP64 (the pair mode converts the interior values and the results)
             const long long cp = g.at(side == 0 ? m - 1 : g.mx - m, j, k);
             const auto rd = [&](const R* a, long long e) { return to_d<R>(a[e]); };
             double ug, vg, wg, pg, Tg;
@@ -351,47 +344,9 @@ __device__ __forceinline__ void ghost_vel_cell(const Geom& g, const Phys& ph, do
     for (int q = 0; q < 3; q++) F[q][cg] = val[q];
 }
 
-// ---------------------------------------------------------------------------------
-// Velocity gradients gij[0..8] = d(u,v,w)/d(x,y,z) at the viscous order and the
-// dilatation (derVelX/Y/Z + calcDil, src/calc_stress.cu:20-63,87-96).
-// ---------------------------------------------------------------------------------
-// DIL_ONLY: only the three diagonal gradients and theta (the FP32-RHS kernel forms the nine
-// gradients itself from the velocity stencils it loads, and needs theta at its neighbours).
-// own: also write the dilatation's ghost images (dil_ghost_owner; periodic and wall x,
-// periodic z only).
-template <typename R, int V, bool DIL_ONLY = false>
-__device__ __forceinline__ void grad_point(const Geom& g, const CoefT<R>& cf, const R* __restrict__ u,
-                                           const R* __restrict__ v, const R* __restrict__ w, const GradOut<R>& o,
-                                           int i, int j, int k, bool own = false) {
-    const long long c = g.at(i, j, k);
-    const long long st[3] = {1, g.P, g.PS};
-    const R* F[3] = {u, v, w};
-    R out[9];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            if (DIL_ONLY && q != d) continue;
-            const R* f = F[q];
-            R s = cf.c1V[d][1] * (__ldg(f + c + st[d]) - __ldg(f + c - st[d]));
-#pragma unroll
-            for (int kk = 2; kk <= V; kk++)
-                s = fma(cf.c1V[d][kk], __ldg(f + c + kk * st[d]) - __ldg(f + c - kk * st[d]), s);
-            if (d == 0 && g.nonuniform_x) s *= cf.xp[i];
-            out[3 * d + q] = s;
-        }
-    }
-    if constexpr (!DIL_ONLY) {
-#pragma unroll
-        for (int q = 0; q < 9; q++) o.g[q][c] = out[q];
-    }
-    const R th = out[0] + out[4] + out[8];
-    o.dil[c] = th;
-    if (own) dil_ghost_owner<R>(g, o.dil, c, i, j, k, th);
-}
-
 // FP32-RHS dilatation from the packed records qa = (rho, u, v, w): the diagonal gradients
-// du/dx, dv/dy, dw/dz at the viscous order (grad_point's DIL_ONLY arithmetic) and theta.
+// du/dx, dv/dy, dw/dz at the viscous order (derVelX/Y/Z, src/calc_stress.cu:20-63) and theta
+// (calcDil, src/calc_stress.cu:87-96).
 template <int V>
 __device__ __forceinline__ void dil_point_packed(const Geom& g, const CoefT<float>& cf,
                                                  const float4* __restrict__ qa, float* __restrict__ dil, int i, int j,
@@ -421,7 +376,7 @@ __device__ __forceinline__ void dil_point_packed(const Geom& g, const CoefT<floa
 // edges also load the x and y halos; the next plane's loads are issued before the current
 // plane is computed. About 2 + 2V/TY + 2V/32 record loads per point instead of the 6V of a
 // point-per-thread stencil (each record is 16 bytes of which one value is used); the
-// arithmetic per point is grad_point's (DIL_ONLY): the same sums in the same order. Tile
+// arithmetic per point is dil_point_packed's: the same sums in the same order. Tile
 // slots outside [-V, mx + V) x [-V, my + V) are never read by an interior point and are not
 // loaded; every loaded slot lies in the ghosted allocation (G = S >= V). All threads of the
 // block call it (it synchronises the block).

@@ -24,270 +24,6 @@
 
 namespace cns {
 
-template <typename R>
-__device__ __forceinline__ R ld(const R* __restrict__ p, int o) { return __ldg(p + o); }
-
-// Neighbours of the centre point along one direction, in global memory at a stride.
-//
-// Element offsets are 32-bit: every padded field holds fewer than 2^31 elements (checked
-// when a solver is created), and 64-bit offset arithmetic costs two integer instructions
-// per neighbour address.
-template <typename R>
-struct NbGlobal {
-    const RhsIn<R>* in;
-    int c, st;
-    __device__ __forceinline__ R u(int l) const { return ld(in->u, c + l * st); }
-    __device__ __forceinline__ R v(int l) const { return ld(in->v, c + l * st); }
-    __device__ __forceinline__ R w(int l) const { return ld(in->w, c + l * st); }
-    __device__ __forceinline__ R r(int l) const { return ld(in->r, c + l * st); }
-    __device__ __forceinline__ R h(int l) const { return ld(in->h, c + l * st); }
-    __device__ __forceinline__ R p(int l) const { return ld(in->p, c + l * st); }
-    __device__ __forceinline__ R t(int l) const { return ld(in->t, c + l * st); }
-    __device__ __forceinline__ R m(int l) const { return ld(in->m, c + l * st); }
-    __device__ __forceinline__ R dil(int l) const { return ld(in->dil, c + l * st); }
-};
-
-// first derivative sum_k co[k] (f_k - f_-k) and second derivative co[0] f_0 +
-// sum_k co[k] (f_k + f_-k) of the values get(l), l = -K..K
-template <typename R, int K, class Get>
-__device__ __forceinline__ R d1(const Get& get, const R* co) {
-    R s = co[1] * (get(1) - get(-1));
-#pragma unroll
-    for (int k = 2; k <= K; k++) s = fma(co[k], get(k) - get(-k), s);
-    return s;
-}
-
-template <typename R, int K, class Get>
-__device__ __forceinline__ R d2u(const Get& get, const R* co) {
-    R s = co[0] * get(0);
-#pragma unroll
-    for (int k = 1; k <= K; k++) s = fma(co[k], get(k) + get(-k), s);
-    return s;
-}
-
-// non-uniform x second derivative with the per-point table (derDevSharedV2x, nonUniformX)
-template <typename R, int V, class Get>
-__device__ __forceinline__ R d2x_nu(const Get& get, const R* __restrict__ cvsx, int mx, int i) {
-    R s = (R)0;
-#pragma unroll
-    for (int it = 0; it < 2 * V + 1; it++) s = fma(__ldg(cvsx + it * mx + i), get(it - V), s);
-    return s;
-}
-
-// f(a[k]) for k = 0, 1, 2 of a register array, with k a literal after inlining or uniform
-// at run time: branches, no indexed (local-memory) access
-template <typename T, int N, class F>
-__device__ __forceinline__ void at3(T (&a)[N], int k, F f) {
-    if (k == 0) f(a[0]); else if (k == 1) f(a[1]); else f(a[2]);
-}
-
-// FP64 body: contribution of direction DIR (deviceRHSX/Y/Z) on the separate stencil fields.
-// Terms that every direction multiplies by the same centre value are summed over the
-// directions first and multiplied once per point (rhs_point_nb): the second derivatives of
-// u, v, w, T in L[] (times mu), the viscous momentum terms grad mu . s + mu/3 grad theta in
-// W[] (the energy equation's work u_i W_i), the conduction in cond (times lambda/mu), and
-// the mass flux, whose half carries the centre value of the four cubic fluxes. The stress
-// row tau_{DIR,c}/mu comes from rhs_point_nb, which forms the symmetric tensor once. The
-// direction is an argument: called with a literal it folds like a template parameter; the
-// pair type calls it in a loop that is not unrolled (rhs_point_nb).
-// (The FP32-RHS mode has its own body on the packed records, rhs_dir_packed below.)
-template <typename R, int S, int V, bool MAYBE_X, class NB>
-__device__ __forceinline__ void rhs_direction(const Geom& g, const CoefT<R>& cf, const NB& nb, int i, const int DIR,
-                                              const R (&tau)[3], R m3, R u0, R v0, R w0, R r0, R (&acc)[5],
-                                              R (&W)[3], R (&L)[4], R& cond) {
-    const bool nux = MAYBE_X && DIR == 0 && g.nonuniform_x;   // MAYBE_X false: y or z (folds)
-    const R xpi = nux ? cf.xp[i] : (R)1;
-    const R* c1V = cf.c1V[DIR];
-    const R* c1S = cf.c1S[DIR];
-    const R* c2V = cf.c2V[DIR];
-
-    // velocity stencils, loaded once for the viscous second derivatives and the fluxes
-    R us[2 * S + 1], vs[2 * S + 1], ws[2 * S + 1];
-    us[S] = u0; vs[S] = v0; ws[S] = w0;
-#pragma unroll
-    for (int l = 1; l <= S; l++) {
-        us[S + l] = nb.u(l); us[S - l] = nb.u(-l);
-        vs[S + l] = nb.v(l); vs[S - l] = nb.v(-l);
-        ws[S + l] = nb.w(l); ws[S - l] = nb.w(-l);
-    }
-    // d mu/dx s_{DIR,c}; the second derivatives d2 u_c/dx2 continue the sums L[]
-    const auto gm = [&](int l) { return nb.m(l); };
-    const auto gt = [&](int l) { return nb.t(l); };
-    const auto gd = [&](int l) { return nb.dil(l); };
-    const auto gp = [&](int l) { return nb.p(l); };
-    const R dmu = d1<R, V>(gm, c1V) * xpi;
-    if (nux) {
-#pragma unroll
-        for (int it = 0; it < 2 * V + 1; it++) {
-            const R cw = __ldg(cf.cvsx + it * g.mx + i);
-            L[0] = fma(cw, us[S + it - V], L[0]);
-            L[1] = fma(cw, vs[S + it - V], L[1]);
-            L[2] = fma(cw, ws[S + it - V], L[2]);
-            L[3] = fma(cw, nb.t(it - V), L[3]);
-        }
-    } else {
-        L[0] = fma(c2V[0], us[S], L[0]);
-        L[1] = fma(c2V[0], vs[S], L[1]);
-        L[2] = fma(c2V[0], ws[S], L[2]);
-        L[3] = fma(c2V[0], nb.t(0), L[3]);
-#pragma unroll
-        for (int k = 1; k <= V; k++) {
-            L[0] = fma(c2V[k], us[S + k] + us[S - k], L[0]);
-            L[1] = fma(c2V[k], vs[S + k] + vs[S - k], L[1]);
-            L[2] = fma(c2V[k], ws[S + k] + ws[S - k], L[2]);
-            L[3] = fma(c2V[k], nb.t(k) + nb.t(-k), L[3]);
-        }
-    }
-    W[0] = fma(tau[0], dmu, W[0]);
-    W[1] = fma(tau[1], dmu, W[1]);
-    W[2] = fma(tau[2], dmu, W[2]);
-    // heat conduction lambda d2T + dlambda dT = (lambda/mu) (mu d2T + dmu dT); mu d2T and
-    // the ratio are applied once per point
-    const R dt = d1<R, V>(gt, c1V) * xpi;
-    cond = fma(dt, dmu, cond);
-    // mu/3 d(theta) on the DIR momentum (and its work), pressure gradient
-    const R dth = d1<R, V>(gd, c1V) * xpi;
-    const R dp = d1<R, S>(gp, c1S) * xpi;
-    at3(W, MAYBE_X ? DIR : (DIR == 1 ? 1 : 2), [&](R& w) { w = fma(m3, dth, w); });
-
-    // split-form convective derivatives, telescoped (see file comment); with a uniform
-    // spacing the flux weights already carry 1/2 or 1/4 and 1/dx, so they accumulate
-    // straight into the RHS. With Q-(l) = (rho_{-l}+rho_0)(g_{-l}+g_0) and
-    // Q+(l) = (rho_0+rho_l)(g_0+g_l), the cubic flux of phi is
-    //   sum_l a_l [Q-(phi_{-l}+phi_0) - Q+(phi_0+phi_l)]
-    //     = sum_l [(a_l Q-) phi_{-l} - (a_l Q+) phi_l]  +  phi_0 sum_l a_l (Q- - Q+),
-    // and the last sum is half the mass flux, so the products a_l Q+- are shared by the four
-    // cubic fluxes. The phi_0 terms of all directions are added from the summed mass flux
-    // once per point.
-    // The mass flux weights are twice the cubic ones (fq = 0.5 c1S, fc = 0.25 c1S: exactly
-    // 2 fc), so the mass flux is 2 sum_l (a_l Q- - a_l Q+); a_l Q+- = (a_l rho_0 + a_l rho_+-)
-    // (g_+- + g_0) with a_l rho_0 shared by the two: 17 operations per l.
-    const R un = (MAYBE_X && DIR == 0) ? u0 : (DIR == 1 ? v0 : w0);
-    R sd = (R)0, fu = nux ? (R)0 : acc[1], fv = nux ? (R)0 : acc[2], fw = nux ? (R)0 : acc[3],
-      fe = nux ? (R)0 : acc[4];
-    const R* fcb = cf.fc[DIR];
-#pragma unroll
-    for (int l = 1; l <= S; l++) {
-        const R rm = nb.r(-l), rp = nb.r(l);
-        const R um = us[S - l], up = us[S + l];
-        const R vm = vs[S - l], vp = vs[S + l];
-        const R wm = ws[S - l], wp = ws[S + l];
-        const R hm = nb.h(-l), hp = nb.h(l);
-        const R gm = (MAYBE_X && DIR == 0) ? um : (DIR == 1 ? vm : wm);
-        const R gp = (MAYBE_X && DIR == 0) ? up : (DIR == 1 ? vp : wp);
-        const R ar0 = fcb[l] * r0;
-        const R am = fma(fcb[l], rm, ar0) * (gm + un);
-        const R ap = fma(fcb[l], rp, ar0) * (un + gp);
-        sd += am - ap;
-        fu = fma(am, um, fma(-ap, up, fu));
-        fv = fma(am, vm, fma(-ap, vp, fv));
-        fw = fma(am, wm, fma(-ap, wp, fw));
-        fe = fma(am, hm, fma(-ap, hp, fe));
-    }
-    const R fr = nux ? sd + sd : fma((R)2, sd, acc[0]);
-    if (nux) {
-        acc[0] = fma(xpi, fr, acc[0]);
-        acc[1] = fma(xpi, fu, acc[1]);
-        acc[2] = fma(xpi, fv, acc[2]);
-        acc[3] = fma(xpi, fw, acc[3]);
-        acc[4] = fma(xpi, fe, acc[4]);
-    } else {
-        acc[0] = fr; acc[1] = fu; acc[2] = fv; acc[3] = fw; acc[4] = fe;
-    }
-    if (MAYBE_X && DIR == 0) acc[1] -= dp; else if (DIR == 1) acc[2] -= dp; else acc[3] -= dp;
-}
-
-// Pair-type body of one direction: the sums of rhs_direction in one pass over the offsets
-// l = 1..S that is not unrolled (the pair arithmetic is ~15 instructions per operation, and
-// the unrolled body does not fit the instruction caches). At each l it loads the neighbours
-// on either side and feeds every sum that needs them; each sum keeps rhs_direction's terms
-// and order (centre term, then l ascending; the stretched-x second derivative adds the pair
-// (-l, l) per l) in an accumulator whose tail is normalised once at the end, two sums at a
-// time through the packed FP32x2 forms (ffacc2, ff.cuh).
-template <int S, int V, bool MAYBE_X>
-__device__ __forceinline__ void rhs_dir_pair(const Geom& g, const CoefT<ff>& cf, const NbGlobal<ff>& nb, int i,
-                                             const int DIR, const ff (&tau)[3], ff m3, ff u0, ff v0, ff w0, ff r0,
-                                             ff (&acc)[5], ff (&W)[3], ff (&L)[4], ff& cond) {
-    const bool nux = MAYBE_X && DIR == 0 && g.nonuniform_x;
-    const ff t0 = nb.t(0);
-    {   // centre terms of the second derivatives
-        const ff cw = nux ? __ldg(cf.cvsx + V * g.mx + i) : cf.c2V[DIR][0];
-        const ff2 cw2 = mk2(cw, cw);
-        const ff2 luv = fma(cw2, mk2(u0, v0), mk2(L[0], L[1])), lwt = fma(cw2, mk2(w0, t0), mk2(L[2], L[3]));
-        L[0] = lane0(luv); L[1] = lane1(luv); L[2] = lane0(lwt); L[3] = lane1(lwt);
-    }
-    const ff un = (MAYBE_X && DIR == 0) ? u0 : (DIR == 1 ? v0 : w0);
-    const ff zero(0);
-    const ff2 zero2 = mk2(zero, zero), un2 = mk2(un, un);
-    // lanes: (p, theta), (mu, T), (L_u, L_v), (L_w, L_T), (F_u, F_v), (F_w, F_e), and the mass
-    // flux as (sum a_l Q-, -sum a_l Q+)
-    ffacc2 Dpth(zero2), Dmt(zero2), Luv(mk2(L[0], L[1])), Lwt(mk2(L[2], L[3])), Sd(zero2);
-    ffacc2 Fuv(nux ? zero2 : mk2(acc[1], acc[2])), Fwe(nux ? zero2 : mk2(acc[3], acc[4]));
-#pragma unroll 1
-    for (int l = 1; l <= S; l++) {
-        const ff um = nb.u(-l), up = nb.u(l), vm = nb.v(-l), vp = nb.v(l), wm = nb.w(-l), wp = nb.w(l);
-        // theta's weight is zero beyond the viscous half-width (its ghosts hold finite values)
-        Dpth.add_prod(mk2(cf.c1S[DIR][l], l <= V ? cf.c1V[DIR][l] : zero),
-                      mk2(nb.p(l), nb.dil(l)) - mk2(nb.p(-l), nb.dil(-l)));
-        if (l <= V) {
-            const ff c1 = cf.c1V[DIR][l];
-            const ff tm = nb.t(-l), tp = nb.t(l);
-            Dmt.add_prod(mk2(c1, c1), mk2(nb.m(l), tp) - mk2(nb.m(-l), tm));
-            if (nux) {
-                const ff cm = __ldg(cf.cvsx + (V - l) * g.mx + i), cp = __ldg(cf.cvsx + (V + l) * g.mx + i);
-                const ff2 cm2 = mk2(cm, cm), cp2 = mk2(cp, cp);
-                Luv.add_prod(cm2, mk2(um, vm)); Luv.add_prod(cp2, mk2(up, vp));
-                Lwt.add_prod(cm2, mk2(wm, tm)); Lwt.add_prod(cp2, mk2(wp, tp));
-            } else {
-                const ff c2 = cf.c2V[DIR][l];
-                const ff2 c22 = mk2(c2, c2);
-                Luv.add_prod(c22, mk2(up, vp) + mk2(um, vm));
-                Lwt.add_prod(c22, mk2(wp, tp) + mk2(wm, tm));
-            }
-        }
-        // telescoped split-form fluxes (rhs_direction): lanes (a_l Q-, a_l Q+)
-        const ff gm = (MAYBE_X && DIR == 0) ? um : (DIR == 1 ? vm : wm);
-        const ff gp = (MAYBE_X && DIR == 0) ? up : (DIR == 1 ? vp : wp);
-        const ff fc = cf.fc[DIR][l];
-        const ff ar0 = fc * r0;
-        const ff2 q = fma(mk2(fc, fc), mk2(nb.r(-l), nb.r(l)), mk2(ar0, ar0)) * (mk2(gm, gp) + un2);
-        const float2 sgn = make_float2(1.0f, -1.0f);   // (a_l Q-, -a_l Q+), exact
-        const ff2 qs = ff2{__fmul2_rn(q.h, sgn), __fmul2_rn(q.l, sgn)};
-        Sd.add(qs);
-        const ff2 am2 = mk2(lane0(qs), lane0(qs)), ap2 = mk2(lane1(qs), lane1(qs));
-        Fuv.add_prod(am2, mk2(um, vm)); Fuv.add_prod(ap2, mk2(up, vp));
-        Fwe.add_prod(am2, mk2(wm, nb.h(-l))); Fwe.add_prod(ap2, mk2(wp, nb.h(l)));
-    }
-    const ff2 luv = Luv.value(), lwt = Lwt.value(), pth = Dpth.value(), mt = Dmt.value();
-    const ff2 s2 = Sd.value(), fuv = Fuv.value(), fwe = Fwe.value();
-    L[0] = lane0(luv); L[1] = lane1(luv); L[2] = lane0(lwt); L[3] = lane1(lwt);
-    ff dmu = lane0(mt), dt = lane1(mt), dth = lane1(pth), dp = lane0(pth);
-    const ff sd = lane0(s2) + lane1(s2);
-    if (nux) {
-        const ff xpi = cf.xp[i];
-        const ff2 x2 = mk2(xpi, xpi), a = mt * x2, b = pth * x2;
-        dmu = lane0(a); dt = lane1(a); dp = lane0(b); dth = lane1(b);
-    }
-    {   // W_q += tau_q dmu, cond += dT dmu (two packed multiply-adds)
-        const ff2 d2 = mk2(dmu, dmu);
-        const ff2 w01 = fma(mk2(tau[0], tau[1]), d2, mk2(W[0], W[1])), w2c = fma(mk2(tau[2], dt), d2, mk2(W[2], cond));
-        W[0] = lane0(w01); W[1] = lane1(w01); W[2] = lane0(w2c); cond = lane1(w2c);
-    }
-    at3(W, MAYBE_X ? DIR : (DIR == 1 ? 1 : 2), [&](ff& w) { w = fma(m3, dth, w); });
-    const ff fr = nux ? sd + sd : fma(ff(2), sd, acc[0]);
-    if (nux) {
-        const ff xpi = cf.xp[i];
-        const ff2 x2 = mk2(xpi, xpi);
-        const ff2 a01 = fma(x2, mk2(fr, lane0(fuv)), mk2(acc[0], acc[1]));
-        const ff2 a23 = fma(x2, mk2(lane1(fuv), lane0(fwe)), mk2(acc[2], acc[3]));
-        acc[0] = lane0(a01); acc[1] = lane1(a01); acc[2] = lane0(a23); acc[3] = lane1(a23);
-        acc[4] = fma(xpi, lane1(fwe), acc[4]);
-    } else {
-        acc[0] = fr; acc[1] = lane0(fuv); acc[2] = lane1(fuv); acc[3] = lane0(fwe); acc[4] = lane1(fwe);
-    }
-    if (MAYBE_X && DIR == 0) acc[1] -= dp; else if (DIR == 1) acc[2] -= dp; else acc[3] -= dp;
-}
-
 // Body force, sponge, stage update and the new state's recovery of the point at element
 // c, given its RHS accumulators acc (convective, pressure and viscous terms) and centre
 // values u0, v0, w0, r0 in the arithmetic type R
@@ -302,13 +38,12 @@ __device__ __forceinline__ void stage_tail(const Geom& g, const Update<R>& up, d
     if (up.spx) {
         const R sg = to_r<R>(up.spx[i] + up.spz[k]);
         const long long i2 = (long long)i + (long long)k * g.mx;
-        if constexpr (sizeof(R) == 8) {   // FP64 (and the pair type: the term in FP64, then split)
-            const double sgd = up.spx[i] + up.spz[k];
-            acc[0] += to_r<R>(sgd * (up.rref[i2] - rr));
-            acc[1] += to_r<R>(sgd * (up.uref[i2] - rr * uu));
-            acc[2] += to_r<R>(sgd * (up.vref[i2] - rr * vv));
-            acc[3] += to_r<R>(sgd * (up.wref[i2] - rr * ww));
-            acc[4] += to_r<R>(sgd * (up.eref[i2] - ee));
+        if constexpr (sizeof(R) == 8) {
+            acc[0] += sg * (up.rref[i2] - rr);
+            acc[1] += sg * (up.uref[i2] - rr * uu);
+            acc[2] += sg * (up.vref[i2] - rr * vv);
+            acc[3] += sg * (up.wref[i2] - rr * ww);
+            acc[4] += sg * (up.eref[i2] - ee);
         } else {
             acc[0] += sg * (to_r<R>(up.rref[i2]) - r0);
             acc[1] += sg * (to_r<R>(up.uref[i2]) - r0 * u0);
@@ -393,66 +128,6 @@ __device__ __forceinline__ void stage_tail(const Geom& g, const Update<R>& up, d
     // the next stage's state recovery from the values in registers (bit for bit the state
     // kernel's result on the stored state)
     if (up.fuse) state_store<R>(up.ph, up.dnext, scal, c, qn[0], inv, un, vn, wn, qn[4]);
-}
-
-// FP64 RHS + stage update of one interior point (i, ., k) at element c, with the neighbours
-// along x, y, z from the accessors nx, ny, nz and the centre values given
-template <typename R, int S, int V, class NX, class NY, class NZ>
-__device__ __forceinline__ void rhs_point_nb(const Geom& g, const CoefT<R>& cf, const RhsIn<R>& in,
-                                             const Update<R>& up, double* __restrict__ scal, int quirk, int i,
-                                             int k, int c, const NX& nx, const NY& ny, const NZ& nz, R th0,
-                                             R m0, R u0, R v0, R w0, R r0, R h0) {
-    R Gr[9];   // the gradient kernel's fields, Gr[3 a + b] = d u_b / d x_a
-#pragma unroll
-    for (int q = 0; q < 9; q++) Gr[q] = ld(in.g[q], c);
-    // the stress tensor tau / mu (uXtmp, vXtmp, wXtmp of deviceRHSX and its y/z twins) and
-    // the viscous dissipation tau_ab d u_b / d x_a / mu; an off-diagonal pair contributes
-    // tau_ab (d u_b/d x_a + d u_a/d x_b) = tau_ab^2, except y-z with the quirk
-    // (cuda_rhs.cu:175: tau_yz dv/dz in the y sum as in the z sum)
-    const R th23 = (R)(2. / 3.) * th0;
-    const R t00 = fma((R)2, Gr[0], -th23), t11 = fma((R)2, Gr[4], -th23), t22 = fma((R)2, Gr[8], -th23);
-    const R t01 = Gr[1] + Gr[3], t02 = Gr[2] + Gr[6], t12 = Gr[5] + Gr[7];
-    const R q12 = quirk ? Gr[7] + Gr[7] : t12;
-    const R diss = fma(t00, Gr[0], fma(t11, Gr[4], fma(t22, Gr[8], fma(t01, t01, fma(t02, t02, t12 * q12)))));
-    const R tx[3] = {t00, t01, t02}, ty[3] = {t01, t11, t12}, tz[3] = {t02, t12, t22};
-    const R m3 = m0 * (R)(1.0 / 3.0);
-    R acc[5] = {0, 0, 0, 0, 0};
-    R W[3] = {0, 0, 0};
-    R L[4] = {0, 0, 0, 0};
-    R cond = 0;
-    if constexpr (is_ff<R> && std::is_same<NX, NbGlobal<R>>::value && std::is_same<NY, NX>::value &&
-                  std::is_same<NZ, NX>::value) {
-        // the pair arithmetic is ~15 instructions per operation: x (with the stretched-grid
-        // terms) and one copy of the y / z body walked twice, each a loop over the offsets
-        // (rhs_dir_pair), keep the kernel's code within the instruction caches
-        rhs_dir_pair<S, V, true>(g, cf, nx, i, 0, tx, m3, u0, v0, w0, r0, acc, W, L, cond);
-#pragma unroll 1
-        for (int d = 1; d < 3; d++) {
-            const R td[3] = {d == 1 ? t01 : t02, d == 1 ? t11 : t12, d == 1 ? t12 : t22};
-            NX nb = ny;   // the accessors differ in their stride only
-            nb.st = d == 1 ? ny.st : nz.st;
-            rhs_dir_pair<S, V, false>(g, cf, nb, i, d, td, m3, u0, v0, w0, r0, acc, W, L, cond);
-        }
-    } else {
-        rhs_direction<R, S, V, true>(g, cf, nx, i, 0, tx, m3, u0, v0, w0, r0, acc, W, L, cond);
-        rhs_direction<R, S, V, false>(g, cf, ny, i, 1, ty, m3, u0, v0, w0, r0, acc, W, L, cond);
-        rhs_direction<R, S, V, false>(g, cf, nz, i, 2, tz, m3, u0, v0, w0, r0, acc, W, L, cond);
-    }
-    // the centre values of the cubic fluxes: phi_0 times half the mass flux
-    const R half = (R)0.5 * acc[0];
-    acc[1] = fma(u0, half, acc[1]);
-    acc[2] = fma(v0, half, acc[2]);
-    acc[3] = fma(w0, half, acc[3]);
-    acc[4] = fma(h0, half, acc[4]);
-#pragma unroll
-    for (int q = 0; q < 3; q++) W[q] = fma(m0, L[q], W[q]);
-    cond = fma(m0, L[3], cond);
-    acc[1] += W[0];
-    acc[2] += W[1];
-    acc[3] += W[2];
-    acc[4] += fma(m0, diss, cf.lam_mu * cond) + fma(u0, W[0], fma(v0, W[1], w0 * W[2]));
-
-    stage_tail<R>(g, up, scal, i, k, c, acc, u0, v0, w0, r0);
 }
 
 // ---------------------------------------------------------------------------------
@@ -640,25 +315,20 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
                                           double* __restrict__ scal, int quirk, int i, int j, int k) {
     if constexpr (sizeof(R) == 4) {
         rhs_point_packed<S, V, CW>(g, cf, in, up, scal, quirk, i, j, k);
-    } else if constexpr (!is_ff<R>) {
+    } else {
         const int c = (int)g.at(i, j, k);
         const double u0 = up.qin.u[c], v0 = up.qin.v[c], w0 = up.qin.w[c];
         double acc[5];
         rhs_acc_fx<S, V>(g, cf.fx, in, quirk, i, c, u0, v0, w0, acc);
         stage_tail<double>(g, up, scal, i, k, c, acc, u0, v0, w0, up.qin.r[c]);
-    } else {
-        const int c = (int)g.at(i, j, k);
-        const R th0 = ld(in.dil, c), m0 = ld(in.m, c);
-        const R u0 = ld(in.u, c), v0 = ld(in.v, c), w0 = ld(in.w, c), r0 = ld(in.r, c), h0 = ld(in.h, c);
-        const NbGlobal<R> nx{&in, c, 1}, ny{&in, c, (int)g.P}, nz{&in, c, (int)g.PS};
-        rhs_point_nb<R, S, V>(g, cf, in, up, scal, quirk, i, k, c, nx, ny, nz, th0, m0, u0, v0, w0, r0, h0);
     }
 }
 
 // FP32: 7 blocks of 128 per SM (72 registers) measured fastest (6: 80 registers, +13 %
-// time; 5: 96 registers, and stages that read the RK register ran 3.5x slower); FP64: the
-// FP64 pipe bounds the kernel at 3 to 5 blocks alike; pairs: 4 blocks (122 registers)
-// 856 Mpoint-steps/s on the channel against 815 with 5 (96 registers)
+// time; 5: 96 registers, and stages that read the RK register ran 3.5x slower). FP64: 5 blocks
+// (96 registers): latency bound at 43 % issue, FP64 pipe 54 % busy; 4 blocks 1.14 ms, 6 blocks
+// 1.07 ms against 1.09 on the channel 128x160x192, but 6 (80 registers, spilling) 0.088 against
+// 0.081 ms on a 64^3 box.
 //
 // One launch covers the 4-row bands [band0, band0 + gridDim.y) of every plane; blocks are
 // dispatched x fastest, then bands, then planes. On large planes the bands are split into
@@ -666,7 +336,7 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
 // group's blocks sweep them (one launch over whole planes would cycle ~2S planes of the
 // inputs through L2 between their uses).
 template <typename R, int S, int V>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : is_ff<R> ? 4 : 5) k_rhs(Geom g, const __grid_constant__ CoefT<R> cf,
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 5) k_rhs(Geom g, const __grid_constant__ CoefT<R> cf,
                                                                                    const __grid_constant__ RhsIn<R> in, Update<R> up,
                                              double* __restrict__ scal, int quirk, int band0) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

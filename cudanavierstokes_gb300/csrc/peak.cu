@@ -4,6 +4,7 @@
 
 #include "../../include/cns.h"
 #include "cns_common.cuh"
+#include "ff.cuh"
 
 namespace {
 

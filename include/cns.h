@@ -67,9 +67,9 @@ extern "C" {
 #define CNS_PREC_FP64      0   /* plain FP64 everywhere, as the reference                */
 #define CNS_PREC_FP32_RHS  1   /* RHS in FP32; state, RK accumulation, T/p recovery and
                                   reductions in FP64                                     */
-#define CNS_PREC_PAIR_RHS  2   /* RHS in FP32-pair ("double-float", ~48-bit) arithmetic;
-                                  state, RK accumulation, T/p recovery and reductions
-                                  in FP64 (single solvers; batches take modes 0 and 1)   */
+#define CNS_PREC_PAIR_RHS  2   /* at least ~48-bit RHS arithmetic (FP32 pairs): served by the
+                                  FP64 mode's RHS, which is faster and more accurate on
+                                  this GPU (single solvers; batches take modes 0 and 1)  */
 
 /*
  * Runtime mirror of the reference's compile-time parameter surface
@@ -379,8 +379,8 @@ CNS_API int cns_selftest_pow(int device, const double* x, long long n, double a,
  * recovery) next to the IEEE division 1.0 / x on the same n <= 2^27 host values. */
 CNS_API int cns_selftest_rcp(int device, const double* x, long long n, double* fast, double* lib);
 
-/* Self test with no counterpart in the reference: the pair arithmetic of
- * CNS_PREC_PAIR_RHS on n <= 2^24 host triples (a, b, c), each first split into its nearest
+/* Self test with no counterpart in the reference: the FP32-pair arithmetic (ff.cuh)
+ * on n <= 2^24 host triples (a, b, c), each first split into its nearest
  * pair. out[(t * 15 + q) * 2 + {0, 1}] holds the two floats of result q of element t:
  * q = 0..2 the pairs of a, b, c; 3..6 a + b, a b, fma(a, b, c) and the compensated
  * accumulation c + a b; 7..10 the same four from the packed two-lane forms, lane 0 on
