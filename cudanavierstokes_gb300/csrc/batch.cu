@@ -90,7 +90,10 @@ struct cns_batch {
     unsigned long long* d_cnt = nullptr;   // the persistent kernel's four phase unit counters
     std::vector<BatchInst<float>> h_tab32;   // host copy of the FP32 member table (the launch argument's source)
     int* d_err = nullptr;
-    int threads = 128, blocks_per_sm = 1, nsm = 152;
+    // full residency unless a shape is set or tuned (choose_shape clamps it): 20 steps of 8
+    // FP32 boxes 32..128 take 42 ms with 7 blocks per SM, 115 ms with 1
+    int threads = 128, blocks_per_sm = 32, nsm = 152;
+    long long units = 0;                 // point units of all members
     bool tuned = false;
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
     int64_t launches = 0;
@@ -189,6 +192,8 @@ int upload_table(cns_batch* b) {
     BCK(cudaMemcpyAsync(b->d_tab, tab.data(), sizeof(BatchInst<R>) * n, cudaMemcpyHostToDevice, b->stream));
     BCK(cudaMemcpyAsync(b->d_ctl, &ctl, sizeof ctl, cudaMemcpyHostToDevice, b->stream));
     BCK(cudaStreamSynchronize(b->stream));
+    if (b->units != ctl.unit_off[n]) b->drop_graphs();   // the grid follows the units (launch_stage)
+    b->units = ctl.unit_off[n];
     if constexpr (sizeof(R) == 4) {
         // the member table is a launch argument, baked into the captured steps
         b->h_tab32.assign(tab.begin(), tab.begin() + n);
@@ -246,7 +251,9 @@ MemberTable<float> member_table(const cns_batch* b, int s, int cur) {
 }
 
 int launch_stage(cns_batch* b, int s, int cur) {
-    const dim3 grid(b->nsm * b->blocks_per_sm);
+    // no more blocks than units, in whole blocks per SM: idle blocks only lengthen the barriers
+    const long long need = (b->units + b->nsm - 1) / b->nsm;
+    const dim3 grid((unsigned)(b->nsm * std::min<long long>(b->blocks_per_sm, std::max<long long>(need, 1))));
     const bool f32 = b->precision == CNS_PREC_FP32_RHS;
     if (s == 0) {   // the step's time advance, before the stage reads the time
         if (f32) launch_batch_time_fp32((const BatchInst<float>*)b->d_tab, b->d_ctl, b->stream);
