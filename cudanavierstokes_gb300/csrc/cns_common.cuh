@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fx.cuh"
 #include "pow_tables.h"
 
 namespace cns {
@@ -203,7 +204,7 @@ __device__ __forceinline__ bool positive_bits(double x) {
 // pow, which runs on the FP64 pipe. The error of exp(y) is that of y, about |y| ulp, so it
 // serves |a ln x| < 1 (T^0.7 for 0.24 < T < 4.2, the temperatures of these flows), within a
 // few ulp of pow (a GPU test bounds it); other arguments take pow itself.
-__device__ __forceinline__ double pow_visc(double x, double a) {
+static __device__ __noinline__ double pow_tables(double x, double a) {
     const double INV_LN2_64 = 92.33248261689366, SHIFT = 6755399441055744.0;   // 64/ln2, 1.5 * 2^52
     if (!(x > 1e-300 && x < 1e300)) return pow(x, a);
     const unsigned hx = (unsigned)__double2hiint(x);
@@ -234,6 +235,52 @@ __device__ __forceinline__ double pow_visc(double x, double a) {
     const double th = __ldg(&kPowExpHi[ti]);
     const double res = th + fma(th, em1, __ldg(&kPowExpLo[ti]));
     return __hiloint2double(__double2hiint(res) + (int)((unsigned)e << 20), __double2loint(res));
+}
+
+// The same on the integer units for 1/4 <= x < 8, |a| < 2 and |a ln x| < 1, other arguments to
+// pow_tables: 135 integer instructions, one conversion and no FP64 arithmetic, where one FP64
+// instruction holds its pipe as long as ~60 of them (channel 128x160x192: RHS kernel with the
+// state recovery 1.078 -> 1.038 ms, ghost kernel 0.036 -> 0.028 ms).
+//   x = 2^k m, i = the top 6 fraction bits of m, R_i = 2^16 / c_i rounded to an integer: m R_i /
+//   2^16 = 1 + d with d 2^68 the product's low 64 bits, exactly (the 1 is 2^68); ln(1 + d) = d
+//   (1 - d/2 + ... - d^7/8), |d| < 2^-6.9; ln x in 2^-60, y = a ln x in 2^-59;
+//   exp y = 2^(j/64) exp(r), r = y - j ln2/64 in 2^-66 (the difference modulo 2^64), exp(r) - 1
+//   = r (1 + r/2 + ... + r^5/720), |r| < 2^-7.5.
+// Each level of the two series is held to the bits that reach the result, the last ones in 32
+// bits. Before its one rounding the result is within 0.04 ulp.
+__device__ __forceinline__ double pow_visc(double x, double a) {
+    const unsigned hx = (unsigned)__double2hiint(x);
+    const i64 A = fx_from(a, 1);   // a 2^61
+    const int k = (int)(hx >> 20) - 1023;
+    if (k < -2 || k > 2 || ((unsigned)__double2hiint(a) & 0x7fffffffu) >= 0x40000000u) return pow_tables(x, a);
+    const int i = (int)((hx >> 14) & 63u);
+    const int R = __ldg(&kFxRcp[i]);
+    const unsigned mh = (hx & 0x000fffffu) | 0x00100000u, ml = (unsigned)__double2loint(x);
+    const unsigned long long lo = (unsigned long long)ml * (unsigned)R;
+    const i64 D = (i64)(lo + ((unsigned long long)(mh * (unsigned)R) << 32));   // d 2^68
+    const auto mulhi = [](int u, int v) { return fx_word1(fx_mad(u, v, 0)); };
+    const int d = (int)(D >> 36);                                                // d 2^32
+    int q = 306783378 - mulhi(d, 268435456);                                     // 1/7 - d/8, in 2^-31
+    q = -357913941 + mulhi(d, q);                                                // -1/6
+    q = 429496730 + mulhi(d, q);                                                 // 1/5
+    q = -536870912 + mulhi(d, q);                                                // -1/4
+    const i64 A2 = 768614336404564651LL + (fx_mad((int)(D >> 31), q, 0) >> 7);   // 1/3, in 2^-61
+    const i64 A1 = -(1LL << 60) + (fx_mul(D, A2) >> 4);                          // -1/2
+    const i64 S = (1LL << 61) + (fx_mul(D, A1) >> 4);
+    const i64 L = (i64)k * FX_LN2 + __ldg(&kFxLn[i]) + (fx_mul(D, S) >> 5);
+    const i64 Y = fx_mul_by4(L, A);
+    if (fx_word1(Y) >= (1 << 27) || fx_word1(Y) < -(1 << 27)) return pow_tables(x, a);
+    const int j = fx_word1(fx_mad(fx_word1(Y), FX_64_LN2, 1LL << 48)) >> 17;
+    const i64 r = (i64)(((unsigned long long)Y << 7) - (unsigned long long)((i64)j * FX_LN2_64));
+    const int r32 = (int)(r >> 34);                                              // r 2^32
+    int g = 35791394 + mulhi(r32, 5965232);                                      // 1/120 + r/720, in 2^-32
+    g = 178956971 + mulhi(r32, g);                                               // 1/24
+    const i64 G2 = 384307168202282326LL + (fx_mad((int)(r >> 29), g, 0) >> 8);   // 1/6, in 2^-61
+    const i64 G1 = (1LL << 60) + (fx_mul(r, G2) >> 2);
+    const i64 G = (1LL << 61) + (fx_mul(r, G1) >> 2);
+    const i64 T = __ldg(&kFxExp[j & 63]);
+    const double res = (double)(T + 2 * fx_mul(T, fx_mul(r, G)));                // 2^62 .. 2^63
+    return __hiloint2double(__double2hiint(res) + (((j >> 6) - 62) << 20), __double2loint(res));
 }
 
 template <typename R> __device__ __forceinline__ R cns_pow(R a, R b);

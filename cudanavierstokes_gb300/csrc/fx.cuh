@@ -48,6 +48,13 @@ __device__ __forceinline__ i64 fx_mul(i64 a, i64 b) {
     return fx_mad(ah, bh, (i64)fx_word1(m));
 }
 
+// a b / 2^62, |a b| < 2^124.6
+__device__ __forceinline__ i64 fx_mul_by4(i64 a, i64 b) {
+    const int ah = fx_hi(a), al = fx_lo(a), bh = fx_hi(b), bl = fx_lo(b);
+    const i64 m = fx_mad(ah, bl, fx_mad(al, bh, FX_HALF / 4));
+    return (fx_mad(ah, bh, 0) << 2) + (m >> 30);
+}
+
 // sum of products a_k w_k / 2^32 with small-integer weights: two accumulators, the high
 // halves' and the low halves'. With |a| < 2^63 and sum |w| <= 2^30.8 both stay below 2^61.8.
 struct FxSum {

@@ -10,6 +10,14 @@ exact hexadecimal double literals.
   POW_LN2_64_HI / LO    ln(2)/64 split: hi with 40 significant bits (j * hi exact for
                         |j| < 2^13), lo the rest
 
+and the same in integers for its fixed-point form:
+
+  kFxRcp[i]             R_i = 2^16 / c_i rounded to an integer
+  kFxLn[i]              -ln(R_i / 2^16) 2^60
+  kFxExp[i]             2^(i/64) 2^62
+  FX_LN2, FX_LN2_64     ln(2) 2^60, ln(2)/64 2^66
+  FX_64_LN2             64/ln(2) 2^22
+
 Run from this directory: python gen_pow_tables.py > pow_tables.h
 """
 import mpmath
@@ -56,6 +64,19 @@ def main():
     for name, vals in (("kPowRcp", rcp), ("kPowLnHi", lnh), ("kPowLnLo", lnl), ("kPowExpHi", exh),
                        ("kPowExpLo", exl)):
         print(arr(name, vals))
+
+    def fixed(v, bits):
+        return int(mpmath.nint(mpmath.ldexp(v, bits)))
+
+    frcp = [fixed(1 / (1 + (mpmath.mpf(i) + mpmath.mpf("0.5")) / 64), 16) for i in range(64)]
+    fln = [fixed(-mpmath.log(mpmath.mpf(r) / 65536), 60) for r in frcp]
+    fexp = [fixed(mpmath.power(2, mpmath.mpf(i) / 64), 62) for i in range(64)]
+    print(f"constexpr long long FX_LN2 = {fixed(mpmath.log(2), 60)}LL;")
+    print(f"constexpr long long FX_LN2_64 = {fixed(mpmath.log(2) / 64, 66)}LL;")
+    print(f"constexpr int FX_64_LN2 = {fixed(64 / mpmath.log(2), 22)};\n")
+    for kind, name, vals in (("int", "kFxRcp", frcp), ("long long", "kFxLn", fln), ("long long", "kFxExp", fexp)):
+        body = ",\n".join("    " + ", ".join(str(v) for v in vals[k:k + 4]) for k in range(0, 64, 4))
+        print(f"static __device__ const {kind} {name}[64] = {{\n{body}}};\n")
 
 
 if __name__ == "__main__":

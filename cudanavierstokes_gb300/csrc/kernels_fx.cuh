@@ -338,13 +338,6 @@ __device__ __forceinline__ i64 fx_mulk(i64 v, i64 k) {
     return fx_mad(vh, kh, (i64)fx_word1(m));
 }
 
-// a b / 2^62, |a b| < 2^124.6
-__device__ __forceinline__ i64 fx_mul_by4(i64 a, i64 b) {
-    const int ah = fx_hi(a), al = fx_lo(a), bh = fx_hi(b), bl = fx_lo(b);
-    const i64 m = fx_mad(ah, bl, fx_mad(al, bh, FX_HALF / 4));
-    return (fx_mad(ah, bh, 0) << 2) + (m >> 30);
-}
-
 // sum of three products / 2^64, the low halves' products (below a quarter each) left out;
 // factors below 2^62 and 2^62: the cross sums < 2^62.6 in pairs of products
 __device__ __forceinline__ i64 fx_dot3(i64 a0, i64 b0, i64 a1, i64 b1, i64 a2, i64 b2) {
