@@ -7,6 +7,7 @@ namespace cns {
 
 constexpr int RED_THREADS = 256;
 constexpr int RED_BLOCKS = 1024;   // partial slots per reduced quantity
+constexpr int RED_PEAK = 0;        // the largest rate's slot (the sums start at RED_BLOCKS)
 enum { RED_DT = 1, RED_FORCE = 2, RED_ENERGY = 4, RED_KE = 8 };
 
 struct StateIn {

@@ -591,6 +591,7 @@ int cns_create(const cns_params* pin, int device, cns_solver** out) {
     for (int b = 0; b < 2; b++)
         for (int f = 0; f < 5; f++) CK(cudaMemsetAsync(h->q[b][f], 0, (size_t)h->nalloc * 8, h->stream));
     for (int f = 0; f < 5; f++) CK(cudaMemsetAsync(h->rb[f], 0, (size_t)h->nalloc * rs, h->stream));
+    CK(cudaMemsetAsync(h->part, 0, 6 * RED_BLOCKS * sizeof(double), h->stream));
     double sc[SC_COUNT] = {0};
     sc[SC_DPDZ] = p.forcing ? p.dpdz_init : 0.0;   // cuda_utils.cu:68-70
     CK(cudaMemcpyAsync(h->scal, sc, sizeof sc, cudaMemcpyHostToDevice, h->stream));
