@@ -292,8 +292,9 @@ __device__ __forceinline__ void dil_ghost_owner(const Geom& g, R* __restrict__ f
 }
 
 // Ghost cell t of the velocity alone (the u, v, w part of ghost_state_cell, for FP64
-// velocity fields whose other stencil inputs are not needed: the dissipation diagnostic)
-__device__ __forceinline__ void ghost_vel_cell(const Geom& g, const Phys& ph, double* u, double* v, double* w,
+// velocity fields whose other stencil inputs are not needed: the dissipation diagnostic);
+// returns its element
+__device__ __forceinline__ long long ghost_vel_cell(const Geom& g, const Phys& ph, double* u, double* v, double* w,
                                                const double* scal, int t) {
     double* F[3] = {u, v, w};
     const GhostCell gc = ghost_cell_of(g, t);
@@ -317,7 +318,7 @@ __device__ __forceinline__ void ghost_vel_cell(const Geom& g, const Phys& ph, do
                 wg = 2.0 * w[cl] - w[cm];
             }
             u[cg] = ug; v[cg] = vg; w[cg] = wg;
-            return;
+            return cg;
         }
         cs = g.at(side == 0 ? g.mx - m : m - 1, j, k);
     } else if (gc.face == 1) {
@@ -333,7 +334,7 @@ __device__ __forceinline__ void ghost_vel_cell(const Geom& g, const Phys& ph, do
             for (int q = 0; q < 3; q++) { a[q] = F[q][c0]; b[q] = F[q][cm]; }
 #pragma unroll
             for (int q = 0; q < 3; q++) F[q][cg] = 2.0 * a[q] - b[q];
-            return;
+            return cg;
         }
         cs = g.at(gc.i, gc.j, side == 0 ? g.mz - m : m - 1);
     }
@@ -342,6 +343,7 @@ __device__ __forceinline__ void ghost_vel_cell(const Geom& g, const Phys& ph, do
     for (int q = 0; q < 3; q++) val[q] = F[q][cs];
 #pragma unroll
     for (int q = 0; q < 3; q++) F[q][cg] = val[q];
+    return cg;
 }
 
 // FP32-RHS dilatation from the packed records qa = (rho, u, v, w): the diagonal gradients

@@ -54,6 +54,8 @@ struct cns_solver {
     void* k2[5] = {};            // classic RK3 k2 / RK4 accumulator (R)
     double* q0[5] = {};          // classic schemes: conserved state at the step start
     double* staging = nullptr;   // N doubles, host <-> device layout conversion
+    double* scratch = nullptr;   // of solver_scratch, scratch_n doubles
+    size_t scratch_n = 0;
     double* scal = nullptr;      // device scalars (SC_*)
     double* part = nullptr;      // reduction partials 5 * RED_BLOCKS
     double* diag = nullptr;      // per-step bulk diagnostics (2 per step)
@@ -149,6 +151,20 @@ inline void solver_set_parity(cns_solver* h, int want) {
     h->drop_graphs();
 }
 int solver_reduce(cns_solver* h, int want, double* diag);
+// n doubles of device scratch for the work of one call on h->stream: the copy staging, or,
+// where that is smaller (tiny grids), a buffer that the handle keeps
+inline int solver_scratch(cns_solver* h, size_t n, double** out) {
+    *out = h->staging;
+    if (n <= (size_t)h->p.mx * h->p.my * h->p.mz) return CNS_OK;
+    if (h->scratch_n < n) {
+        double* p = nullptr;
+        if (int rc = h->alloc(&p, n)) return rc;
+        h->scratch = p;
+        h->scratch_n = n;
+    }
+    *out = h->scratch;
+    return CNS_OK;
+}
 // stencil inputs (+ theta) of state buffer b
 template <typename R>
 RhsIn<R> solver_rhs_in(cns_solver* h, int b);
