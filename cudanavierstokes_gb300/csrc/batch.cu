@@ -39,6 +39,10 @@ void launch_batch_stage_fp32(int S, int V, dim3 grid, const BatchInst<float>* ta
                              const MemberTable<float>& rt, cudaStream_t s);
 void launch_batch_time_fp64(const BatchInst<double>* tab, const BatchCtl* ctl, cudaStream_t s);
 void launch_batch_time_fp32(const BatchInst<float>* tab, const BatchCtl* ctl, cudaStream_t s);
+cudaError_t launch_batch_status_fp64(const BatchInst<double>* tab, const BatchCtl* ctl, const int* err, int* status,
+                                     cudaStream_t s);
+cudaError_t launch_batch_status_fp32(const BatchInst<float>* tab, const BatchCtl* ctl, const int* err, int* status,
+                                     cudaStream_t s);
 int batch_stage_occupancy(int fp32, int S, int V, int* blocks_per_sm);
 }  // namespace cns
 
@@ -90,6 +94,7 @@ struct cns_batch {
     unsigned long long* d_cnt = nullptr;   // the persistent kernel's four phase unit counters
     std::vector<BatchInst<float>> h_tab32;   // host copy of the FP32 member table (the launch argument's source)
     int* d_err = nullptr;
+    int *d_status = nullptr, *h_status = nullptr;   // k_batch_status; h_status page-locked
     // full residency unless a shape is set or tuned (choose_shape clamps it): 20 steps of 8
     // FP32 boxes 32..128 take 42 ms with 7 blocks per SM, 115 ms with 1
     int threads = 128, blocks_per_sm = 32, nsm = 152;
@@ -115,6 +120,8 @@ struct cns_batch {
         if (d_bar) cudaFree(d_bar);
         if (d_cnt) cudaFree(d_cnt);
         if (d_err) cudaFree(d_err);
+        if (d_status) cudaFree(d_status);
+        if (h_status) cudaFreeHost(h_status);
         for (auto s : lanes) cudaStreamDestroy(s);
         for (auto e : lane_done) cudaEventDestroy(e);
         if (fork) cudaEventDestroy(fork);
@@ -385,6 +392,8 @@ int cns_batch_create(int device, int precision, int stencil_size, int stencil_vi
     if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_cnt, 4 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(b->d_cnt, 0, 4 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(b->d_err, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_status, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_status, 2 * sizeof(int));
     if (e != cudaSuccess) {
         delete b;
         return cns::set_error(CNS_ERR_OOM, "batch set-up allocation failed");
@@ -560,23 +569,25 @@ int cns_batch_step(cns_batch* b, int nsteps) {
             }
         }
     }
+    // one copy and one wait for all members (a copy per member cost a server tick ~60 us)
+    if (b->precision == CNS_PREC_FP32_RHS)
+        BCK(launch_batch_status_fp32((const BatchInst<float>*)b->d_tab, b->d_ctl, b->d_err, b->d_status, b->stream));
+    else
+        BCK(launch_batch_status_fp64((const BatchInst<double>*)b->d_tab, b->d_ctl, b->d_err, b->d_status, b->stream));
+    b->launches++;
+    BCK(cudaMemcpyAsync(b->h_status, b->d_status, 2 * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
     BCK(cudaStreamSynchronize(b->stream));
-    int err = 0;
-    BCK(cudaMemcpy(&err, b->d_err, sizeof err, cudaMemcpyDeviceToHost));
-    if (err) {
+    if (b->h_status[0]) {
         cudaMemset(b->d_err, 0, sizeof(int));
         cudaMemset(b->d_bar, 0, 2 * sizeof(unsigned));
         cudaMemset(b->d_cnt, 0, 4 * sizeof(unsigned long long));
         return cns::set_error(CNS_ERR_TIMEOUT, "batch grid barrier gave up (bounded wait)");
     }
-    for (auto& m : b->members) {
-        double sc[SC_COUNT];
-        BCK(cudaMemcpy(sc, m.h->scal, sizeof sc, cudaMemcpyDeviceToHost));
-        if (sc[SC_NONFINITE] != 0.0) {
-            char buf[160];
-            snprintf(buf, sizeof buf, "batch member %d: non-positive or non-finite density/temperature", m.id);
-            return cns::set_error(CNS_ERR_NONFINITE, buf);
-        }
+    if (b->h_status[1] < (int)b->members.size()) {
+        char buf[160];
+        snprintf(buf, sizeof buf, "batch member %d: non-positive or non-finite density/temperature",
+                 b->members[b->h_status[1]].id);
+        return cns::set_error(CNS_ERR_NONFINITE, buf);
     }
     return CNS_OK;
 }

@@ -14,6 +14,10 @@ void launch_batch_stage_fp32(int S, int V, dim3 grid, const BatchInst<float>* ta
 void launch_batch_time_fp32(const BatchInst<float>* tab, const BatchCtl* ctl, cudaStream_t s) {
     batch_time_launch<float>(tab, ctl, s);
 }
+cudaError_t launch_batch_status_fp32(const BatchInst<float>* tab, const BatchCtl* ctl, const int* err, int* status,
+                                     cudaStream_t s) {
+    return batch_status_launch<float>(tab, ctl, err, status, s);
+}
 cudaError_t batch_occ_fp32(int S, int V, int* nb) { return batch_occ_dispatch<float>(S, V, nb); }
 
 int batch_stage_occupancy(int fp32, int S, int V, int* blocks_per_sm) {

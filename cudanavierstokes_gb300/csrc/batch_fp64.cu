@@ -10,5 +10,9 @@ void launch_batch_stage_fp64(int S, int V, dim3 grid, const BatchInst<double>* t
 void launch_batch_time_fp64(const BatchInst<double>* tab, const BatchCtl* ctl, cudaStream_t s) {
     batch_time_launch<double>(tab, ctl, s);
 }
+cudaError_t launch_batch_status_fp64(const BatchInst<double>* tab, const BatchCtl* ctl, const int* err, int* status,
+                                     cudaStream_t s) {
+    return batch_status_launch<double>(tab, ctl, err, status, s);
+}
 cudaError_t batch_occ_fp64(int S, int V, int* nb) { return batch_occ_dispatch<double>(S, V, nb); }
 }  // namespace cns

@@ -121,6 +121,25 @@ __global__ void k_batch_time(const BatchInst<R>* __restrict__ tab, const BatchCt
     if (q < ctl->n) advance_time(tab[q].scal, tab[q].tlog, tab[q].tcap);
 }
 
+// Status of the batch after its steps, one block: status[0] the barrier's error flag,
+// status[1] the first member whose state was found non-finite (n: none), gathered on the device
+// so that the host reads it in one copy
+template <typename R>
+__global__ void k_batch_status(const BatchInst<R>* __restrict__ tab, const BatchCtl* __restrict__ ctl, const int* err,
+                               int* status) {
+    __shared__ int first;
+    const int n = ctl->n;
+    if (threadIdx.x == 0) first = n;
+    __syncthreads();
+    for (int q = threadIdx.x; q < n; q += blockDim.x)
+        if (tab[q].scal[SC_NONFINITE] != 0.0) atomicMin(&first, q);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        status[0] = *err;
+        status[1] = first;
+    }
+}
+
 // the (i, j, k) point of thread (tx, ty) in point unit lu of an instance
 template <typename R>
 __device__ __forceinline__ void unit_point(const BatchInst<R>& I, long long lu, int tx, int ty, int& i, int& j,

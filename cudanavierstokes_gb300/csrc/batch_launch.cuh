@@ -39,6 +39,13 @@ cudaError_t batch_time_launch(const BatchInst<R>* tab, const BatchCtl* ctl, cuda
     return cudaGetLastError();
 }
 
+template <typename R>
+cudaError_t batch_status_launch(const BatchInst<R>* tab, const BatchCtl* ctl, const int* err, int* status,
+                                cudaStream_t s) {
+    k_batch_status<R><<<1, CNS_BATCH_MAX, 0, s>>>(tab, ctl, err, status);
+    return cudaGetLastError();
+}
+
 // resident blocks per SM: the smaller of the two RHS-phase variants
 template <typename R, int S, int V>
 cudaError_t batch_occ_t(int* nb) {
