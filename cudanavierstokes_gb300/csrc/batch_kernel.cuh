@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, sizeof(R) == 4 ? 7 : 4)
             fx_exponents(in.fx.gmax, e);
             if (u == ctl->unit_off[q] && threadIdx.x < FXK_COUNT)
                 in.fx.k[threadIdx.x] =
-                    fx_table(I.cf.fx, in.fx.gmax, I.g.nonuniform_x, I.cf.lam_mu, (int)threadIdx.x);
+                    fx_table(I.cf.fx, in.fx.gmax, I.cf.lam_mu, (int)threadIdx.x);
             if (i < I.g.mx && j < I.g.my) fx_point<V>(I.g, I.cf.fx, in, e, I.cf.xp, i, j, k);
         }
     });

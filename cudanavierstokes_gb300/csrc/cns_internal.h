@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "cns_common.cuh"
+#include "fx.cuh"
 
 namespace cns {
 
@@ -47,10 +48,11 @@ enum { FXK_U = 0, FXK_MU = 3, FXK_T = 4, FXK_TH = 5, FXK_P = 6, FXK_L = 7, FXK_L
        FXK_DIR = 16, FXK_CTR = 48, FXK_A = 52, FXK_UL = 57, FXK_UD = 61, FXK_UC = 62, FXK_UE = 63, FXK_TG = 64,
        FXK_COUNT = 65 };
 
-// FP64 mode: the ghosted stencil inputs as pairs of 64-bit fixed-point values, (rho, u),
-// (v, w), (T, p), (H, mu), theta, and the stage's scale factors
+// FP64 mode: the ghosted stencil inputs as 64-bit fixed-point records, (u, v, w, p), (T, mu),
+// (rho, H), theta, and the stage's scale factors
 struct FxFields {
-    longlong2* f[4];
+    Fx4* v;
+    longlong2 *t, *r;
     long long* th;
     long long* k;
     unsigned *gmax, *gnext;   // maxima of this state's fields; of the next state's

@@ -59,13 +59,13 @@ __device__ __forceinline__ i64 fx_mul_by4(i64 a, i64 b) {
 // halves' and the low halves'. With |a| < 2^63 and sum |w| <= 2^30.8 both stay below 2^61.8.
 struct FxSum {
     i64 h, l;
-    __device__ __forceinline__ FxSum() : h(0), l(0) {}
+    __device__ __forceinline__ FxSum() : h(0), l(FX_HALF) {}   // rounds value()
     __device__ __forceinline__ void add(i64 a, int w) {
         h = fx_mad(fx_hi(a), w, h);
         l = fx_mad(fx_lo(a), w, l);
     }
-    __device__ __forceinline__ i64 value() const { return h + (i64)fx_word1(l + FX_HALF); }
-    __device__ __forceinline__ i64 twice() const { return (h << 1) + ((l + FX_HALF / 2) >> 31); }
+    __device__ __forceinline__ i64 value() const { return h + (i64)fx_word1(l); }
+    __device__ __forceinline__ i64 twice() const { return (h << 1) + ((l - FX_HALF / 2) >> 31); }
 };
 
 // ---- central-difference weights as integers: c1[k] = fxw1(K, k) / fxn1(K) etc., scaled by
@@ -86,6 +86,19 @@ __host__ __device__ constexpr int fxw2(int K, int k) {
             : K == 2 ? (k == 0 ? -30 : k == 1 ? 16 : -1)
             : K == 3 ? (k == 0 ? -490 : k == 1 ? 270 : k == 2 ? -27 : 2)
                      : (k == 0 ? -14350 : k == 1 ? 8064 : k == 2 ? -1008 : k == 3 ? 128 : -9)) * (1 << fxs2(K));
+}
+
+// ---- four values of a 32-byte record, one load or store ----
+struct __align__(32) Fx4 {
+    i64 x, y, z, w;
+};
+__device__ __forceinline__ Fx4 fx_load4(const Fx4* p) {
+    Fx4 r;
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(r.x), "=l"(r.y), "=l"(r.z), "=l"(r.w) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ void fx_store4(Fx4* p, i64 x, i64 y, i64 z, i64 w) {
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" : : "l"(p), "l"(x), "l"(y), "l"(z), "l"(w) : "memory");
 }
 
 // ---- exponents ----

@@ -44,9 +44,11 @@ __global__ void __launch_bounds__(DIL_TX * DIL_TY) k_dil_march(Geom g, CoefT<flo
                                  min(k0 + DIL_NZ, g.mz), own != 0, (int)threadIdx.x, (int)threadIdx.y, su, sv);
 }
 
-// FP64 mode: fixed-point conversion and theta. Blocks of 32 x 8 threads: the first `tiles`
-// march nz planes of a 32 x 8 tile each (fx_column), the others convert 256 ghost cells each;
-// the first block also writes the stage's scale factors.
+// FP64 mode: fixed-point conversion and theta. Blocks of 32 x 8 threads: the first ones write
+// the stage's scale factors (16^3 box: by one block beside its tile 14 us for the kernel, so
+// 9.9), the next `tiles` march nz planes of a 32 x 8 tile each (fx_column), the others convert
+// 256 ghost cells each.
+constexpr int FX_TABLE_BLOCKS = (FXK_COUNT + DIL_TY - 1) / DIL_TY;
 template <int V>
 __global__ void __launch_bounds__(DIL_TX * DIL_TY, 4) k_fx(Geom g, const __grid_constant__ FxBase b,
                                                            const __grid_constant__ RhsIn<double> in,
@@ -57,8 +59,12 @@ __global__ void __launch_bounds__(DIL_TX * DIL_TY, 4) k_fx(Geom g, const __grid_
     const int tid = threadIdx.y * DIL_TX + threadIdx.x;
     int e[8];
     fx_exponents(in.fx.gmax, e);   // out of range: the factors are NaN
-    int t = (int)blockIdx.x;
-    if (t == 0 && tid < FXK_COUNT) in.fx.k[tid] = fx_table(b, in.fx.gmax, g.nonuniform_x, lam_mu, tid);
+    int t = (int)blockIdx.x - FX_TABLE_BLOCKS;
+    if (t < 0) {   // an entry per warp: the entries' branches differ, one warp would take them in turn
+        const int q = blockIdx.x * DIL_TY + threadIdx.y;
+        if (threadIdx.x == 0 && q < FXK_COUNT) in.fx.k[q] = fx_table(b, in.fx.gmax, lam_mu, q);
+        return;
+    }
     if (t >= tiles) {
         t = (t - tiles) * DIL_TX * DIL_TY + tid;
         if (t < ghost_count(g)) fx_ghost(g, in, e, t);
@@ -266,7 +272,7 @@ void launch_fx(int V, const Geom& g, const CoefT<double>& cf, const RhsIn<double
     int nz = DIL_NZ;
     while (nz > 1 && (long long)nbx * nby * ((g.mz + nz - 1) / nz) < 4 * 152) nz /= 2;
     const int tiles = nbx * nby * ((g.mz + nz - 1) / nz);
-    const unsigned grid = (unsigned)tiles + ghost_blocks(g);
+    const unsigned grid = FX_TABLE_BLOCKS + (unsigned)tiles + ghost_blocks(g);
     const dim3 block(DIL_TX, DIL_TY, 1);
     switch (V) {
     case 1: k_fx<1><<<grid, block, 0, s>>>(g, cf.fx, in, cf.xp, cf.lam_mu, own, tiles, nbx, nby, nz); break;

@@ -85,7 +85,7 @@ __device__ __forceinline__ double fx_factor(const FxBase& b, const int (&e)[8], 
 // entry t of the stage's table (FXK_*). The factors from the RHS integers to real values are
 // NaN if a field is out of range, so that the state becomes NaN and is reported as every
 // other non-finite state.
-__device__ __forceinline__ i64 fx_table(const FxBase& b, const unsigned* gmax, int nonuniform_x, double lam_mu, int t) {
+static __device__ __noinline__ i64 fx_table(const FxBase& b, const unsigned* gmax, double lam_mu, int t) {
     int e[8];
     if (!fx_exponents(gmax, e)) return 0x7ff8000000000000LL;
     const int xth = fx_unit_theta(b, e);
@@ -143,10 +143,9 @@ __device__ __forceinline__ i64 fx_mul2(i64 a0, i64 b0, i64 a1, i64 b1) {
 // the eight fields of element c as integers; u and v given if the caller has them
 __device__ __forceinline__ void fx_store(const FxFields& o, const RhsIn<double>& in, const int (&e)[8], int c, i64 u,
                                          i64 v, i64 w) {
-    o.f[0][c] = make_longlong2(u, v);
-    o.f[1][c] = make_longlong2(w, fx_from(in.p[c], e[5]));
-    o.f[2][c] = make_longlong2(fx_from(in.t[c], e[4]), fx_from(in.m[c], e[7]));
-    o.f[3][c] = make_longlong2(fx_from(in.r[c], e[0]), fx_from(in.h[c], e[6]));
+    fx_store4(o.v + c, u, v, w, fx_from(in.p[c], e[5]));
+    o.t[c] = make_longlong2(fx_from(in.t[c], e[4]), fx_from(in.m[c], e[7]));
+    o.r[c] = make_longlong2(fx_from(in.r[c], e[0]), fx_from(in.h[c], e[6]));
 }
 
 // the conversion of ghost cell t
@@ -227,10 +226,9 @@ __device__ __forceinline__ void fx_column(const Geom& g, const FxBase& b, const 
             const i64 th = fx_mul(sx.value(), kx) + fx_mul(sy.value(), ky) + fx_mul(sz.value(), kz);
             in.fx.th[ck] = th;
             if (own) dil_ghost_owner<i64>(g, in.fx.th, ck, i, j, k, th);
-            in.fx.f[0][ck] = make_longlong2(cu, cv);
-            in.fx.f[1][ck] = make_longlong2(ring[V], fx_from(q[0], e[5]));
-            in.fx.f[2][ck] = make_longlong2(fx_from(q[1], e[4]), fx_from(q[2], e[7]));
-            in.fx.f[3][ck] = make_longlong2(fx_from(q[3], e[0]), fx_from(q[4], e[6]));
+            fx_store4(in.fx.v + ck, cu, cv, ring[V], fx_from(q[0], e[5]));
+            in.fx.t[ck] = make_longlong2(fx_from(q[1], e[4]), fx_from(q[2], e[7]));
+            in.fx.r[ck] = make_longlong2(fx_from(q[3], e[0]), fx_from(q[4], e[6]));
         }
 #pragma unroll
         for (int l = 0; l < 2 * V; l++) ring[l] = ring[l + 1];
@@ -258,7 +256,9 @@ __device__ __forceinline__ void fx_point(const Geom& g, const FxBase& b, const R
 }
 
 // The sums of one direction at a point, in two passes over the neighbour pairs (-l, l), each of
-// which loads a pair once and feeds every sum that needs it:
+// which loads a pair once and feeds every sum that needs it (one pass for all of them needs 150
+// registers: 640 bytes spilled and 1.28 against 1.23 ms on the channel; with the four values
+// both passes read as one 32-byte load and both loops unrolled 0.93 ms):
 //   fx_visc  first derivatives of u, v, w, mu, T, theta and second ones of u, v, w, T (viscous
 //            order)
 //   fx_conv  first derivative of p and the telescoped split-form fluxes (advective order)
@@ -280,18 +280,17 @@ __device__ __forceinline__ FxVisc fx_visc(const FxFields& in, int c, int st, con
     for (int q = 0; q < 4; q++) L[q].add(ctr[q], fxw2(V, 0));
 #pragma unroll
     for (int l = 1; l <= V; l++) {
-        const longlong2 am = __ldg(in.f[0] + c - l * st), ap = __ldg(in.f[0] + c + l * st);
-        const longlong2 bm = __ldg(in.f[1] + c - l * st), bp = __ldg(in.f[1] + c + l * st);
-        const longlong2 tm = __ldg(in.f[2] + c - l * st), tp = __ldg(in.f[2] + c + l * st);
+        const Fx4 am = fx_load4(in.v + c - l * st), ap = fx_load4(in.v + c + l * st);
+        const longlong2 tm = __ldg(in.t + c - l * st), tp = __ldg(in.t + c + l * st);
         D[0].add(ap.x - am.x, fxw1(V, l));
         D[1].add(ap.y - am.y, fxw1(V, l));
-        D[2].add(bp.x - bm.x, fxw1(V, l));
+        D[2].add(ap.z - am.z, fxw1(V, l));
         D[3].add(tp.y - tm.y, fxw1(V, l));
         D[4].add(tp.x - tm.x, fxw1(V, l));
         D[5].add(__ldg(in.th + c + l * st) - __ldg(in.th + c - l * st), fxw1(V, l));
         L[0].add(ap.x + am.x, fxw2(V, l));
         L[1].add(ap.y + am.y, fxw2(V, l));
-        L[2].add(bp.x + bm.x, fxw2(V, l));
+        L[2].add(ap.z + am.z, fxw2(V, l));
         L[3].add(tp.x + tm.x, fxw2(V, l));
     }
     FxVisc o;
@@ -305,18 +304,17 @@ __device__ __forceinline__ FxVisc fx_visc(const FxFields& in, int c, int st, con
 template <int S, int DIR>
 __device__ __forceinline__ FxConv fx_conv(const FxFields& in, int c, int st, i64 r0, i64 g0) {
     FxSum P, F[5];
-#pragma unroll 1
+#pragma unroll
     for (int l = 1; l <= S; l++) {
-        const longlong2 am = __ldg(in.f[0] + c - l * st), ap = __ldg(in.f[0] + c + l * st);
-        const longlong2 bm = __ldg(in.f[1] + c - l * st), bp = __ldg(in.f[1] + c + l * st);
-        const longlong2 hm = __ldg(in.f[3] + c - l * st), hp = __ldg(in.f[3] + c + l * st);
-        P.add(bp.y - bm.y, fxw1(S, l));
-        const i64 gm = DIR == 0 ? am.x : DIR == 1 ? am.y : bm.x;
-        const i64 gp = DIR == 0 ? ap.x : DIR == 1 ? ap.y : bp.x;
+        const Fx4 am = fx_load4(in.v + c - l * st), ap = fx_load4(in.v + c + l * st);
+        const longlong2 hm = __ldg(in.r + c - l * st), hp = __ldg(in.r + c + l * st);
+        P.add(ap.w - am.w, fxw1(S, l));
+        const i64 gm = DIR == 0 ? am.x : DIR == 1 ? am.y : am.z;
+        const i64 gp = DIR == 0 ? ap.x : DIR == 1 ? ap.y : ap.z;
         const i64 qm = fx_mul(hm.x + r0, gm + g0), qp = -fx_mul(hp.x + r0, gp + g0);
         F[0].add(qm + qp, fxw1(S, l));
         const int qmh = fx_hi(qm), qml = fx_lo(qm), qph = fx_hi(qp), qpl = fx_lo(qp);
-        const i64 phm[4] = {am.x, am.y, bm.x, hm.y}, php[4] = {ap.x, ap.y, bp.x, hp.y};
+        const i64 phm[4] = {am.x, am.y, am.z, hm.y}, php[4] = {ap.x, ap.y, ap.z, hp.y};
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const int mh = fx_hi(phm[q]), ml = fx_lo(phm[q]), ph = fx_hi(php[q]), pl = fx_lo(php[q]);
@@ -363,7 +361,8 @@ __device__ __forceinline__ void rhs_acc_fx(const Geom& g, const FxBase& b, const
     i64 acc[5] = {0, 0, 0, 0, 0};
     const bool nux = g.nonuniform_x;
     const i64 xp = nux ? __ldg(b.xpk + i) : 0;
-    const longlong2 A = __ldg(x.f[0] + c), B = __ldg(x.f[1] + c), H = __ldg(x.f[3] + c);
+    const Fx4 A = fx_load4(x.v + c);
+    const longlong2 H = __ldg(x.r + c);
     const auto conv = [&](const FxConv& o, int d, bool sx) {
         const i64* k = K + d * FXK_DIR;
         const auto f = [&](i64 v, int q) { return fx_mulk(sx ? fx_mulk(v, xp) : v, k[q]); };
@@ -373,13 +372,13 @@ __device__ __forceinline__ void rhs_acc_fx(const Geom& g, const FxBase& b, const
     };
     conv(fx_conv<S, 0>(x, c, 1, H.x, A.x), 0, nux);
     conv(fx_conv<S, 1>(x, c, (int)g.P, H.x, A.y), 1, false);
-    conv(fx_conv<S, 2>(x, c, (int)g.PS, H.x, B.x), 2, false);
+    conv(fx_conv<S, 2>(x, c, (int)g.PS, H.x, A.z), 2, false);
     // the cubic fluxes' centre values: phi_0 times half the mass flux
-    const i64 phi[4] = {A.x, A.y, B.x, H.y};
+    const i64 phi[4] = {A.x, A.y, A.z, H.y};
 #pragma unroll
     for (int q = 0; q < 4; q++) acc[1 + q] += fx_mulk(fx_mul_by4(phi[q], acc[0]), K[FXK_CTR + q]);
-    const longlong2 T = __ldg(x.f[2] + c);
-    const i64 ctr[4] = {A.x, A.y, B.x, T.x};
+    const longlong2 T = __ldg(x.t + c);
+    const i64 ctr[4] = {A.x, A.y, A.z, T.x};
     const longlong2 xx = nux ? __ldg(b.xx + i) : make_longlong2(0, 0);
     i64 G[9], dmu[3], dT[3], L[4] = {0, 0, 0, 0};
     const auto visc = [&](const FxVisc& o, int d, bool sx) {

@@ -325,10 +325,9 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
 }
 
 // FP32: 7 blocks of 128 per SM (72 registers) measured fastest (6: 80 registers, +13 %
-// time; 5: 96 registers, and stages that read the RK register ran 3.5x slower). FP64: 5 blocks
-// (96 registers): latency bound at 43 % issue, FP64 pipe 54 % busy; 4 blocks 1.14 ms, 6 blocks
-// 1.07 ms against 1.09 on the channel 128x160x192, but 6 (80 registers, spilling) 0.088 against
-// 0.081 ms on a 64^3 box.
+// time; 5: 96 registers, and stages that read the RK register ran 3.5x slower). FP64: 4 blocks
+// (128 registers), bound by latency: issue 38 %, FP64 pipe 44 %, ~3,700 instructions per point;
+// on the channel 128x160x192 0.93 ms, with 3 blocks (168 registers) 1.11, 5 (96, spilling) 0.98.
 //
 // One launch covers the 4-row bands [band0, band0 + gridDim.y) of every plane; blocks are
 // dispatched x fastest, then bands, then planes. On large planes the bands are split into
@@ -336,7 +335,7 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
 // group's blocks sweep them (one launch over whole planes would cycle ~2S planes of the
 // inputs through L2 between their uses).
 template <typename R, int S, int V>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 5) k_rhs(Geom g, const __grid_constant__ CoefT<R> cf,
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 4) k_rhs(Geom g, const __grid_constant__ CoefT<R> cf,
                                                                                    const __grid_constant__ RhsIn<R> in, Update<R> up,
                                              double* __restrict__ scal, int quirk, int band0) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

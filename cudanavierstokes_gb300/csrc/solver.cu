@@ -567,7 +567,9 @@ int cns_create(const cns_params* pin, int device, cns_solver** out) {
     }
     if (!rc) rc = h->alloc_field(&h->dil, rs);
     if (!h->fp32) {
-        for (int f = 0; f < 4 && !rc; f++) rc = h->alloc_field((void**)&h->fx.f[f], sizeof(longlong2));
+        rc = rc ? rc : h->alloc_field((void**)&h->fx.v, sizeof(Fx4));
+        if (!rc) rc = h->alloc_field((void**)&h->fx.t, sizeof(longlong2));
+        if (!rc) rc = h->alloc_field((void**)&h->fx.r, sizeof(longlong2));
         h->fx.th = (long long*)h->dil;
         if (!rc) rc = h->alloc(&h->fx.k, FXK_COUNT);
         for (int b = 0; b < 2 && !rc; b++) rc = h->alloc(&h->gmax[b], 8);
