@@ -6,7 +6,8 @@
 //               integers of u, v, w (fx_point: of one point)
 //   fx_ghost    the same conversion of a ghost cell
 //   fx_table    the stage's scale factors (one thread each)
-//   rhs_acc_fx  the RHS of a point on the integer units; the five sums are converted once
+//   fx_convective, fx_viscous  the two parts of the RHS of a point on the integer units; each
+//               sum is converted once
 #pragma once
 #include "cns_common.cuh"
 #include "cns_internal.h"
@@ -301,10 +302,10 @@ __device__ __forceinline__ FxVisc fx_visc(const FxFields& in, int c, int st, con
     return o;
 }
 
-template <int S, int DIR>
+template <int S, int DIR, bool ROLLED>
 __device__ __forceinline__ FxConv fx_conv(const FxFields& in, int c, int st, i64 r0, i64 g0) {
     FxSum P, F[5];
-#pragma unroll
+#pragma unroll(ROLLED ? 1 : S)
     for (int l = 1; l <= S; l++) {
         const Fx4 am = fx_load4(in.v + c - l * st), ap = fx_load4(in.v + c + l * st);
         const longlong2 hm = __ldg(in.r + c - l * st), hp = __ldg(in.r + c + l * st);
@@ -350,13 +351,20 @@ __device__ __forceinline__ i64 fx_dot3(i64 a0, i64 b0, i64 a1, i64 b1, i64 a2, i
 __device__ __forceinline__ int fx_bits(i64 v) { return fx_word1(v) ^ (fx_word1(v) >> 31); }
 __device__ __forceinline__ int fx_room(int bits) { return max(__clz(bits) - 2, 0); }
 
-// RHS of one interior point at element c into out (without body force and sponge). Bounds in
-// the units of fx_table: gradients < 2^59.8, theta, stress < 2^61.8, grad mu, grad T < 2^60.8,
-// second derivatives < 2^62.3, RHS sums < 2^62.4.
-template <int S, int V>
-__device__ __forceinline__ void rhs_acc_fx(const Geom& g, const FxBase& b, const RhsIn<double>& in, int quirk, int i,
-                                           int c, double u0, double v0, double w0, double (&out)[5]) {
-    const FxFields& x = in.fx;
+// table unit q times 2^-s
+__device__ __forceinline__ double fx_unit(const i64* K, int q, int s) {
+    const double k = __longlong_as_double(K[q]);
+    return __hiloint2double(__double2hiint(k) - (s << 20), __double2loint(k));
+}
+
+// RHS of one interior point at element c (without body force and sponge), in two parts that
+// share no intermediate value. Bounds in the units of fx_table: gradients < 2^59.8, theta,
+// stress < 2^61.8, grad mu, grad T < 2^60.8, second derivatives < 2^62.3, RHS sums < 2^62.4.
+//
+// The convective and pressure terms. ROLLED: the loops over the offsets are not unrolled.
+template <int S, bool ROLLED>
+__device__ __forceinline__ void fx_convective(const Geom& g, const FxBase& b, const FxFields& x, int i, int c,
+                                              double (&out)[5]) {
     const i64* __restrict__ K = x.k;
     i64 acc[5] = {0, 0, 0, 0, 0};
     const bool nux = g.nonuniform_x;
@@ -370,13 +378,26 @@ __device__ __forceinline__ void rhs_acc_fx(const Geom& g, const FxBase& b, const
 #pragma unroll
         for (int q = 0; q < 5; q++) acc[q] += f(o.F[q], FXK_F0 + q);
     };
-    conv(fx_conv<S, 0>(x, c, 1, H.x, A.x), 0, nux);
-    conv(fx_conv<S, 1>(x, c, (int)g.P, H.x, A.y), 1, false);
-    conv(fx_conv<S, 2>(x, c, (int)g.PS, H.x, A.z), 2, false);
+    conv(fx_conv<S, 0, ROLLED>(x, c, 1, H.x, A.x), 0, nux);
+    conv(fx_conv<S, 1, ROLLED>(x, c, (int)g.P, H.x, A.y), 1, false);
+    conv(fx_conv<S, 2, ROLLED>(x, c, (int)g.PS, H.x, A.z), 2, false);
     // the cubic fluxes' centre values: phi_0 times half the mass flux
     const i64 phi[4] = {A.x, A.y, A.z, H.y};
 #pragma unroll
     for (int q = 0; q < 4; q++) acc[1 + q] += fx_mulk(fx_mul_by4(phi[q], acc[0]), K[FXK_CTR + q]);
+#pragma unroll
+    for (int q = 0; q < 5; q++) out[q] = (double)acc[q] * fx_unit(K, FXK_A + q, 0);
+}
+
+// The viscous terms: force in out[0..2], conduction, dissipation and work in out[3]
+template <int V>
+__device__ __forceinline__ void fx_viscous(const Geom& g, const FxBase& b, const RhsIn<double>& in, int quirk, int i,
+                                           int c, double u0, double v0, double w0, double (&out)[4]) {
+    const FxFields& x = in.fx;
+    const i64* __restrict__ K = x.k;
+    const bool nux = g.nonuniform_x;
+    const i64 xp = nux ? __ldg(b.xpk + i) : 0;
+    const Fx4 A = fx_load4(x.v + c);
     const longlong2 T = __ldg(x.t + c);
     const i64 ctr[4] = {A.x, A.y, A.z, T.x};
     const longlong2 xx = nux ? __ldg(b.xx + i) : make_longlong2(0, 0);
@@ -396,10 +417,6 @@ __device__ __forceinline__ void rhs_acc_fx(const Geom& g, const FxBase& b, const
     visc(fx_visc<V>(x, c, 1, ctr), 0, nux);
     visc(fx_visc<V>(x, c, (int)g.P, ctr), 1, false);
     visc(fx_visc<V>(x, c, (int)g.PS, ctr), 2, false);
-    const auto unit = [&](int q, int s) {   // table unit times 2^-s
-        const double k = __longlong_as_double(K[q]);
-        return __hiloint2double(__double2hiint(k) - (s << 20), __double2loint(k));
-    };
     // grad mu and the stress tensor tau / mu, each scaled to the full range
     const int sm = fx_room(fx_bits(dmu[0]) | fx_bits(dmu[1]) | fx_bits(dmu[2]));
 #pragma unroll
@@ -415,22 +432,17 @@ __device__ __forceinline__ void rhs_acc_fx(const Geom& g, const FxBase& b, const
     q12 <<= st;
     // dissipation / mu: tau_ab du_b/dx_a = sum t_aa^2 / 2 (the trace of t is zero) + sum t_ab^2
     const i64 diss = (fx_dot3(t[0], t[0], t[1], t[1], t[2], t[2]) >> 1) + fx_dot3(t[3], t[3], t[4], t[4], t[5], q12);
-    const double ud = unit(FXK_UD, sm + st);
-    const double W[3] = {fma((double)fx_mul(T.y, L[0]), unit(FXK_UL, 0),
-                             (double)fx_dot3(t[0], dmu[0], t[3], dmu[1], t[4], dmu[2]) * ud),
-                         fma((double)fx_mul(T.y, L[1]), unit(FXK_UL + 1, 0),
-                             (double)fx_dot3(t[3], dmu[0], t[1], dmu[1], t[5], dmu[2]) * ud),
-                         fma((double)fx_mul(T.y, L[2]), unit(FXK_UL + 2, 0),
-                             (double)fx_dot3(t[4], dmu[0], t[5], dmu[1], t[2], dmu[2]) * ud)};
-    double en = (double)acc[4] * unit(FXK_A + 4, 0);
-    en = fma((double)fx_mul(T.y, L[3]), unit(FXK_UL + 3, 0), en);
-    en = fma((double)fx_dot3(dT[0], dmu[0], dT[1], dmu[1], dT[2], dmu[2]), unit(FXK_UC, sm), en);
-    en = fma(in.m[c], (double)diss * unit(FXK_UE, 2 * st), en);
-    out[0] = (double)acc[0] * unit(FXK_A, 0);
-    out[1] = fma((double)acc[1], unit(FXK_A + 1, 0), W[0]);
-    out[2] = fma((double)acc[2], unit(FXK_A + 2, 0), W[1]);
-    out[3] = fma((double)acc[3], unit(FXK_A + 3, 0), W[2]);
-    out[4] = en + fma(u0, W[0], fma(v0, W[1], w0 * W[2]));
+    const double ud = fx_unit(K, FXK_UD, sm + st);
+    out[0] = fma((double)fx_mul(T.y, L[0]), fx_unit(K, FXK_UL, 0),
+                 (double)fx_dot3(t[0], dmu[0], t[3], dmu[1], t[4], dmu[2]) * ud);
+    out[1] = fma((double)fx_mul(T.y, L[1]), fx_unit(K, FXK_UL + 1, 0),
+                 (double)fx_dot3(t[3], dmu[0], t[1], dmu[1], t[5], dmu[2]) * ud);
+    out[2] = fma((double)fx_mul(T.y, L[2]), fx_unit(K, FXK_UL + 2, 0),
+                 (double)fx_dot3(t[4], dmu[0], t[5], dmu[1], t[2], dmu[2]) * ud);
+    double en = (double)fx_mul(T.y, L[3]) * fx_unit(K, FXK_UL + 3, 0);
+    en = fma((double)fx_dot3(dT[0], dmu[0], dT[1], dmu[1], dT[2], dmu[2]), fx_unit(K, FXK_UC, sm), en);
+    en = fma(in.m[c], (double)diss * fx_unit(K, FXK_UE, 2 * st), en);
+    out[3] = fma(u0, out[0], fma(v0, out[1], fma(w0, out[2], en)));
 }
 
 }  // namespace cns

@@ -17,6 +17,8 @@
 // which is the same value with 2 instead of l(l+1) pair products per l. The product
 // (rho_a+rho_b)(g_a+g_b) is shared by the mass flux and the four cubic fluxes.
 #pragma once
+#include <type_traits>
+
 #include "cns_common.cuh"
 #include "cns_internal.h"
 #include "kernels_fx.cuh"
@@ -318,30 +320,68 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
     } else {
         const int c = (int)g.at(i, j, k);
         const double u0 = up.qin.u[c], v0 = up.qin.v[c], w0 = up.qin.w[c];
-        double acc[5];
-        rhs_acc_fx<S, V>(g, cf.fx, in, quirk, i, c, u0, v0, w0, acc);
+        double acc[5], vis[4];
+        fx_convective<S, CW>(g, cf.fx, in.fx, i, c, acc);
+        fx_viscous<V>(g, cf.fx, in, quirk, i, c, u0, v0, w0, vis);
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[1 + q] += vis[q];
         stage_tail<double>(g, up, scal, i, k, c, acc, u0, v0, w0, up.qin.r[c]);
     }
 }
 
+// One launch covers the rows [row0, row0 + gridDim.y * rows per block) of every plane; blocks are
+// dispatched x fastest, then rows, then planes. On large planes the rows are split into groups
+// launched one after another, so the planes a z stencil spans stay in L2 while a group's blocks
+// sweep them (one launch over whole planes would cycle ~2S planes of the inputs through L2
+// between their uses).
+//
 // FP32: 7 blocks of 128 per SM (72 registers) measured fastest (6: 80 registers, +13 %
 // time; 5: 96 registers, and stages that read the RK register ran 3.5x slower). FP64: 4 blocks
 // (128 registers), bound by latency: issue 38 %, FP64 pipe 44 %, ~3,700 instructions per point;
 // on the channel 128x160x192 0.93 ms, with 3 blocks (168 registers) 1.11, 5 (96, spilling) 0.98.
-//
-// One launch covers the 4-row bands [band0, band0 + gridDim.y) of every plane; blocks are
-// dispatched x fastest, then bands, then planes. On large planes the bands are split into
-// groups launched one after another, so the planes a z stencil spans stay in L2 while a
-// group's blocks sweep them (one launch over whole planes would cycle ~2S planes of the
-// inputs through L2 between their uses).
 template <typename R, int S, int V>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 4) k_rhs(Geom g, const __grid_constant__ CoefT<R> cf,
-                                                                                   const __grid_constant__ RhsIn<R> in, Update<R> up,
-                                             double* __restrict__ scal, int quirk, int band0) {
+                                                                     const __grid_constant__ RhsIn<R> in, Update<R> up,
+                                                                     double* __restrict__ scal, int quirk, int row0) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = (band0 + (int)blockIdx.y) * blockDim.y + threadIdx.y;
+    const int j = row0 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
     if (i >= g.mx || j >= g.my) return;
     rhs_point<R, S, V>(g, cf, in, up, scal, quirk, i, j, (int)blockIdx.z);
+}
+
+// FP64 on boxes with at most one block of k_rhs per SM, where a thread's dependent chain is the
+// kernel's time: a point takes two threads. The first half of a block's warps form the
+// convective part of its 32 x 2 points and, with the viscous part that the other warps hand over
+// in shared memory, the stage update. 14^3 .. 28^3 boxes 14.3 .. 16.4 us against 16.4 .. 18.4; from
+// 32^3 (18.8 us against 18.4) on one thread per point is the faster, on the channel 128x160x192
+// 0.93 ms against 1.12.
+constexpr int SPLIT_ROWS = 2;
+template <int S, int V>
+__global__ void __launch_bounds__(64 * SPLIT_ROWS, 4) k_rhs_split(Geom g, const __grid_constant__ CoefT<double> cf,
+                                                                  const __grid_constant__ RhsIn<double> in,
+                                                                  Update<double> up, double* __restrict__ scal,
+                                                                  int quirk) {
+    __shared__ double sv[4][32 * SPLIT_ROWS];
+    const int row = (int)threadIdx.y % SPLIT_ROWS, s = row * 32 + threadIdx.x;
+    const int i = blockIdx.x * 32 + threadIdx.x, j = (int)blockIdx.y * SPLIT_ROWS + row, k = (int)blockIdx.z;
+    const bool inside = i < g.mx && j < g.my, first = threadIdx.y < SPLIT_ROWS;
+    const int c = (int)g.at(i, j, k);
+    double acc[5];
+    if (inside) {
+        if (first) {
+            fx_convective<S, false>(g, cf.fx, in.fx, i, c, acc);
+        } else {
+            double vis[4];
+            fx_viscous<V>(g, cf.fx, in, quirk, i, c, up.qin.u[c], up.qin.v[c], up.qin.w[c], vis);
+#pragma unroll
+            for (int q = 0; q < 4; q++) sv[q][s] = vis[q];
+        }
+    }
+    __syncthreads();
+    if (!inside || !first) return;
+#pragma unroll
+    for (int q = 0; q < 4; q++) acc[1 + q] += sv[q][s];
+    stage_tail<double>(g, up, scal, i, k, c, acc, up.qin.u[c], up.qin.v[c], up.qin.w[c], up.qin.r[c]);
 }
 
 // Bands per launch: all of them while 3 S planes of a band group at 72 B per point (the
@@ -359,21 +399,34 @@ inline int rhs_band_group(const Geom& g) {
     return fit < 8 ? 8 : (int)fit;
 }
 
+// f(S, V) with the orders as integral constants; false: no such instantiation
+template <class F>
+bool rhs_dispatch(int S, int V, F f) {
+#define CNS_RHS_CASE(SS, VV)                                                               \
+    if (S == SS && V == VV) {                                                              \
+        f(std::integral_constant<int, SS>(), std::integral_constant<int, VV>());           \
+        return true;                                                                       \
+    }
+    CNS_RHS_CASE(1, 1)
+    CNS_RHS_CASE(2, 1) CNS_RHS_CASE(2, 2)
+    CNS_RHS_CASE(3, 1) CNS_RHS_CASE(3, 2) CNS_RHS_CASE(3, 3)
+    CNS_RHS_CASE(4, 1) CNS_RHS_CASE(4, 2) CNS_RHS_CASE(4, 3) CNS_RHS_CASE(4, 4)
+#undef CNS_RHS_CASE
+    return false;
+}
+
 template <typename R>
 int launch_rhs_t(int S, int V, const Geom& g, const CoefT<R>& cf, const RhsIn<R>& in, const Update<R>& up,
                  double* scal, int quirk, cudaStream_t s) {
-    const int nby = (g.my + 3) / 4, group = rhs_band_group(g);
+    const int rows = 4 * rhs_band_group(g);   // per launch
     int n = 0;
-    for (int b0 = 0; b0 < nby; b0 += group, n++) {
-        dim3 grid((g.mx + 31) / 32, (unsigned)(nby - b0 < group ? nby - b0 : group), g.mz), block(32, 4, 1);
-#define CNS_RHS_CASE(SS, VV) \
-    if (S == SS && V == VV) { k_rhs<R, SS, VV><<<grid, block, 0, s>>>(g, cf, in, up, scal, quirk, b0); continue; }
-        CNS_RHS_CASE(1, 1)
-        CNS_RHS_CASE(2, 1) CNS_RHS_CASE(2, 2)
-        CNS_RHS_CASE(3, 1) CNS_RHS_CASE(3, 2) CNS_RHS_CASE(3, 3)
-        CNS_RHS_CASE(4, 1) CNS_RHS_CASE(4, 2) CNS_RHS_CASE(4, 3) CNS_RHS_CASE(4, 4)
-#undef CNS_RHS_CASE
-        return n;   // no instantiation for these orders
+    for (int j0 = 0; j0 < g.my; j0 += rows, n++) {
+        const int r = g.my - j0 < rows ? g.my - j0 : rows;
+        const dim3 grid((g.mx + 31) / 32, (r + 3) / 4, g.mz), block(32, 4, 1);
+        if (!rhs_dispatch(S, V, [&](auto s_, auto v_) {
+                k_rhs<R, decltype(s_)::value, decltype(v_)::value><<<grid, block, 0, s>>>(g, cf, in, up, scal, quirk, j0);
+            }))
+            break;
     }
     return n;
 }

@@ -92,3 +92,24 @@ def test_batch_modes(gpu_lib, oracle_mod, mode, mx):
     b.step(3)
     errs = state_errors(b.fields(i), o.get_state())
     assert max(errs) <= TOL64, errs
+
+
+@pytest.mark.parametrize("mx,my,mz", [(9, 8, 9), (33, 7, 38), (32, 8, 76), (32, 8, 77), (31, 9, 50), (65, 6, 29)])
+@pytest.mark.parametrize("S,V", [(4, 4), (3, 1)])
+def test_small_box_kernel(gpu_lib, oracle_mod, mx, my, mz, S, V):
+    """Both sides of the switch between two threads and one thread per point (152 blocks of 32 x
+    4 points: 32 x 8 x 76 is the last box below it), with ragged tiles, on channel walls."""
+    if my < 2 * S:
+        pytest.skip("fewer points than the stencil")
+    p = channel_params(mx, my, mz).copy(stencil_size=S, stencil_visc=V)
+    f = wall_state(p, oracle_mod.Oracle(p).grid()["x"])
+    o = oracle_mod.Oracle(p)
+    o.set_state(*f)
+    s = Solver(p)
+    s.copy_field_in(*f)
+    errs = field_errors(s.calc_rhs(), o.rhs())
+    assert max(errs) <= TOL64, errs
+    o.run(2)
+    s.run(2)
+    errs = state_errors(s.copy_field_out(), o.get_state())
+    assert max(errs) <= TOL64, errs
