@@ -361,12 +361,13 @@ __device__ __forceinline__ double fx_unit(const i64* K, int q, int s) {
 // share no intermediate value. Bounds in the units of fx_table: gradients < 2^59.8, theta,
 // stress < 2^61.8, grad mu, grad T < 2^60.8, second derivatives < 2^62.3, RHS sums < 2^62.4.
 //
-// The convective and pressure terms. ROLLED: the loops over the offsets are not unrolled.
+// The convective and pressure terms as integer sums. ROLLED: the loops over the offsets are not unrolled.
 template <int S, bool ROLLED>
 __device__ __forceinline__ void fx_convective(const Geom& g, const FxBase& b, const FxFields& x, int i, int c,
-                                              double (&out)[5]) {
+                                              i64 (&acc)[5]) {
     const i64* __restrict__ K = x.k;
-    i64 acc[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+    for (int q = 0; q < 5; q++) acc[q] = 0;
     const bool nux = g.nonuniform_x;
     const i64 xp = nux ? __ldg(b.xpk + i) : 0;
     const Fx4 A = fx_load4(x.v + c);
@@ -385,8 +386,11 @@ __device__ __forceinline__ void fx_convective(const Geom& g, const FxBase& b, co
     const i64 phi[4] = {A.x, A.y, A.z, H.y};
 #pragma unroll
     for (int q = 0; q < 4; q++) acc[1 + q] += fx_mulk(fx_mul_by4(phi[q], acc[0]), K[FXK_CTR + q]);
+}
+// their values
+__device__ __forceinline__ void fx_values(const FxFields& x, const i64 (&acc)[5], double (&out)[5]) {
 #pragma unroll
-    for (int q = 0; q < 5; q++) out[q] = (double)acc[q] * fx_unit(K, FXK_A + q, 0);
+    for (int q = 0; q < 5; q++) out[q] = (double)acc[q] * fx_unit(x.k, FXK_A + q, 0);
 }
 
 // The viscous terms: force in out[0..2], conduction, dissipation and work in out[3]

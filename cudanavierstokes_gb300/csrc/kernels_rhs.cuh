@@ -17,6 +17,8 @@
 // which is the same value with 2 instead of l(l+1) pair products per l. The product
 // (rho_a+rho_b)(g_a+g_b) is shared by the mass flux and the four cubic fluxes.
 #pragma once
+#include <algorithm>
+#include <cstdlib>
 #include <type_traits>
 
 #include "cns_common.cuh"
@@ -320,9 +322,11 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
     } else {
         const int c = (int)g.at(i, j, k);
         const double u0 = up.qin.u[c], v0 = up.qin.v[c], w0 = up.qin.w[c];
+        i64 sums[5];
         double acc[5], vis[4];
-        fx_convective<S, CW>(g, cf.fx, in.fx, i, c, acc);
+        fx_convective<S, CW>(g, cf.fx, in.fx, i, c, sums);
         fx_viscous<V>(g, cf.fx, in, quirk, i, c, u0, v0, w0, vis);
+        fx_values(in.fx, sums, acc);
 #pragma unroll
         for (int q = 0; q < 4; q++) acc[1 + q] += vis[q];
         stage_tail<double>(g, up, scal, i, k, c, acc, u0, v0, w0, up.qin.r[c]);
@@ -351,25 +355,27 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 4) k_rhs(Geom g, con
 
 // FP64 on boxes with at most one block of k_rhs per SM, where a thread's dependent chain is the
 // kernel's time: a point takes two threads. The first half of a block's warps form the
-// convective part of its 32 x 2 points and, with the viscous part that the other warps hand over
+// convective part of its 64 points (32 x 2, or 16 x 4 on a narrow box) and, with the viscous part that the other warps hand over
 // in shared memory, the stage update. 14^3 .. 28^3 boxes 14.3 .. 16.4 us against 16.4 .. 18.4; from
 // 32^3 (18.8 us against 18.4) on one thread per point is the faster, on the channel 128x160x192
 // 0.93 ms against 1.12.
-constexpr int SPLIT_ROWS = 2;
+constexpr int SPLIT_POINTS = 64;
 template <int S, int V>
-__global__ void __launch_bounds__(64 * SPLIT_ROWS, 4) k_rhs_split(Geom g, const __grid_constant__ CoefT<double> cf,
+__global__ void __launch_bounds__(2 * SPLIT_POINTS, 4) k_rhs_split(Geom g, const __grid_constant__ CoefT<double> cf,
                                                                   const __grid_constant__ RhsIn<double> in,
                                                                   Update<double> up, double* __restrict__ scal,
                                                                   int quirk) {
-    __shared__ double sv[4][32 * SPLIT_ROWS];
-    const int row = (int)threadIdx.y % SPLIT_ROWS, s = row * 32 + threadIdx.x;
-    const int i = blockIdx.x * 32 + threadIdx.x, j = (int)blockIdx.y * SPLIT_ROWS + row, k = (int)blockIdx.z;
-    const bool inside = i < g.mx && j < g.my, first = threadIdx.y < SPLIT_ROWS;
+    __shared__ double sv[4][SPLIT_POINTS];
+    const int bh = (int)blockDim.y / 2, row = (int)threadIdx.y % bh, s = row * (int)blockDim.x + (int)threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = (int)blockIdx.y * bh + row, k = (int)blockIdx.z;
+    const bool inside = i < g.mx && j < g.my, first = (int)threadIdx.y < bh;
     const int c = (int)g.at(i, j, k);
     double acc[5];
     if (inside) {
         if (first) {
-            fx_convective<S, false>(g, cf.fx, in.fx, i, c, acc);
+            i64 sums[5];
+            fx_convective<S, false>(g, cf.fx, in.fx, i, c, sums);
+            fx_values(in.fx, sums, acc);
         } else {
             double vis[4];
             fx_viscous<V>(g, cf.fx, in, quirk, i, c, up.qin.u[c], up.qin.v[c], up.qin.w[c], vis);
@@ -399,6 +405,30 @@ inline int rhs_band_group(const Geom& g) {
     return fit < 8 ? 8 : (int)fit;
 }
 
+// Block of up to `threads` threads over an x-y plane: bw columns, a tile width that divides mx
+// into equal parts (12 <= bw <= 64 unless mx is smaller), and bh rows, with the fewest warps for
+// the plane and, among equals, bw nearest 32; 32 columns unless that saves 5 % of the warps
+// (rows of 32 coalesce best: 150 x 91 is 2 to 6 % slower in 25 columns at 1 % fewer warps). Fixed
+// 32 x 4 tiles left 24 % of the lanes idle on a 75 x 53 plane, 25 % at mx = 72 or 48, half at 16:
+// FP64 RHS of 72x20x320 158 -> 135 us, 100^3 301 -> 259, 40^3 37 -> 26; FP32 48^3 18.4 -> 14.3.
+struct PlaneTile {
+    int bw, bh;
+};
+inline PlaneTile plane_tile(int mx, int my, int threads) {
+    PlaneTile best{32, threads / 32};
+    const long long wide = (long long)((mx + 31) / 32) * ((my + best.bh - 1) / best.bh) * best.bh;   // in 32 columns
+    long long cost = wide * 19 / 20;
+    for (int n = (mx + 63) / 64; n <= (mx + 11) / 12; n++) {
+        const int bw = (mx + n - 1) / n, bh = std::min(threads / bw, my);
+        const long long c = (long long)((mx + bw - 1) / bw) * ((my + bh - 1) / bh) * ((bw * bh + 31) / 32);
+        if (c < cost || (c == cost && std::abs(bw - 32) < std::abs(best.bw - 32))) {
+            cost = c;
+            best = PlaneTile{bw, bh};
+        }
+    }
+    return best;
+}
+
 // f(S, V) with the orders as integral constants; false: no such instantiation
 template <class F>
 bool rhs_dispatch(int S, int V, F f) {
@@ -418,11 +448,12 @@ bool rhs_dispatch(int S, int V, F f) {
 template <typename R>
 int launch_rhs_t(int S, int V, const Geom& g, const CoefT<R>& cf, const RhsIn<R>& in, const Update<R>& up,
                  double* scal, int quirk, cudaStream_t s) {
-    const int rows = 4 * rhs_band_group(g);   // per launch
+    const PlaneTile t = plane_tile(g.mx, g.my, 128);
+    const int rows = (4 * rhs_band_group(g) + t.bh - 1) / t.bh * t.bh;   // per launch
     int n = 0;
     for (int j0 = 0; j0 < g.my; j0 += rows, n++) {
         const int r = g.my - j0 < rows ? g.my - j0 : rows;
-        const dim3 grid((g.mx + 31) / 32, (r + 3) / 4, g.mz), block(32, 4, 1);
+        const dim3 grid((g.mx + t.bw - 1) / t.bw, (r + t.bh - 1) / t.bh, g.mz), block(t.bw, t.bh, 1);
         if (!rhs_dispatch(S, V, [&](auto s_, auto v_) {
                 k_rhs<R, decltype(s_)::value, decltype(v_)::value><<<grid, block, 0, s>>>(g, cf, in, up, scal, quirk, j0);
             }))
