@@ -104,7 +104,8 @@ void launch_state(const Geom& g, const Phys& ph, const StateIn& q, const Derived
                   int advance_time, double* time_log, long long tcap, cudaStream_t s);
 void launch_advance_time(double* scal, double* time_log, long long tcap, cudaStream_t s);
 template <typename R>
-void launch_ghost_state(const Geom& g, const Phys& ph, const StencilFields<R>& f, const double* scal, cudaStream_t s);
+void launch_ghost_state(const Geom& g, const Phys& ph, const StencilFields<R>& f, double* scal, int adv,
+                        double* time_log, long long tcap, cudaStream_t s);
 template <typename R>
 void launch_ghost_scalar(const Geom& g, R* f, cudaStream_t s);
 // FP32-RHS dilatation (and its ghost images with own) from the packed records (rho, u, v, w)

@@ -24,9 +24,13 @@ __global__ void k_advance_time(double* scal, double* time_log, long long tcap) {
     if (threadIdx.x == 0 && blockIdx.x == 0) advance_time(scal, time_log, tcap);
 }
 
+// adv: the first stage of a step also advances the time here, unless the ghosts depend on it
+// (wall perturbation): one launch fewer per step
 template <typename R>
-__global__ void __launch_bounds__(256) k_ghost_state(Geom g, Phys ph, StencilFields<R> f, const double* scal) {
+__global__ void __launch_bounds__(256) k_ghost_state(Geom g, Phys ph, StencilFields<R> f, double* scal, int adv,
+                                                     double* time_log, long long tcap) {
     const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (adv && t == 0) advance_time(scal, time_log, tcap);
     if (t < ghost_count(g)) ghost_state_cell<R>(g, ph, f, scal, t);
 }
 
@@ -247,8 +251,9 @@ void launch_advance_time(double* scal, double* time_log, long long tcap, cudaStr
     k_advance_time<<<1, 32, 0, s>>>(scal, time_log, tcap);
 }
 template <typename R>
-void launch_ghost_state(const Geom& g, const Phys& ph, const StencilFields<R>& f, const double* scal, cudaStream_t s) {
-    k_ghost_state<R><<<ghost_blocks(g), 256, 0, s>>>(g, ph, f, scal);
+void launch_ghost_state(const Geom& g, const Phys& ph, const StencilFields<R>& f, double* scal, int adv,
+                        double* time_log, long long tcap, cudaStream_t s) {
+    k_ghost_state<R><<<ghost_blocks(g), 256, 0, s>>>(g, ph, f, scal, adv, time_log, tcap);
 }
 template <typename R>
 void launch_ghost_scalar(const Geom& g, R* f, cudaStream_t s) {
@@ -303,8 +308,8 @@ void launch_pack(const Geom& g, const T* src, double* dst, cudaStream_t s) {
 #define CNS_INST(R)                                                                                               \
     template void launch_state<R>(const Geom&, const Phys&, const StateIn&, const DerivedOut<R>&, double*, int,   \
                                   double*, long long, cudaStream_t);                                                        \
-    template void launch_ghost_state<R>(const Geom&, const Phys&, const StencilFields<R>&, const double*,          \
-                                        cudaStream_t);                                                           \
+    template void launch_ghost_state<R>(const Geom&, const Phys&, const StencilFields<R>&, double*, int, double*,  \
+                                        long long, cudaStream_t);                                                \
     template void launch_ghost_scalar<R>(const Geom&, R*, cudaStream_t);                                          \
     template int launch_reduce<R>(const Geom&, const Phys&, const StateIn&, const R*, int, double*, int, double*, \
                                   double*, cudaStream_t);                                                        \

@@ -3,7 +3,7 @@
 // One handle = one simulation resident on one GPU. A time step is
 //   [every check_cfl / check_bulk steps: one fused two-pass reduction for dt, the body
 //    force controller and the bulk diagnostics, all on the device]
-//   k_advance_time, then per Runge-Kutta stage:
+//   then per Runge-Kutta stage (the first one advances the time):
 //     k_ghost_state -> k_fx (the stencil inputs as fixed-point values, theta; FP32-RHS:
 //     k_dil_march, theta only; both write theta's ghost images on periodic and wall
 //     boundaries, the boundary layer adds k_ghost_scalar) -> k_rhs (RHS of x, y, z + body force + sponge + update, and T, p, H,
@@ -155,8 +155,9 @@ int state_phase(cns_solver* h) {
 }
 
 // ghost cells of the stencil inputs of the current state
+// (adv: and the step's time advance, with a time log)
 template <typename R>
-int ghost_phase(cns_solver* h) {
+int ghost_phase(cns_solver* h, bool adv, double* time_log) {
     const int c = h->cur;
     const DerivedOut<R> o = derived_out<R>(h, c);
     StencilFields<R> f{};
@@ -167,7 +168,7 @@ int ghost_phase(cns_solver* h) {
         f.t = o.t; f.p = o.p; f.h = o.h; f.m = o.m;
         f.gmax = h->gmax[c]; f.gnext = h->gmax[1 - c];
     }
-    launch_ghost_state<R>(h->geom, h->phys, f, h->scal, h->stream);
+    launch_ghost_state<R>(h->geom, h->phys, f, h->scal, adv ? 1 : 0, time_log, h->diag_cap, h->stream);
     h->launches += 1;
     CKL();
     return CNS_OK;
@@ -252,8 +253,8 @@ int rhs_phase(cns_solver* h, int kind, double a, double b) {
 int state_any(cns_solver* h) {
     return h->fp32 ? state_phase<float>(h) : state_phase<double>(h);
 }
-int ghost_any(cns_solver* h) {
-    return h->fp32 ? ghost_phase<float>(h) : ghost_phase<double>(h);
+int ghost_any(cns_solver* h, bool adv = false, double* time_log = nullptr) {
+    return h->fp32 ? ghost_phase<float>(h, adv, time_log) : ghost_phase<double>(h, adv, time_log);
 }
 // the derived fields of the current state, recovered unless the last stage did it
 int ensure_state(cns_solver* h) { return h->der_ok[h->cur] ? CNS_OK : state_any(h); }
@@ -304,11 +305,14 @@ int step_stages(cns_solver* h, double* time_log) {
     // the state recovery of each stage's input comes from the previous stage's RHS kernel
     // (ensure_state before the first step)
     for (int s = 0; s < nst; s++) {
-        if (s == 0) {
+        // the time advances before the stages read it: in the ghost kernel, or, where the wall
+        // perturbation there depends on it, in a launch of its own
+        const bool apart = h->p.boundary_layer && h->p.perturbed;
+        if (s == 0 && apart) {
             launch_advance_time(h->scal, time_log, h->diag_cap, h->stream);
             h->launches += 1;
         }
-        if ((rc = ghost_any(h))) return rc;
+        if ((rc = ghost_any(h, s == 0 && !apart, time_log))) return rc;
         if ((rc = grad_any(h))) return rc;
         int kind;
         double a = 0, b = 0;
