@@ -40,12 +40,12 @@ constexpr int DIL_TX = 32, DIL_TY = 8, DIL_NZ = 8;
 
 template <int V>
 __global__ void __launch_bounds__(DIL_TX * DIL_TY) k_dil_march(Geom g, CoefT<float> cf, const float4* __restrict__ qa,
-                                                               float* __restrict__ dil, int own) {
+                                                               float* __restrict__ dil, int own, int nz) {
     __shared__ float su[DIL_TY][DIL_TX + 2 * V];   // u of the tile rows, x halo V on each side
     __shared__ float sv[DIL_TY + 2 * V][DIL_TX];   // v of the tile columns, y halo V on each side
-    const int k0 = blockIdx.z * DIL_NZ;
+    const int k0 = blockIdx.z * nz;
     dil_column_packed<V, DIL_TY>(g, cf, qa, dil, blockIdx.x * DIL_TX, blockIdx.y * DIL_TY, k0,
-                                 min(k0 + DIL_NZ, g.mz), own != 0, (int)threadIdx.x, (int)threadIdx.y, su, sv);
+                                 min(k0 + nz, g.mz), own != 0, (int)threadIdx.x, (int)threadIdx.y, su, sv);
 }
 
 // FP64 mode: fixed-point conversion and theta. Blocks of 32 x 8 threads: the first ones write
@@ -261,13 +261,20 @@ void launch_ghost_scalar(const Geom& g, R* f, cudaStream_t s) {
 }
 void launch_dil_packed(int V, const Geom& g, const CoefT<float>& cf, const float4* qa, float* dil, int own,
                        cudaStream_t s) {
-    const dim3 grid((g.mx + DIL_TX - 1) / DIL_TX, (g.my + DIL_TY - 1) / DIL_TY, (g.mz + DIL_NZ - 1) / DIL_NZ);
+    const int nbx = (g.mx + DIL_TX - 1) / DIL_TX, nby = (g.my + DIL_TY - 1) / DIL_TY;
+    // Planes per block: 8, halved while the tiles would not make two blocks per SM (a plane is a
+    // dependent step of a block). 16^3 9.0 -> 5.8 us, 24^3 9.8 -> 5.7, 48^3 9.7 -> 7.8, 64^3 9.8 -> 7.8. The
+    // line at four blocks per SM was slower (64^3 9.3 us, 75 x 53 x 91 11.7 against 9.8: more z halos), at
+    // one the same (64^3 7.9, 75 x 53 x 91 10.9).
+    int nz = DIL_NZ;
+    while (nz > 1 && (long long)nbx * nby * ((g.mz + nz - 1) / nz) < 2 * 152) nz /= 2;
+    const dim3 grid(nbx, nby, (g.mz + nz - 1) / nz);
     const dim3 block(DIL_TX, DIL_TY, 1);
     switch (V) {
-    case 1: k_dil_march<1><<<grid, block, 0, s>>>(g, cf, qa, dil, own); break;
-    case 2: k_dil_march<2><<<grid, block, 0, s>>>(g, cf, qa, dil, own); break;
-    case 3: k_dil_march<3><<<grid, block, 0, s>>>(g, cf, qa, dil, own); break;
-    default: k_dil_march<4><<<grid, block, 0, s>>>(g, cf, qa, dil, own); break;
+    case 1: k_dil_march<1><<<grid, block, 0, s>>>(g, cf, qa, dil, own, nz); break;
+    case 2: k_dil_march<2><<<grid, block, 0, s>>>(g, cf, qa, dil, own, nz); break;
+    case 3: k_dil_march<3><<<grid, block, 0, s>>>(g, cf, qa, dil, own, nz); break;
+    default: k_dil_march<4><<<grid, block, 0, s>>>(g, cf, qa, dil, own, nz); break;
     }
 }
 // Planes per block: 8, halved while the tiles would not fill the GPU's four blocks per SM

@@ -113,3 +113,20 @@ def test_small_box_kernel(gpu_lib, oracle_mod, mx, my, mz, S, V):
     s.run(2)
     errs = state_errors(s.copy_field_out(), o.get_state())
     assert max(errs) <= TOL64, errs
+
+
+@pytest.mark.parametrize("V", [1, 4])
+def test_dilatation_planes_per_block(gpu_lib, V):
+    """FP32: boxes repeated along z take 1, 2 and 8 planes per block of the dilatation kernel (6
+    tiles a plane, the last block ragged); each copy of the box has the same RHS bit for bit."""
+    def rhs(r):
+        p = tgv_params(33).copy(my=20, mz=14 * r, precision=1, stencil_visc=V)
+        p = p.copy(Lz=p.Lz / 32 * r)
+        s = Solver(p)
+        s.copy_field_in(*[np.tile(f, (r, 1, 1)) for f in base])
+        return s.calc_rhs()
+    base = smooth_random_state(tgv_params(33).copy(my=20, mz=14), seed=3)
+    one = rhs(1)
+    for r in (8, 32):
+        for a, b in zip(one, rhs(r)):
+            assert np.array_equal(np.tile(a, (r, 1, 1)), b)
