@@ -99,7 +99,9 @@ __global__ void __launch_bounds__(256) k_ghost_scalar(Geom g, R* f) {
 // square root, ~60 FP64 instructions; an FP32 estimate of it, within 1e-5 where the internal
 // energy is no small difference, rules out the points that cannot exceed the largest rate found
 // so far, in any block, and few are evaluated in FP64 (channel 128x160x192, a one-step run
-// with its reduction and synchronisation: 0.58 -> 0.27 ms beyond the step).
+// with its reduction and synchronisation: 0.58 -> 0.27 ms beyond the step). Each warp raises the
+// largest rate once: where a thread has one point every rate exceeds the zero it starts from, and
+// an atomic per point serialises at the one address (a one-step run of 77x60x41 230 -> 167 us, FP32).
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -142,8 +144,14 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce_partial(Geom g, Phys ph,
                 const double d2x = dx * dx, md = to_d<R>(mr);
                 const double ci = fmax((fabs(uu) + sos) / dx, fmax((fabs(vv) + sos) * g.dy, (fabs(ww) + sos) * g.dz));
                 const double vi = fmax(md / d2x, fmax(md * g.d2y, md * g.d2z));
-                const double x = fmax(ci, vi);
-                if (x > found) atomicMax(peak, (unsigned long long)__double_as_longlong(x));
+                double x = fmax(ci, vi);
+                if (!(x > found)) x = 0.0;   // NaN too
+                const unsigned mask = __activemask();
+                const unsigned hi = __reduce_max_sync(mask, (unsigned)__double2hiint(x));
+                const unsigned lo =
+                    __reduce_max_sync(mask, (unsigned)__double2hiint(x) == hi ? (unsigned)__double2loint(x) : 0u);
+                const unsigned long long m64 = (unsigned long long)hi << 32 | lo;
+                if ((threadIdx.x & 31) == __ffs(mask) - 1 && m64 > __ldcg(peak)) atomicMax(peak, m64);
             }
         }
         if (want & RED_FORCE) { s_r += rr * wv; s_rw += rr * ww * wv; }
