@@ -12,12 +12,12 @@ path is not sharded across GPUs, each rank advances its own channel).
   e2e         the same through the C ABI with pinned host buffers: copy the five fields
               in, advance K steps, copy them out (host wall clock)
   roofline    the RHS + stage-update kernel (dominant kernel): its event-timed average
-              launch against the FP64 pipe (measured live) and against HBM
+              launch against HBM, with the algorithmic FLOP rate beside the live FP64 peak
   cpu_baseline  the CPU oracle (the reference's algorithm restated, OpenMP) on the host
               cores, on the same full channel (whole RK3 steps for ~12 s)
   fp32_rhs    the same workload with the RHS in FP32 (state/accumulation FP64)
-  pair_rhs    the same workload with the RHS in FP32-pair (~48-bit) arithmetic, and its
-              largest state difference from the FP64 run after the same steps
+  pair_rhs    the same workload with the precision switch at pair (served by the FP64 mode's
+              kernels), and its largest state difference from the FP64 run after the same steps
   batched     48 Taylor-Green boxes of uneven size (seeded), FP32 RHS / FP64 state, in the
               execution mode the autotuner picks (one persistent launch per RK stage for the
               whole ensemble, or every member's step graph on concurrent streams), graph
@@ -362,14 +362,14 @@ def at_time(t, y, t0):
 
 def run_precision(args):
     """The precision study: Taylor-Green to t_end, FP32 RHS (or, with --precision pair, the
-    FP32-pair RHS; FP64 state, accumulation, T/p recovery, reductions in both) against
+    pair mode; FP64 state, accumulation, T/p recovery, reductions in both) against
     all-FP64; relative error of <u.u>, <rho|u|^2>/2, of the dissipation rate eps = -dK/dt at
     t_end (K = <rho|u|^2>/2) and of the viscous dissipation <tau_ij du_i/dx_j> at t_end
     (cns_dissipation)."""
     from cudanavierstokes_gb300.initial import tgv_fields
     from cudanavierstokes_gb300.params import PREC_FP32_RHS, PREC_PAIR_RHS, tgv_params
     n = int(args.grid.split(",")[0]) if args.grid else 128
-    mode, prec, dtype = (("pair_rhs", PREC_PAIR_RHS, "f32x2-rhs/f64-state vs f64") if args.precision == "pair"
+    mode, prec, dtype = (("pair_rhs", PREC_PAIR_RHS, "f64 (pair mode) vs f64") if args.precision == "pair"
                          else ("fp32_rhs", PREC_FP32_RHS, "f32-rhs/f64-state vs f64"))
     p64 = tgv_params(n)
     f = tgv_fields(p64)
@@ -382,7 +382,7 @@ def run_precision(args):
         b, db = at_time(r32["t"], r32[key], args.t_end)
         res[key] = {"fp64": a, mode: b, "rel_err": abs(b - a) / abs(a),
                     "eps_fp64": -da, "eps_" + mode: -db, "eps_rel_err": abs(db - da) / abs(da)}
-    what = "FP32-pair RHS" if prec == PREC_PAIR_RHS else "FP32 RHS"
+    what = "pair mode" if prec == PREC_PAIR_RHS else "FP32 RHS"
     line = {"metric": f"kinetic-energy relative error at t_end, {what} vs FP64", "value": res["ke_rho"]["rel_err"],
             "unit": "relative", "higher_is_better": False, "dtype": dtype,
             "data": "synthetic", "config": {"workload": f"Taylor-Green {n}^3, Ma 0.1, Re 1600, Pr 0.71, S=V=4, "
@@ -519,35 +519,28 @@ def run_gb300(args, world, rank, local):
                                                  native.ctypes.byref(t64)))
     hbm_peak, hbm_src = hbm_peak_gbs()
     traffic = read_traffic(N, fp32=args.precision == "fp32")
-    roof = {"bound": "fp64" if args.precision == "fp64" else "fp32", "kernel": "k_rhs (RHS x/y/z + body force + "
-            "sponge + RK stage update)", "achieved": ach_tf, "peak": t64.value, "unit": "TFLOP/s",
-            "frac": ach_tf / t64.value, "peak_source": "measured live (FMA-chain probe, cns_probe_fma_peak)",
-            "traffic": traffic, "launch_ms": ph["rhs_ms"],
+    # the stencil sums run in 64-bit fixed point on the integer units, so the reference's FP64
+    # operation count over the launch time is an equivalent rate, past what the FP64 pipe can reach
+    roof = {"bound": "hbm", "kernel": "k_rhs (RHS x/y/z + body force + sponge + RK stage update + next-stage state "
+            "recovery)", "achieved": ach_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": ach_gbs / hbm_peak,
+            "peak_source": hbm_src, "traffic": traffic, "launch_ms": ph["rhs_ms"],
             "flops_per_point": rf.fused_rhs_kernel_flops(S, V), "bytes_per_point": rf.RHS_KERNEL_BYTES,
-            "hbm": {"achieved": ach_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": ach_gbs / hbm_peak,
-                    "peak_source": hbm_src},
+            "fp64_equivalent": {"achieved": ach_tf, "peak": t64.value, "unit": "TFLOP/s", "ratio": ach_tf / t64.value,
+                                "peak_source": "measured live (FMA-chain probe, cns_probe_fma_peak)"},
             "phase_ms": ph}
     kv = read_profile_summary()
     if args.precision == "fp32":
         roof = fp32_roofline(N, S, V, ph, t64.value)
-    if args.precision == "pair":
-        # FP64-equivalent rate of the reference's operation count against the FP64 pipe: the
-        # pair arithmetic runs on the FP32 pipe, so frac > 1 is past what FP64 can reach
-        roof["bound"] = "fp32 issue (pair arithmetic)"
-        roof["peak_source"] = "the FP64 pipe peak, measured live (FMA-chain probe): FP64-equivalent comparison"
-        roof["traffic"] = None
-    if args.precision == "fp64" and "fp64_inst_per_point" in kv:
-        # the algorithmic count above is the reference's operation structure; the kernel
-        # executes fewer FP64 instructions (shared flux products, lambda/mu), so the
-        # algorithmic rate can exceed the pipe peak; the pipe utilisation is measured by ncu
+    elif "fp64_inst_per_point" in kv:
         roof["executed"] = {"fp64_inst_per_point": float(kv["fp64_inst_per_point"]),
                             "fp64_pipe_active": float(kv["fp64_pipe_active_pct"]) / 100.0,
+                            "issue_active": float(kv["issue_active_pct"]) / 100.0,
                             "source": "ncu --set full, profiles/rhs_kernel_channel_fp64.md"}
 
     line = {"metric": METRIC, "value": value, "unit": "Mpoint-steps/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None,
-            "dtype": {"fp64": "f64", "fp32": "f32-rhs/f64-state", "pair": "f32x2-rhs/f64-state"}[args.precision],
+            "dtype": {"fp64": "f64", "fp32": "f32-rhs/f64-state", "pair": "f64"}[args.precision],
             "data": "synthetic",
             "config": {"workload": desc, "grid": [p.mx, p.my, p.mz], "points": N,
                        "precision": args.precision, "parallelism": f"replicas x{world}",
@@ -596,7 +589,7 @@ def run_gb300(args, world, rank, local):
                                 "speedup_vs_fp64": (ms / ms32),
                                 "roofline": fp32_roofline(N, S, V, ph32, t32.value)}
             s32.close()
-            # FP32-pair RHS variant: its rate, and its largest state difference from an FP64
+            # pair mode: its rate, and its largest state difference from an FP64
             # run of the same steps from the same start (both fresh solvers)
             pp, _ = workload(args.workload, "pair", args.grid)
             states = []

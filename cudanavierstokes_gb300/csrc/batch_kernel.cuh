@@ -2,8 +2,8 @@
 // advances every instance of a batch (many simulations of different grid sizes and
 // physical parameters sharing the stencil orders and the precision).
 //
-// The launch runs the four stage phases (ghost fill of the stencil inputs, velocity
-// gradients / dilatation, dilatation ghosts, RHS + update + the new state's recovery) over
+// The launch runs the four stage phases (ghost fill of the stencil inputs,
+// dilatation (FP64: with the fixed-point conversion), dilatation ghosts, RHS + update + the new state's recovery) over
 // the work units of all instances, with a grid barrier between phases. Work unit = a
 // 32 x 4 tile of one x-y plane of one instance (point phases, the standalone RHS kernel's
 // block) or 128 ghost cells (ghost phases); units of all instances are numbered
@@ -30,7 +30,7 @@ struct BatchInst {
     double* scal;
     double* tlog;
     long long tcap;          // capacity of tlog
-    RhsIn<R> in[2];          // stencil inputs (+ theta, gradients) of state buffer b
+    RhsIn<R> in[2];          // stencil inputs (+ theta) of state buffer b
     Update<R> up[3][2];      // Wray stage s from state buffer b into 1 - b, with the new
                              // state's recovery (its derived fields of buffer 1 - b)
     int nbx, nby;            // units per plane: ceil(mx/32) x ceil(my/4)

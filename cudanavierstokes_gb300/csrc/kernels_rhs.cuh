@@ -16,6 +16,9 @@
 //   factors) or 1/4 (three factors),
 // which is the same value with 2 instead of l(l+1) pair products per l. The product
 // (rho_a+rho_b)(g_a+g_b) is shared by the mass flux and the four cubic fluxes.
+//
+// FP64 and pair mode: the sums over the neighbours in 64-bit fixed point (kernels_fx.cuh), the
+// stage update and the recovery in FP64. FP32-RHS mode: rhs_point_packed on FP32 records.
 #pragma once
 #include <algorithm>
 #include <cstdlib>
@@ -395,8 +398,8 @@ __global__ void __launch_bounds__(2 * SPLIT_POINTS, 4) k_rhs_split(Geom g, const
 // through L2 alongside) fit in half of L2, else the largest group that does (at least 8
 // bands). Measured on a 512^3 channel, FP32 RHS step: one launch 45.1 ms, groups of 75
 // bands 38.6, 37 bands 36.9, 18 bands 36.9, 9 bands 37.3 ms; on 256^3 one launch (this
-// rule) 4.64 ms, groups of 37 bands 4.69, 18 bands 4.74 ms; the FP64 step is the same
-// either way (FP64-pipe bound).
+// rule) 4.64 ms, groups of 37 bands 4.69, 18 bands 4.74 ms. FP64, a stage on 512 x 512 x 96: one
+// launch 6.75 ms, this rule 5.91.
 inline int rhs_band_group(const Geom& g) {
     const int nby = (g.my + 3) / 4;
     const size_t budget = (size_t)64 << 20, per_band = (size_t)3 * g.G * g.mx * 4 * 72;

@@ -1,5 +1,5 @@
 // peak.cu -- FMA-throughput probe used to state the FP64 / FP32 pipe roofline next to the
-// measured HBM bandwidth (the stencil path is bounded by the FP64 pipe, not by HBM).
+// measured HBM bandwidth.
 #include <cuda_runtime.h>
 
 #include "../../include/cns.h"

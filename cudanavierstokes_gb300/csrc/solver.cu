@@ -177,7 +177,7 @@ int ghost_phase(cns_solver* h, bool adv, double* time_log) {
 template <typename R>
 int grad_phase(cns_solver* h) {
     // every dilatation ghost is a copy of one interior value unless the boundary layer
-    // extrapolates: then the gradient kernel writes them itself
+    // extrapolates: otherwise this phase's kernel writes them itself
     const bool own = h->geom.xbc != XBC_BL && !h->geom.zbl;
     if constexpr (std::is_same<R, float>::value) {   // FP32-RHS: theta alone, from the packed records
         launch_dil_packed(h->p.stencil_visc, h->geom, h->cf32, (const float4*)h->der[h->cur][0], (float*)h->dil,

@@ -195,8 +195,8 @@ CNS_API int cns_set_scalars(cns_solver* h, double dt, double dpdz, double time, 
 
 /* Time `nstages` Runge-Kutta stages (low-storage coefficients, the state advances) phase
  * by phase with CUDA events on the handle's stream. ms[0]: ghost fill of the stencil
- * inputs, ms[1]: velocity gradients + dilatation ghosts, ms[2]: the RHS + stage-update
- * kernel, which also recovers T, p, H, mu of the new state for the next stage; averages
+ * inputs, ms[1]: dilatation and its ghosts (FP64: with the stencil inputs'
+ * conversion to fixed point), ms[2]: the RHS + stage-update kernel, which also recovers T, p, H, mu of the new state for the next stage; averages
  * per stage. No counterpart in the reference (it has no timers, src/main.cpp:71-75). */
 CNS_API int cns_time_phases(cns_solver* h, int nstages, double* ms);
 
