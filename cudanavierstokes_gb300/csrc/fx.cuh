@@ -1,8 +1,8 @@
 // fx.cuh -- 64-bit fixed-point arithmetic of the FP64 mode's stencil sums.
 //
 // On this GPU an FP64 instruction issues to 2 lanes per SM per cycle, a 32 x 32 + 64-bit
-// integer multiply-add to 64 and a 32-bit addition to ~104 (measured), so a stencil sum of
-// FP64 values is ~20 times cheaper on the integer units. A field f with |f| < 2^e over the
+// integer multiply-add to 32 and a 32-bit addition to ~104 (measured), so a term of a weighted
+// sum (two multiply-adds and about four additions) costs a fifth of an FP64 one. A field f with |f| < 2^e over the
 // whole grid, ghosts included, is held as F = f 2^(62 - e), truncated: exact wherever |f| >=
 // 2^(e - 10) (an FP64 value has 53 bits, the format 62), elsewhere within 2^(e - 62), 2^-9 of
 // the rounding of the field's large values. Sums and differences of fields are exact; the
