@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, sizeof(R) == 4 ? 7 : 4)
                     for (int l = 0; l < 5; l++) cf.c1V[d][l] = M.c1V[d][l];
                 cf.xp = M.xp;
                 const int k0 = bz * COL_NZ;
-                dil_column_packed<V, 4>(member_geom(M), cf, M.qa, (float*)M.dil, bx * 32, by * 4, k0,
+                dil_column_packed<V, 4, false>(member_geom(M), cf, M.qa, (float*)M.dil, bx * 32, by * 4, k0,
                                         min(k0 + COL_NZ, M.mz), false, tx, ty, su, sv);
             });
         }

@@ -87,11 +87,25 @@ __host__ __device__ constexpr int fxw2(int K, int k) {
                      : (k == 0 ? -14350 : k == 1 ? 8064 : k == 2 ? -1008 : k == 3 ? 128 : -9)) * (1 << fxs2(K));
 }
 
+// ---- stencil inputs. RO: no thread of the launch writes them (the read-only path, which PTX
+// allows for such data alone); otherwise an earlier phase of the same launch has written them
+// and the loads are ordinary ones, ordered by the barrier between the phases ----
+template <bool RO, typename T>
+__device__ __forceinline__ T ld(const T* p) {
+    if constexpr (RO) return __ldg(p);
+    else return *p;
+}
+
 // ---- four values of a 32-byte record, one load or store ----
 struct __align__(32) Fx4 {
     i64 x, y, z, w;
 };
+template <bool RO>
 __device__ __forceinline__ Fx4 fx_load4(const Fx4* p) {
+    if constexpr (!RO) {
+        const longlong4_32a v = *reinterpret_cast<const longlong4_32a*>(p);
+        return Fx4{v.x, v.y, v.z, v.w};
+    }
     Fx4 r;
     asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(r.x), "=l"(r.y), "=l"(r.z), "=l"(r.w) : "l"(p));
     return r;

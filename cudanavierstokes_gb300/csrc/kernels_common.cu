@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(DIL_TX * DIL_TY) k_dil_march(Geom g, CoefT<flo
     __shared__ float su[DIL_TY][DIL_TX + 2 * V];   // u of the tile rows, x halo V on each side
     __shared__ float sv[DIL_TY + 2 * V][DIL_TX];   // v of the tile columns, y halo V on each side
     const int k0 = blockIdx.z * nz;
-    dil_column_packed<V, DIL_TY>(g, cf, qa, dil, blockIdx.x * DIL_TX, blockIdx.y * DIL_TY, k0,
+    dil_column_packed<V, DIL_TY, true>(g, cf, qa, dil, blockIdx.x * DIL_TX, blockIdx.y * DIL_TY, k0,
                                  min(k0 + nz, g.mz), own != 0, (int)threadIdx.x, (int)threadIdx.y, su, sv);
 }
 

@@ -274,21 +274,21 @@ struct FxConv {
     i64 p, F[5];   // mass flux; u, v, w, H fluxes, doubled
 };
 
-template <int V>
+template <int V, bool RO>
 __device__ __forceinline__ FxVisc fx_visc(const FxFields& in, int c, int st, const i64 (&ctr)[4]) {
     FxSum D[6], L[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) L[q].add(ctr[q], fxw2(V, 0));
 #pragma unroll
     for (int l = 1; l <= V; l++) {
-        const Fx4 am = fx_load4(in.v + c - l * st), ap = fx_load4(in.v + c + l * st);
-        const longlong2 tm = __ldg(in.t + c - l * st), tp = __ldg(in.t + c + l * st);
+        const Fx4 am = fx_load4<RO>(in.v + c - l * st), ap = fx_load4<RO>(in.v + c + l * st);
+        const longlong2 tm = ld<RO>(in.t + c - l * st), tp = ld<RO>(in.t + c + l * st);
         D[0].add(ap.x - am.x, fxw1(V, l));
         D[1].add(ap.y - am.y, fxw1(V, l));
         D[2].add(ap.z - am.z, fxw1(V, l));
         D[3].add(tp.y - tm.y, fxw1(V, l));
         D[4].add(tp.x - tm.x, fxw1(V, l));
-        D[5].add(__ldg(in.th + c + l * st) - __ldg(in.th + c - l * st), fxw1(V, l));
+        D[5].add(ld<RO>(in.th + c + l * st) - ld<RO>(in.th + c - l * st), fxw1(V, l));
         L[0].add(ap.x + am.x, fxw2(V, l));
         L[1].add(ap.y + am.y, fxw2(V, l));
         L[2].add(ap.z + am.z, fxw2(V, l));
@@ -302,13 +302,13 @@ __device__ __forceinline__ FxVisc fx_visc(const FxFields& in, int c, int st, con
     return o;
 }
 
-template <int S, int DIR, bool ROLLED>
+template <int S, int DIR, bool ROLLED, bool RO>
 __device__ __forceinline__ FxConv fx_conv(const FxFields& in, int c, int st, i64 r0, i64 g0) {
     FxSum P, F[5];
 #pragma unroll(ROLLED ? 1 : S)
     for (int l = 1; l <= S; l++) {
-        const Fx4 am = fx_load4(in.v + c - l * st), ap = fx_load4(in.v + c + l * st);
-        const longlong2 hm = __ldg(in.r + c - l * st), hp = __ldg(in.r + c + l * st);
+        const Fx4 am = fx_load4<RO>(in.v + c - l * st), ap = fx_load4<RO>(in.v + c + l * st);
+        const longlong2 hm = ld<RO>(in.r + c - l * st), hp = ld<RO>(in.r + c + l * st);
         P.add(ap.w - am.w, fxw1(S, l));
         const i64 gm = DIR == 0 ? am.x : DIR == 1 ? am.y : am.z;
         const i64 gp = DIR == 0 ? ap.x : DIR == 1 ? ap.y : ap.z;
@@ -352,8 +352,9 @@ __device__ __forceinline__ int fx_bits(i64 v) { return fx_word1(v) ^ (fx_word1(v
 __device__ __forceinline__ int fx_room(int bits) { return max(__clz(bits) - 2, 0); }
 
 // table unit q times 2^-s
+template <bool RO>
 __device__ __forceinline__ double fx_unit(const i64* K, int q, int s) {
-    const double k = __longlong_as_double(K[q]);
+    const double k = __longlong_as_double(ld<RO>(K + q));
     return __hiloint2double(__double2hiint(k) - (s << 20), __double2loint(k));
 }
 
@@ -361,71 +362,81 @@ __device__ __forceinline__ double fx_unit(const i64* K, int q, int s) {
 // share no intermediate value. Bounds in the units of fx_table: gradients < 2^59.8, theta,
 // stress < 2^61.8, grad mu, grad T < 2^60.8, second derivatives < 2^62.3, RHS sums < 2^62.4.
 //
-// The convective and pressure terms as integer sums. ROLLED: the loops over the offsets are not unrolled.
-template <int S, bool ROLLED>
+// BATCH: the persistent batch kernel's form, the loops over the offsets not unrolled and the
+// inputs written by earlier phases of the same launch.
+//
+// The convective and pressure terms as integer sums.
+template <int S, bool BATCH>
 __device__ __forceinline__ void fx_convective(const Geom& g, const FxBase& b, const FxFields& x, int i, int c,
                                               i64 (&acc)[5]) {
-    const i64* __restrict__ K = x.k;
+    constexpr bool RO = !BATCH;
+    const i64* K = x.k;
 #pragma unroll
     for (int q = 0; q < 5; q++) acc[q] = 0;
     const bool nux = g.nonuniform_x;
     const i64 xp = nux ? __ldg(b.xpk + i) : 0;
-    const Fx4 A = fx_load4(x.v + c);
-    const longlong2 H = __ldg(x.r + c);
+    const Fx4 A = fx_load4<RO>(x.v + c);
+    const longlong2 H = ld<RO>(x.r + c);
     const auto conv = [&](const FxConv& o, int d, bool sx) {
         const i64* k = K + d * FXK_DIR;
-        const auto f = [&](i64 v, int q) { return fx_mulk(sx ? fx_mulk(v, xp) : v, k[q]); };
+        const auto f = [&](i64 v, int q) { return fx_mulk(sx ? fx_mulk(v, xp) : v, ld<RO>(k + q)); };
         acc[1 + d] -= f(o.p, FXK_P);
 #pragma unroll
         for (int q = 0; q < 5; q++) acc[q] += f(o.F[q], FXK_F0 + q);
     };
-    conv(fx_conv<S, 0, ROLLED>(x, c, 1, H.x, A.x), 0, nux);
-    conv(fx_conv<S, 1, ROLLED>(x, c, (int)g.P, H.x, A.y), 1, false);
-    conv(fx_conv<S, 2, ROLLED>(x, c, (int)g.PS, H.x, A.z), 2, false);
+    conv(fx_conv<S, 0, BATCH, RO>(x, c, 1, H.x, A.x), 0, nux);
+    conv(fx_conv<S, 1, BATCH, RO>(x, c, (int)g.P, H.x, A.y), 1, false);
+    conv(fx_conv<S, 2, BATCH, RO>(x, c, (int)g.PS, H.x, A.z), 2, false);
     // the cubic fluxes' centre values: phi_0 times half the mass flux
     const i64 phi[4] = {A.x, A.y, A.z, H.y};
 #pragma unroll
-    for (int q = 0; q < 4; q++) acc[1 + q] += fx_mulk(fx_mul_by4(phi[q], acc[0]), K[FXK_CTR + q]);
+    for (int q = 0; q < 4; q++) acc[1 + q] += fx_mulk(fx_mul_by4(phi[q], acc[0]), ld<RO>(K + FXK_CTR + q));
 }
-// their values
-__device__ __forceinline__ void fx_values(const FxFields& x, const i64 (&acc)[5], double (&out)[5]) {
+// the point's RHS from them and the viscous terms (explicit operations: the same bits in every kernel)
+template <bool BATCH>
+__device__ __forceinline__ void fx_values(const FxFields& x, const i64 (&acc)[5], const double (&vis)[4],
+                                          double (&out)[5]) {
 #pragma unroll
-    for (int q = 0; q < 5; q++) out[q] = (double)acc[q] * fx_unit(x.k, FXK_A + q, 0);
+    for (int q = 0; q < 5; q++) {
+        const double v = (double)acc[q], unit = fx_unit<!BATCH>(x.k, FXK_A + q, 0);
+        out[q] = q == 0 ? __dmul_rn(v, unit) : fma(v, unit, vis[q > 0 ? q - 1 : 0]);
+    }
 }
 
 // The viscous terms: force in out[0..2], conduction, dissipation and work in out[3]
-template <int V>
+template <int V, bool BATCH>
 __device__ __forceinline__ void fx_viscous(const Geom& g, const FxBase& b, const RhsIn<double>& in, int quirk, int i,
                                            int c, double u0, double v0, double w0, double (&out)[4]) {
     const FxFields& x = in.fx;
-    const i64* __restrict__ K = x.k;
+    constexpr bool RO = !BATCH;
+    const i64* K = x.k;
     const bool nux = g.nonuniform_x;
     const i64 xp = nux ? __ldg(b.xpk + i) : 0;
-    const Fx4 A = fx_load4(x.v + c);
-    const longlong2 T = __ldg(x.t + c);
+    const Fx4 A = fx_load4<RO>(x.v + c);
+    const longlong2 T = ld<RO>(x.t + c);
     const i64 ctr[4] = {A.x, A.y, A.z, T.x};
     const longlong2 xx = nux ? __ldg(b.xx + i) : make_longlong2(0, 0);
     i64 G[9], dmu[3], dT[3], L[4] = {0, 0, 0, 0};
     const auto visc = [&](const FxVisc& o, int d, bool sx) {
         const i64* k = K + d * FXK_DIR;
-        const auto f = [&](i64 v, int q) { return fx_mulk(sx ? fx_mulk(v, xp) : v, k[q]); };
+        const auto f = [&](i64 v, int q) { return fx_mulk(sx ? fx_mulk(v, xp) : v, ld<RO>(k + q)); };
 #pragma unroll
         for (int q = 0; q < 3; q++) G[3 * d + q] = f(o.d[q], FXK_U + q);
         dmu[d] = f(o.d[3], FXK_MU);
         dT[d] = f(o.d[4], FXK_T);
 #pragma unroll
         for (int q = 0; q < 4; q++)
-            L[q] += fx_mulk(sx ? fx_mul2(xx.x, o.L[q], xx.y, o.d[q < 3 ? q : 4]) : o.L[q], k[FXK_L + q]);
+            L[q] += fx_mulk(sx ? fx_mul2(xx.x, o.L[q], xx.y, o.d[q < 3 ? q : 4]) : o.L[q], ld<RO>(k + FXK_L + q));
         L[d] += f(o.d[5], FXK_TH);
     };
-    visc(fx_visc<V>(x, c, 1, ctr), 0, nux);
-    visc(fx_visc<V>(x, c, (int)g.P, ctr), 1, false);
-    visc(fx_visc<V>(x, c, (int)g.PS, ctr), 2, false);
+    visc(fx_visc<V, RO>(x, c, 1, ctr), 0, nux);
+    visc(fx_visc<V, RO>(x, c, (int)g.P, ctr), 1, false);
+    visc(fx_visc<V, RO>(x, c, (int)g.PS, ctr), 2, false);
     // grad mu and the stress tensor tau / mu, each scaled to the full range
     const int sm = fx_room(fx_bits(dmu[0]) | fx_bits(dmu[1]) | fx_bits(dmu[2]));
 #pragma unroll
     for (int q = 0; q < 3; q++) dmu[q] <<= sm;
-    const i64 th3 = fx_mulk(__ldg(x.th + c), K[FXK_TG]);   // theta / 3
+    const i64 th3 = fx_mulk(ld<RO>(x.th + c), ld<RO>(K + FXK_TG));   // theta / 3
     i64 t[6] = {2 * (G[0] - th3), 2 * (G[4] - th3), 2 * (G[8] - th3), G[1] + G[3], G[2] + G[6], G[5] + G[7]};
     // y-z dissipation with the quirk: tau_yz dv/dz in the y sum as in the z sum (src/cuda_rhs.cu:175)
     i64 q12 = quirk ? 2 * G[7] : t[5];
@@ -436,16 +447,16 @@ __device__ __forceinline__ void fx_viscous(const Geom& g, const FxBase& b, const
     q12 <<= st;
     // dissipation / mu: tau_ab du_b/dx_a = sum t_aa^2 / 2 (the trace of t is zero) + sum t_ab^2
     const i64 diss = (fx_dot3(t[0], t[0], t[1], t[1], t[2], t[2]) >> 1) + fx_dot3(t[3], t[3], t[4], t[4], t[5], q12);
-    const double ud = fx_unit(K, FXK_UD, sm + st);
-    out[0] = fma((double)fx_mul(T.y, L[0]), fx_unit(K, FXK_UL, 0),
+    const double ud = fx_unit<RO>(K, FXK_UD, sm + st);
+    out[0] = fma((double)fx_mul(T.y, L[0]), fx_unit<RO>(K, FXK_UL, 0),
                  (double)fx_dot3(t[0], dmu[0], t[3], dmu[1], t[4], dmu[2]) * ud);
-    out[1] = fma((double)fx_mul(T.y, L[1]), fx_unit(K, FXK_UL + 1, 0),
+    out[1] = fma((double)fx_mul(T.y, L[1]), fx_unit<RO>(K, FXK_UL + 1, 0),
                  (double)fx_dot3(t[3], dmu[0], t[1], dmu[1], t[5], dmu[2]) * ud);
-    out[2] = fma((double)fx_mul(T.y, L[2]), fx_unit(K, FXK_UL + 2, 0),
+    out[2] = fma((double)fx_mul(T.y, L[2]), fx_unit<RO>(K, FXK_UL + 2, 0),
                  (double)fx_dot3(t[4], dmu[0], t[5], dmu[1], t[2], dmu[2]) * ud);
-    double en = (double)fx_mul(T.y, L[3]) * fx_unit(K, FXK_UL + 3, 0);
-    en = fma((double)fx_dot3(dT[0], dmu[0], dT[1], dmu[1], dT[2], dmu[2]), fx_unit(K, FXK_UC, sm), en);
-    en = fma(in.m[c], (double)diss * fx_unit(K, FXK_UE, 2 * st), en);
+    double en = (double)fx_mul(T.y, L[3]) * fx_unit<RO>(K, FXK_UL + 3, 0);
+    en = fma((double)fx_dot3(dT[0], dmu[0], dT[1], dmu[1], dT[2], dmu[2]), fx_unit<RO>(K, FXK_UC, sm), en);
+    en = fma(in.m[c], (double)diss * fx_unit<RO>(K, FXK_UE, 2 * st), en);
     out[3] = fma(u0, out[0], fma(v0, out[1], fma(w0, out[2], en)));
 }
 

@@ -348,21 +348,22 @@ __device__ __forceinline__ long long ghost_vel_cell(const Geom& g, const Phys& p
 
 // FP32-RHS dilatation from the packed records qa = (rho, u, v, w): the diagonal gradients
 // du/dx, dv/dy, dw/dz at the viscous order (derVelX/Y/Z, src/calc_stress.cu:20-63) and theta
-// (calcDil, src/calc_stress.cu:87-96).
+// (calcDil, src/calc_stress.cu:87-96). The persistent batch kernel's form: its ghost phase
+// writes qa in the same launch.
 template <int V>
 __device__ __forceinline__ void dil_point_packed(const Geom& g, const CoefT<float>& cf,
-                                                 const float4* __restrict__ qa, float* __restrict__ dil, int i, int j,
+                                                 const float4* qa, float* dil, int i, int j,
                                                  int k, bool own = false) {
     const int c = (int)g.at(i, j, k);
     const int P = (int)g.P, PS = (int)g.PS;
-    float sx = cf.c1V[0][1] * (__ldg(qa + c + 1).y - __ldg(qa + c - 1).y);
-    float sy = cf.c1V[1][1] * (__ldg(qa + c + P).z - __ldg(qa + c - P).z);
-    float sz = cf.c1V[2][1] * (__ldg(qa + c + PS).w - __ldg(qa + c - PS).w);
+    float sx = cf.c1V[0][1] * (ld<false>(qa + c + 1).y - ld<false>(qa + c - 1).y);
+    float sy = cf.c1V[1][1] * (ld<false>(qa + c + P).z - ld<false>(qa + c - P).z);
+    float sz = cf.c1V[2][1] * (ld<false>(qa + c + PS).w - ld<false>(qa + c - PS).w);
 #pragma unroll
     for (int kk = 2; kk <= V; kk++) {
-        sx = fma(cf.c1V[0][kk], __ldg(qa + c + kk).y - __ldg(qa + c - kk).y, sx);
-        sy = fma(cf.c1V[1][kk], __ldg(qa + c + kk * P).z - __ldg(qa + c - kk * P).z, sy);
-        sz = fma(cf.c1V[2][kk], __ldg(qa + c + kk * PS).w - __ldg(qa + c - kk * PS).w, sz);
+        sx = fma(cf.c1V[0][kk], ld<false>(qa + c + kk).y - ld<false>(qa + c - kk).y, sx);
+        sy = fma(cf.c1V[1][kk], ld<false>(qa + c + kk * P).z - ld<false>(qa + c - kk * P).z, sy);
+        sz = fma(cf.c1V[2][kk], ld<false>(qa + c + kk * PS).w - ld<false>(qa + c - kk * PS).w, sz);
     }
     if (g.nonuniform_x) sx *= cf.xp[i];
     const float th = sx + sy + sz;
@@ -376,15 +377,15 @@ __device__ __forceinline__ void dil_point_packed(const Geom& g, const CoefT<floa
 // row tile su, v into the y-halo column tile sv in shared memory) and the record V planes
 // ahead, whose w enters a register ring holding w at k - V .. k + V; threads at the tile
 // edges also load the x and y halos; the next plane's loads are issued before the current
-// plane is computed. About 2 + 2V/TY + 2V/32 record loads per point instead of the 6V of a
+// plane is computed (RO: ld, fx.cuh). About 2 + 2V/TY + 2V/32 record loads per point instead of the 6V of a
 // point-per-thread stencil (each record is 16 bytes of which one value is used); the
 // arithmetic per point is dil_point_packed's: the same sums in the same order. Tile
 // slots outside [-V, mx + V) x [-V, my + V) are never read by an interior point and are not
 // loaded; every loaded slot lies in the ghosted allocation (G = S >= V). All threads of the
 // block call it (it synchronises the block).
-template <int V, int TY>
-__device__ __forceinline__ void dil_column_packed(const Geom& g, const CoefT<float>& cf, const float4* __restrict__ qa,
-                                                  float* __restrict__ dil, int i0, int j0, int k0, int k1, bool own,
+template <int V, int TY, bool RO>
+__device__ __forceinline__ void dil_column_packed(const Geom& g, const CoefT<float>& cf, const float4* qa,
+                                                  float* dil, int i0, int j0, int k0, int k1, bool own,
                                                   int tx, int ty, float (*su)[32 + 2 * V], float (*sv)[32]) {
     static_assert(V <= TY, "the y halo rows are loaded by the first and last V tile rows");
     const int i = i0 + tx, j = j0 + ty;
@@ -397,21 +398,21 @@ __device__ __forceinline__ void dil_column_packed(const Geom& g, const CoefT<flo
     // w at planes k - V .. k + V (ring[V] = the current plane)
     float ring[2 * V + 1];
 #pragma unroll
-    for (int l = 0; l < 2 * V; l++) ring[l] = inside ? __ldg(qa + c0 + (k0 - V + l) * PS).w : 0.0f;
+    for (int l = 0; l < 2 * V; l++) ring[l] = inside ? ld<RO>(qa + c0 + (k0 - V + l) * PS).w : 0.0f;
     // the loads of plane k: w at k + V, the own record's u and v, the x and y halos
     float nw = 0.f, nu = 0.f, nv = 0.f, hxl = 0.f, hxr = 0.f, hyl = 0.f, hyr = 0.f;
     const auto fetch = [&](int k) {
         const int ck = c0 + k * PS;
-        nw = inside ? __ldg(qa + ck + V * PS).w : 0.0f;
+        nw = inside ? ld<RO>(qa + ck + V * PS).w : 0.0f;
         if (ghosted) {
-            const float4 rec = __ldg(qa + ck);
+            const float4 rec = ld<RO>(qa + ck);
             nu = rec.y;
             nv = rec.z;
         }
-        if (tx < V && j < g.my) hxl = __ldg(qa + ck - V).y;                           // x = i - V >= -V
-        if (tx >= 32 - V && i < g.mx && j < g.my) hxr = __ldg(qa + ck + V).y;          // x = i + V < mx + V
-        if (ty < V && i < g.mx) hyl = __ldg(qa + ck - V * P).z;                       // y = j - V >= -V
-        if (ty >= TY - V && j < g.my && i < g.mx) hyr = __ldg(qa + ck + V * P).z;      // y = j + V < my + V
+        if (tx < V && j < g.my) hxl = ld<RO>(qa + ck - V).y;                           // x = i - V >= -V
+        if (tx >= 32 - V && i < g.mx && j < g.my) hxr = ld<RO>(qa + ck + V).y;          // x = i + V < mx + V
+        if (ty < V && i < g.mx) hyl = ld<RO>(qa + ck - V * P).z;                       // y = j - V >= -V
+        if (ty >= TY - V && j < g.my && i < g.mx) hyr = ld<RO>(qa + ck + V * P).z;      // y = j + V < my + V
     };
     if (k0 < k1) fetch(k0);
     for (int k = k0; k < k1; k++) {

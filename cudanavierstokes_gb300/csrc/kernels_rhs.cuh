@@ -152,7 +152,8 @@ __device__ __forceinline__ void stage_tail(const Geom& g, const Update<R>& up, d
 // are scaled by the direction's inverse spacing (or its square) afterwards; the flux sums
 // carry neither 1/2, 1/4 nor 1/dx, which the final combination applies. The batched stage
 // kernel uses this form: its members' coefficients would otherwise come through shared
-// memory and occupy registers. The standalone kernel reads the premultiplied tables from
+// memory and occupy registers. There the inputs are also written by earlier phases of the same
+// launch, so this form loads them by ordinary loads (ld, fx.cuh). The standalone kernel reads the premultiplied tables from
 // its launch parameters (constant bank operands).
 template <int S, int V, int DIR, bool CW>
 __device__ __forceinline__ void rhs_dir_packed(const Geom& g, const CoefT<float>& cf, const RhsIn<float>& in, int c,
@@ -186,10 +187,10 @@ __device__ __forceinline__ void rhs_dir_packed(const Geom& g, const CoefT<float>
           fw = (nux || CW) ? 0.f : acc[3], fe = (nux || CW) ? 0.f : acc[4];
 #pragma unroll
     for (int l = 1; l <= S; l++) {
-        const float4 Ap = __ldg(in.qa + c + l * st), Am = __ldg(in.qa + c - l * st);
-        const float4 Bp = __ldg(in.qb + c + l * st), Bm = __ldg(in.qb + c - l * st);
+        const float4 Ap = ld<!CW>(in.qa + c + l * st), Am = ld<!CW>(in.qa + c - l * st);
+        const float4 Bp = ld<!CW>(in.qb + c + l * st), Bm = ld<!CW>(in.qb + c - l * st);
         if (l <= V) {
-            const float thp = __ldg(in.dil + c + l * st), thm = __ldg(in.dil + c - l * st);
+            const float thp = ld<!CW>(in.dil + c + l * st), thm = ld<!CW>(in.dil + c - l * st);
             if (l == 1) {
                 gu = w1V(1) * (Ap.y - Am.y); gv = w1V(1) * (Ap.z - Am.z); gw = w1V(1) * (Ap.w - Am.w);
                 dmu = w1V(1) * (Bp.w - Bm.w); dT = w1V(1) * (Bp.x - Bm.x); dth = w1V(1) * (thp - thm);
@@ -278,8 +279,8 @@ __device__ __forceinline__ void rhs_point_packed(const Geom& g, const CoefT<floa
                                                  const Update<float>& up, double* __restrict__ scal, int quirk, int i,
                                                  int j, int k) {
     const int c = (int)g.at(i, j, k);
-    const float4 A0 = __ldg(in.qa + c), B0 = __ldg(in.qb + c);
-    const float th0 = __ldg(in.dil + c);
+    const float4 A0 = ld<!CW>(in.qa + c), B0 = ld<!CW>(in.qb + c);
+    const float th0 = ld<!CW>(in.dil + c);
     const float r0 = A0.x, u0 = A0.y, v0 = A0.z, w0 = A0.w;
     const float T0 = B0.x, h0 = B0.z, m0 = B0.w;
     const float m3 = m0 * (float)(1.0 / 3.0);
@@ -328,10 +329,8 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
         i64 sums[5];
         double acc[5], vis[4];
         fx_convective<S, CW>(g, cf.fx, in.fx, i, c, sums);
-        fx_viscous<V>(g, cf.fx, in, quirk, i, c, u0, v0, w0, vis);
-        fx_values(in.fx, sums, acc);
-#pragma unroll
-        for (int q = 0; q < 4; q++) acc[1 + q] += vis[q];
+        fx_viscous<V, CW>(g, cf.fx, in, quirk, i, c, u0, v0, w0, vis);
+        fx_values<CW>(in.fx, sums, vis, acc);
         stage_tail<double>(g, up, scal, i, k, c, acc, u0, v0, w0, up.qin.r[c]);
     }
 }
@@ -373,15 +372,13 @@ __global__ void __launch_bounds__(2 * SPLIT_POINTS, 4) k_rhs_split(Geom g, const
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = (int)blockIdx.y * bh + row, k = (int)blockIdx.z;
     const bool inside = i < g.mx && j < g.my, first = (int)threadIdx.y < bh;
     const int c = (int)g.at(i, j, k);
-    double acc[5];
+    i64 sums[5];
+    double acc[5], vis[4];
     if (inside) {
         if (first) {
-            i64 sums[5];
             fx_convective<S, false>(g, cf.fx, in.fx, i, c, sums);
-            fx_values(in.fx, sums, acc);
         } else {
-            double vis[4];
-            fx_viscous<V>(g, cf.fx, in, quirk, i, c, up.qin.u[c], up.qin.v[c], up.qin.w[c], vis);
+            fx_viscous<V, false>(g, cf.fx, in, quirk, i, c, up.qin.u[c], up.qin.v[c], up.qin.w[c], vis);
 #pragma unroll
             for (int q = 0; q < 4; q++) sv[q][s] = vis[q];
         }
@@ -389,7 +386,8 @@ __global__ void __launch_bounds__(2 * SPLIT_POINTS, 4) k_rhs_split(Geom g, const
     __syncthreads();
     if (!inside || !first) return;
 #pragma unroll
-    for (int q = 0; q < 4; q++) acc[1 + q] += sv[q][s];
+    for (int q = 0; q < 4; q++) vis[q] = sv[q][s];
+    fx_values<false>(in.fx, sums, vis, acc);
     stage_tail<double>(g, up, scal, i, k, c, acc, up.qin.u[c], up.qin.v[c], up.qin.w[c], up.qin.r[c]);
 }
 
