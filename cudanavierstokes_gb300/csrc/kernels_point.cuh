@@ -450,6 +450,14 @@ __device__ __forceinline__ void dil_column_packed(const Geom& g, const CoefT<flo
 
 // Dilatation ghost cell t (BCxNumber2 / BCyNumber1 / BCzNumber1): x periodic | wall:
 // even | boundary layer: bottom even, top extrapolated; y periodic; z periodic | extrapolated.
+//
+// Range of the fixed-point theta (long long, |theta| < 3 x 2^59.8 inside): an extrapolated image
+// 2 a - b stays below 9 x 2^59.8 = 2^62.9, and so does the difference of two values on either
+// side of a point, which is what the sums take. A direction's part of theta is at most 2^59.8
+// where its velocity and the velocity's own images, which the field's exponent covers, keep below
+// 2^62: the part along the axis of extrapolation contributes at most 4 of these units (2 theta_0 -
+// theta_-m - theta_-n), a transverse one 2, since |2 u_0 - u_-m| < 2^62 as well, and 3 beside
+// wall images that are not (the perturbed wall, the corner of two extrapolated faces).
 template <typename R>
 __device__ __forceinline__ void ghost_scalar_cell(const Geom& g, R* f, int t) {
     const GhostCell gc = ghost_cell_of(g, t);
