@@ -42,8 +42,8 @@ struct StencilFields {
 };
 
 // per stage: the integer factors of the sums, 16 per direction (velocity gradients, grad mu,
-// grad T, grad theta / 3, grad p, second derivatives of u, v, w, T, mass flux, fluxes of u, v,
-// w, H); of the centre terms; units as doubles (fx_table)
+// grad T, grad theta / 3 and grad p as doubles, second derivatives of u, v, w, T, mass flux, fluxes
+// of u, v, w, H); of the centre terms; units as doubles (fx_table)
 enum { FXK_U = 0, FXK_MU = 3, FXK_T = 4, FXK_TH = 5, FXK_P = 6, FXK_L = 7, FXK_LT = 10, FXK_F0 = 11, FXK_F = 12,
        FXK_DIR = 16, FXK_CTR = 48, FXK_A = 52, FXK_UL = 57, FXK_UD = 61, FXK_UC = 62, FXK_UE = 63, FXK_TG = 64,
        FXK_COUNT = 65 };

@@ -54,6 +54,11 @@ __device__ __forceinline__ i64 fx_mul_by4(i64 a, i64 b) {
     return (fx_mad(ah, bh, 0) << 2) + (m >> 30);
 }
 
+// magnitude bits of the high word, and the left shift that brings the largest of several
+// values (the OR of their bits) to [2^61, 2^62), or by 30
+__device__ __forceinline__ int fx_bits(i64 v) { return fx_word1(v) ^ (fx_word1(v) >> 31); }
+__device__ __forceinline__ int fx_room(int bits) { return max(__clz(bits) - 2, 0); }
+
 // sum of products a_k w_k / 2^32 with small-integer weights: two accumulators, the high
 // halves' and the low halves'. With |a| < 2^63 and sum |w| <= 2^30.8 both stay below 2^61.8.
 struct FxSum {
@@ -64,6 +69,16 @@ struct FxSum {
         l = fx_mad(fx_lo(a), w, l);
     }
     __device__ __forceinline__ i64 value() const { return h + (i64)fx_word1(l); }
+    // value() 2^s, s the room that it leaves (fx_room, below 32), filled from the low sum: a first
+    // derivative's weights are multiples of 2^21, so where the fields' values are exact the whole
+    // sum is, however close the neighbours are
+    __device__ __forceinline__ i64 normal(int& s) const {
+        const i64 r = l - FX_HALF, v = h + (i64)fx_word1(r);
+        s = fx_room(fx_bits(v));
+        const unsigned lo = __funnelshift_l((unsigned)r, (unsigned)v, s);
+        const unsigned hi = __funnelshift_l((unsigned)v, (unsigned)(v >> 32), s);
+        return (i64)((unsigned long long)hi << 32 | lo);
+    }
     __device__ __forceinline__ i64 twice() const { return (h << 1) + ((l - FX_HALF / 2) >> 31); }
 };
 

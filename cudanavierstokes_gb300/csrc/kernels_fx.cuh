@@ -94,22 +94,16 @@ static __device__ __noinline__ i64 fx_table(const FxBase& b, const unsigned* gma
     const auto ev = [&](int q) { return q == 1 ? e[1] : q == 2 ? e[2] : q == 3 ? e[3] : e[6]; };   // u, v, w, H
     const auto big = [&](int q) { return fx_larger(K(0, q), fx_larger(K(1, q), K(2, q))); };
     // units (2^64 / FX_FULL of the largest factor): the gradients' power of two, above 4 times
-    // their largest factor; the mass sum; the sum of equation q with its centre term's factor;
-    // second derivatives of component q (with grad theta / 3)
+    // their largest factor; the mass sum; the fluxes of equation q with its centre term's factor;
+    // second derivatives of component q
     const int xg = fx_log2(fx_larger(big(FXK_U), fx_larger(big(FXK_U + 1), big(FXK_U + 2)))) + 3;
     const double U0 = big(FXK_F0) * (0x1p64 / FX_FULL);
     const auto ctr = [&](int q) { return fx_scaled(U0, ev(q) - 1); };
     const auto UA = [&](int q) {
         if (q == 0) return U0;
-        double m = fx_larger(big(FXK_F0 + q), ctr(q));
-        if (q < 4) m = fx_larger(m, K(q - 1, FXK_P));
-        return m * (0x1p64 / FX_FULL);
+        return fx_larger(big(FXK_F0 + q), ctr(q)) * (0x1p64 / FX_FULL);
     };
-    const auto UL = [&](int q) {
-        double m = big(FXK_L + q);
-        if (q < 3) m = fx_larger(m, K(q, FXK_TH));
-        return m * (0x1p64 / FX_FULL);
-    };
+    const auto UL = [&](int q) { return big(FXK_L + q) * (0x1p64 / FX_FULL); };
     const double UM = big(FXK_MU) * (0x1p64 / FX_FULL), UT = big(FXK_T) * (0x1p64 / FX_FULL);
     const auto factor = [&](double k, double unit) {   // low word, balanced high half
         const i64 v = __double2ll_rn(k / unit * 0x1p64);
@@ -117,8 +111,10 @@ static __device__ __noinline__ i64 fx_table(const FxBase& b, const unsigned* gma
     };
     if (t < 3 * FXK_DIR) {
         const int d = t / FXK_DIR, q = t % FXK_DIR;
-        const double u = q < FXK_MU ? fx_pow2(xg) : q == FXK_MU ? UM : q == FXK_T ? UT : q == FXK_TH ? UL(d)
-                         : q == FXK_P ? UA(1 + d) : q <= FXK_LT ? UL(q - FXK_L) : UA(q - FXK_F0);
+        if (q == FXK_P) return __double_as_longlong(K(d, q));
+        if (q == FXK_TH) return __double_as_longlong(fx_scaled(K(d, q), e[7] + 2));   // with mu
+        const double u = q < FXK_MU ? fx_pow2(xg) : q == FXK_MU ? UM : q == FXK_T ? UT
+                         : q <= FXK_LT ? UL(q - FXK_L) : UA(q - FXK_F0);
         return factor(K(d, q), u);
     }
     if (t == FXK_TG) return factor(fx_scaled(1.0 / 3.0, xth), fx_pow2(xg));
@@ -272,6 +268,7 @@ struct FxVisc {
 };
 struct FxConv {
     i64 p, F[5];   // mass flux; u, v, w, H fluxes, doubled
+    int ps;        // p is 2^ps times the sum
 };
 
 template <int V, bool RO>
@@ -324,7 +321,7 @@ __device__ __forceinline__ FxConv fx_conv(const FxFields& in, int c, int st, i64
         }
     }
     FxConv o;
-    o.p = P.value();
+    o.p = P.normal(o.ps);
 #pragma unroll
     for (int q = 0; q < 5; q++) o.F[q] = q == 0 ? F[q].value() : F[q].twice();
     return o;
@@ -346,10 +343,6 @@ __device__ __forceinline__ i64 fx_dot3(i64 a0, i64 b0, i64 a1, i64 b1, i64 a2, i
     const i64 o = fx_mad(a2h, fx_lo(b2), fx_mad(fx_lo(a2), b2h, FX_HALF));
     return fx_mad(a0h, b0h, fx_mad(a1h, b1h, fx_mad(a2h, b2h, (i64)fx_word1(m) + fx_word1(n) + fx_word1(o))));
 }
-// magnitude bits of the high word, and the left shift that brings the largest of several
-// values (the OR of their bits) to [2^61, 2^62)
-__device__ __forceinline__ int fx_bits(i64 v) { return fx_word1(v) ^ (fx_word1(v) >> 31); }
-__device__ __forceinline__ int fx_room(int bits) { return max(__clz(bits) - 2, 0); }
 
 // table unit q times 2^-s
 template <bool RO>
@@ -365,14 +358,19 @@ __device__ __forceinline__ double fx_unit(const i64* K, int q, int s) {
 // BATCH: the persistent batch kernel's form, the loops over the offsets not unrolled and the
 // inputs written by earlier phases of the same launch.
 //
-// The convective and pressure terms as integer sums.
+// The convective and pressure terms. Neither grad p nor grad theta (fx_viscous) joins an integer
+// sum: their largest possible values would set its unit, and where a velocity component is far
+// smaller than the others or than the speed of sound, its fluxes and second derivatives would
+// lose bits (spanwise velocity 2^-15 of the stream: joined, its equation was off by 7.6e-12 of its
+// maximum, FP64 sums 8.9e-14; a stage on the channel 128x160x192 1.15 -> 1.20 ms). dp and the sums meet in FP64
+// here, before the viscous part, which holds fewer registers than after it (1.20 against 1.23 ms).
 template <int S, bool BATCH>
 __device__ __forceinline__ void fx_convective(const Geom& g, const FxBase& b, const FxFields& x, int i, int c,
-                                              i64 (&acc)[5]) {
+                                              double (&out)[5]) {
     constexpr bool RO = !BATCH;
     const i64* K = x.k;
-#pragma unroll
-    for (int q = 0; q < 5; q++) acc[q] = 0;
+    i64 acc[5] = {0, 0, 0, 0, 0};
+    double dp[3];
     const bool nux = g.nonuniform_x;
     const i64 xp = nux ? __ldg(b.xpk + i) : 0;
     const Fx4 A = fx_load4<RO>(x.v + c);
@@ -380,7 +378,7 @@ __device__ __forceinline__ void fx_convective(const Geom& g, const FxBase& b, co
     const auto conv = [&](const FxConv& o, int d, bool sx) {
         const i64* k = K + d * FXK_DIR;
         const auto f = [&](i64 v, int q) { return fx_mulk(sx ? fx_mulk(v, xp) : v, ld<RO>(k + q)); };
-        acc[1 + d] -= f(o.p, FXK_P);
+        dp[d] = __dmul_rn((double)(sx ? fx_mulk(o.p, xp) : o.p), fx_unit<RO>(k, FXK_P, o.ps));
 #pragma unroll
         for (int q = 0; q < 5; q++) acc[q] += f(o.F[q], FXK_F0 + q);
     };
@@ -391,15 +389,10 @@ __device__ __forceinline__ void fx_convective(const Geom& g, const FxBase& b, co
     const i64 phi[4] = {A.x, A.y, A.z, H.y};
 #pragma unroll
     for (int q = 0; q < 4; q++) acc[1 + q] += fx_mulk(fx_mul_by4(phi[q], acc[0]), ld<RO>(K + FXK_CTR + q));
-}
-// the point's RHS from them and the viscous terms (explicit operations: the same bits in every kernel)
-template <bool BATCH>
-__device__ __forceinline__ void fx_values(const FxFields& x, const i64 (&acc)[5], const double (&vis)[4],
-                                          double (&out)[5]) {
 #pragma unroll
     for (int q = 0; q < 5; q++) {
-        const double v = (double)acc[q], unit = fx_unit<!BATCH>(x.k, FXK_A + q, 0);
-        out[q] = q == 0 ? __dmul_rn(v, unit) : fma(v, unit, vis[q > 0 ? q - 1 : 0]);
+        const double v = (double)acc[q], unit = fx_unit<RO>(K, FXK_A + q, 0);
+        out[q] = q == 0 || q == 4 ? __dmul_rn(v, unit) : fma(v, unit, -dp[q > 0 ? q - 1 : 0]);
     }
 }
 
@@ -417,6 +410,8 @@ __device__ __forceinline__ void fx_viscous(const Geom& g, const FxBase& b, const
     const i64 ctr[4] = {A.x, A.y, A.z, T.x};
     const longlong2 xx = nux ? __ldg(b.xx + i) : make_longlong2(0, 0);
     i64 G[9], dmu[3], dT[3], L[4] = {0, 0, 0, 0};
+    // mu/3 grad theta, apart from the second derivatives for the same reason as grad p
+    double th[3];
     const auto visc = [&](const FxVisc& o, int d, bool sx) {
         const i64* k = K + d * FXK_DIR;
         const auto f = [&](i64 v, int q) { return fx_mulk(sx ? fx_mulk(v, xp) : v, ld<RO>(k + q)); };
@@ -427,7 +422,8 @@ __device__ __forceinline__ void fx_viscous(const Geom& g, const FxBase& b, const
 #pragma unroll
         for (int q = 0; q < 4; q++)
             L[q] += fx_mulk(sx ? fx_mul2(xx.x, o.L[q], xx.y, o.d[q < 3 ? q : 4]) : o.L[q], ld<RO>(k + FXK_L + q));
-        L[d] += f(o.d[5], FXK_TH);
+        const int s = fx_room(fx_bits(o.d[5]));
+        th[d] = __dmul_rn((double)fx_mul(T.y, sx ? fx_mulk(o.d[5] << s, xp) : o.d[5] << s), fx_unit<RO>(k, FXK_TH, s));
     };
     visc(fx_visc<V, RO>(x, c, 1, ctr), 0, nux);
     visc(fx_visc<V, RO>(x, c, (int)g.P, ctr), 1, false);
@@ -449,11 +445,11 @@ __device__ __forceinline__ void fx_viscous(const Geom& g, const FxBase& b, const
     const i64 diss = (fx_dot3(t[0], t[0], t[1], t[1], t[2], t[2]) >> 1) + fx_dot3(t[3], t[3], t[4], t[4], t[5], q12);
     const double ud = fx_unit<RO>(K, FXK_UD, sm + st);
     out[0] = fma((double)fx_mul(T.y, L[0]), fx_unit<RO>(K, FXK_UL, 0),
-                 (double)fx_dot3(t[0], dmu[0], t[3], dmu[1], t[4], dmu[2]) * ud);
+                 fma((double)fx_dot3(t[0], dmu[0], t[3], dmu[1], t[4], dmu[2]), ud, th[0]));
     out[1] = fma((double)fx_mul(T.y, L[1]), fx_unit<RO>(K, FXK_UL + 1, 0),
-                 (double)fx_dot3(t[3], dmu[0], t[1], dmu[1], t[5], dmu[2]) * ud);
+                 fma((double)fx_dot3(t[3], dmu[0], t[1], dmu[1], t[5], dmu[2]), ud, th[1]));
     out[2] = fma((double)fx_mul(T.y, L[2]), fx_unit<RO>(K, FXK_UL + 2, 0),
-                 (double)fx_dot3(t[4], dmu[0], t[5], dmu[1], t[2], dmu[2]) * ud);
+                 fma((double)fx_dot3(t[4], dmu[0], t[5], dmu[1], t[2], dmu[2]), ud, th[2]));
     double en = (double)fx_mul(T.y, L[3]) * fx_unit<RO>(K, FXK_UL + 3, 0);
     en = fma((double)fx_dot3(dT[0], dmu[0], dT[1], dmu[1], dT[2], dmu[2]), fx_unit<RO>(K, FXK_UC, sm), en);
     en = fma(in.m[c], (double)diss * fx_unit<RO>(K, FXK_UE, 2 * st), en);

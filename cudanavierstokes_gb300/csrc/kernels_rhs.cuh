@@ -326,11 +326,11 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
     } else {
         const int c = (int)g.at(i, j, k);
         const double u0 = up.qin.u[c], v0 = up.qin.v[c], w0 = up.qin.w[c];
-        i64 sums[5];
         double acc[5], vis[4];
-        fx_convective<S, CW>(g, cf.fx, in.fx, i, c, sums);
+        fx_convective<S, CW>(g, cf.fx, in.fx, i, c, acc);
         fx_viscous<V, CW>(g, cf.fx, in, quirk, i, c, u0, v0, w0, vis);
-        fx_values<CW>(in.fx, sums, vis, acc);
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[1 + q] = __dadd_rn(acc[1 + q], vis[q]);
         stage_tail<double>(g, up, scal, i, k, c, acc, u0, v0, w0, up.qin.r[c]);
     }
 }
@@ -372,12 +372,12 @@ __global__ void __launch_bounds__(2 * SPLIT_POINTS, 4) k_rhs_split(Geom g, const
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = (int)blockIdx.y * bh + row, k = (int)blockIdx.z;
     const bool inside = i < g.mx && j < g.my, first = (int)threadIdx.y < bh;
     const int c = (int)g.at(i, j, k);
-    i64 sums[5];
-    double acc[5], vis[4];
+    double acc[5];
     if (inside) {
         if (first) {
-            fx_convective<S, false>(g, cf.fx, in.fx, i, c, sums);
+            fx_convective<S, false>(g, cf.fx, in.fx, i, c, acc);
         } else {
+            double vis[4];
             fx_viscous<V, false>(g, cf.fx, in, quirk, i, c, up.qin.u[c], up.qin.v[c], up.qin.w[c], vis);
 #pragma unroll
             for (int q = 0; q < 4; q++) sv[q][s] = vis[q];
@@ -386,8 +386,7 @@ __global__ void __launch_bounds__(2 * SPLIT_POINTS, 4) k_rhs_split(Geom g, const
     __syncthreads();
     if (!inside || !first) return;
 #pragma unroll
-    for (int q = 0; q < 4; q++) vis[q] = sv[q][s];
-    fx_values<false>(in.fx, sums, vis, acc);
+    for (int q = 0; q < 4; q++) acc[1 + q] = __dadd_rn(acc[1 + q], sv[q][s]);
     stage_tail<double>(g, up, scal, i, k, c, acc, up.qin.u[c], up.qin.v[c], up.qin.w[c], up.qin.r[c]);
 }
 

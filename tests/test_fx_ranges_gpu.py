@@ -3,9 +3,9 @@ import numpy as np
 import pytest
 
 from cudanavierstokes_gb300 import Solver
-from cudanavierstokes_gb300.batch import Batch
-from cudanavierstokes_gb300.params import Derived, boundary_layer_params
-from tests._util import field_errors, state_errors
+from cudanavierstokes_gb300.params import Derived, boundary_layer_params, tgv_params
+from tests._rhs_ref import derived, rhs
+from tests._util import field_errors
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +50,59 @@ def test_dilatation_at_extrapolated_ends(gpu_lib, oracle_mod, S):
     s.copy_field_in(*f)
     errs = field_errors(s.calc_rhs(), o.rhs())
     assert max(errs) <= TOL64, errs
+
+
+def _uniform_pressure(p, u, v, w):
+    """rho = 1 and an internal energy of 64, with velocities whose squares the energy holds exactly: the
+    recovered T, p and mu are the same number at every point, and a small component's equation is its own terms alone."""
+    one = np.ones(p.shape)
+    f = [one, *(np.ascontiguousarray(a * one) for a in (u, v, w))]
+    return f + [64.0 + 0.5 * (f[1] * f[1] + f[2] * f[2] + f[3] * f[3])]
+
+
+def _modes(p, rng, n=3, along=(1, 1, 1)):
+    z, y, x = np.meshgrid(*(2 * np.pi * (np.arange(m) + 0.5) / m for m in p.shape), indexing="ij")
+    f = np.zeros(p.shape)
+    for _ in range(n):
+        k, ph = rng.integers(1, 3, size=3), rng.uniform(0, 2 * np.pi, size=3)
+        for a, q, c in zip((x, y, z), range(3), along):
+            f += c * rng.uniform(0.1, 0.3) * np.sin(k[q] * a + ph[q])
+        f += rng.uniform(-0.3, 0.3) * np.sin(along[0] * k[0] * x + ph[0]) * np.sin(along[2] * k[2] * z + ph[2]) * (
+            np.cos(k[1] * y + ph[1]) if along[1] else 1.0)
+    return f
+
+
+def _grain(f, bits):
+    return np.round(f * 2.0 ** bits) * 2.0 ** -bits
+
+
+def _small_component(kind):
+    """`thin`: a shear layer with a wall-normal spacing 24 and 96 times finer than the others and
+    cross velocities 2^-10 of the stream. `span`: a two-dimensional flow with a spanwise velocity
+    2^-15 of it."""
+    p = tgv_params(16).copy(my=16, mz=24, Re=100.0, viscexp=1.0)
+    p = p.copy(Ma=float(np.sqrt(1.0 / (p.gam * (p.gam - 1.0) * 64.0))))   # T = 1
+    rng = np.random.default_rng(5)
+    if kind == "thin":
+        p = p.copy(Lx=p.Lz * 16 / 24 / 96, Ly=p.Lz * 16 / 24 / 4)
+        u, v = (_grain(_modes(p, rng), 10) * 2.0 ** -10 for _ in range(2))
+        w = _grain(1.0 + 0.1 * _modes(p, rng), 20)
+    else:
+        u, w = (_grain(0.5 * _modes(p, rng, along=(1, 0, 1)), 10) for _ in range(2))
+        v = _grain(_modes(p, rng), 7) * 2.0 ** -15
+    return p, _uniform_pressure(p, u, v, w)
+
+
+@pytest.mark.parametrize("kind", ["thin", "span"])
+def test_small_components_keep_their_own_scale(gpu_lib, kind):
+    """Each equation against the same sums in extended precision, relative to its own maximum: no
+    further off than twice the sums in plain FP64 are, or than 8 roundings of that maximum."""
+    p, f = _small_component(kind)
+    t = derived(p, f, np.float64)[4]
+    assert (t == t.flat[0]).all()   # the state is what it is meant to be
+    exact = rhs(p, f)
+    plain = field_errors(rhs(p, f, np.float64), exact)
+    s = Solver(p)
+    s.copy_field_in(*f)
+    errs = field_errors(s.calc_rhs(), exact)
+    assert all(a <= max(2 * b, 8 * 2.0 ** -53) for a, b in zip(errs, plain)), (errs, plain)
