@@ -395,11 +395,19 @@ __global__ void __launch_bounds__(BATCH_THREADS, sizeof(R) == 4 ? 7 : 4)
             if (i < I.g.mx && j < I.g.my) dil_point_packed<V>(I.g, I.cf, in.qa, (float*)in.dil, i, j, k);
         } else {
             int e[8];
-            fx_exponents(in.fx.gmax, e);
+            const bool wide = !fx_exponents(I.cf.fx, in.fx.gmax, e);
             if (u == ctl->unit_off[q] && threadIdx.x < FXK_COUNT)
                 in.fx.k[threadIdx.x] =
                     fx_table(I.cf.fx, in.fx.gmax, I.cf.lam_mu, (int)threadIdx.x);
-            if (i < I.g.mx && j < I.g.my) fx_point<V>(I.g, I.cf.fx, in, e, I.cf.xp, i, j, k);
+            if (i < I.g.mx && j < I.g.my) {
+                FxLeast least;
+                if (wide) {
+                    const int c = (int)I.g.at(i, j, k);
+                    wide_theta<V, false>(I.g, I.cf, in, i, j, k, false);
+                    least.add(in.r[c], in.t[c]);
+                } else fx_point<V>(I.g, I.cf.fx, in, e, I.cf.xp, i, j, k, least);
+                least.raise(in.fx.gnext);
+            }
         }
     });
     grid_barrier(bar, nb, err);
@@ -413,9 +421,12 @@ __global__ void __launch_bounds__(BATCH_THREADS, sizeof(R) == 4 ? 7 : 4)
             ghost_scalar_cell<R>(I.g, (R*)I.in[cur].dil, (int)t);
         } else {
             int e[8];
-            fx_exponents(I.in[cur].fx.gmax, e);
-            ghost_scalar_cell<i64>(I.g, I.in[cur].fx.th, (int)t);
-            fx_ghost(I.g, I.in[cur], e, (int)t);
+            const bool wide = !fx_exponents(I.cf.fx, I.in[cur].fx.gmax, e);
+            if (wide) ghost_scalar_cell<double>(I.g, (double*)I.in[cur].fx.th, (int)t);
+            else ghost_scalar_cell<i64>(I.g, I.in[cur].fx.th, (int)t);
+            FxLeast least;
+            fx_ghost(I.g, I.in[cur], e, (int)t, wide, least);
+            least.raise(I.in[cur].fx.gnext);
         }
     });
     grid_barrier(bar, nb, err);

@@ -67,6 +67,7 @@ struct Phys {
 struct FxBase {
     double b1V[3], b1S[3], b2[3], b1V3[3];   // b1V3 = b1V / 3
     double th[3], thmax;                     // b1V without the metric; th[0] at the largest 1/x'
+    int span_T;                              // binades of T that the sums serve (fx_exponents)
     const longlong2* xx;    // [mx] factors of f'' and f' (index derivatives) in the second derivative
     const long long* xpk;   // [mx] 1/x' as a factor (low word, balanced high half), the largest 2^63 (1 - 2^-20)
 };

@@ -28,7 +28,7 @@ struct StateOut {
 // neighbour costs two vector loads (and one address each) instead of eight scalar loads.
 template <typename R>
 struct DerivedOut {
-    unsigned* gmax;     // FP64 mode: the fields' maxima (fx_track, fx.cuh)
+    unsigned* gmax;     // FP64 mode: the fields' ranges (FX_SLOTS, fx_track, fx.cuh)
     R *h, *t, *p, *m;   // FP64 mode
     float4 *qa, *qb;    // FP32-RHS mode
 };
@@ -38,24 +38,26 @@ template <typename R>
 struct StencilFields {
     R *r, *u, *v, *w, *t, *p, *h, *m;   // FP64 mode
     float4 *qa, *qb;                    // FP32-RHS mode (packed, see DerivedOut)
-    unsigned *gmax, *gnext;             // FP64 mode: maxima of these fields; of the next state
+    unsigned *gmax, *gnext;             // FP64 mode: ranges of these fields; of the next state's
 };
 
 // per stage: the integer factors of the sums, 16 per direction (velocity gradients, grad mu,
 // grad T, grad theta / 3 and grad p as doubles, second derivatives of u, v, w, T, mass flux, fluxes
-// of u, v, w, H); of the centre terms; units as doubles (fx_table)
+// of u, v, w, H); of the centre terms; units as doubles; whether
+// the stage takes FP64 sums instead (fx_table)
 enum { FXK_U = 0, FXK_MU = 3, FXK_T = 4, FXK_TH = 5, FXK_P = 6, FXK_L = 7, FXK_LT = 10, FXK_F0 = 11, FXK_F = 12,
        FXK_DIR = 16, FXK_CTR = 48, FXK_A = 52, FXK_UL = 57, FXK_UD = 61, FXK_UC = 62, FXK_UE = 63, FXK_TG = 64,
-       FXK_COUNT = 65 };
+       FXK_WIDE = 65, FXK_COUNT = 66 };
 
 // FP64 mode: the ghosted stencil inputs as 64-bit fixed-point records, (u, v, w, p), (T, mu),
-// (rho, H), theta, and the stage's scale factors
+// (rho, H), theta (on a stage with FP64 sums its doubles, and nothing else), and the stage's scale
+// factors
 struct FxFields {
     Fx4* v;
     longlong2 *t, *r;
     long long* th;
     long long* k;
-    unsigned *gmax, *gnext;   // maxima of this state's fields; of the next state's
+    unsigned *gmax, *gnext;   // ranges of this state's fields; of the next state's
 };
 
 // RHS stage kernel inputs (FP64: separate fields and their fixed-point form; FP32-RHS: the
@@ -106,8 +108,9 @@ void launch_advance_time(double* scal, double* time_log, long long tcap, cudaStr
 template <typename R>
 void launch_ghost_state(const Geom& g, const Phys& ph, const StencilFields<R>& f, double* scal, int adv,
                         double* time_log, long long tcap, cudaStream_t s);
-template <typename R>
-void launch_ghost_scalar(const Geom& g, R* f, cudaStream_t s);
+// theta's ghost images: FP32-RHS; FP64 (th as the ranges' slots say, fx_table)
+void launch_ghost_theta(const Geom& g, float* th, cudaStream_t s);
+void launch_ghost_theta(const Geom& g, const FxFields& fx, cudaStream_t s);
 // FP32-RHS dilatation (and its ghost images with own) from the packed records (rho, u, v, w)
 void launch_dil_packed(int V, const Geom& g, const CoefT<float>& cf, const float4* qa, float* dil, int own,
                        cudaStream_t s);

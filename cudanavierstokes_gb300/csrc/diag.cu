@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 
 #include "../../include/cns.h"
 #include "cns_internal.h"
@@ -26,16 +27,15 @@ constexpr int DG_THREADS = 128;   // 32 x 4 points of a plane per block
 constexpr int DG_NZ = 8;          // planes per block
 constexpr int DG_FINAL = 512;
 
-// warp maximum of the three magnitudes' high words into the slots, where it exceeds them
-__device__ __forceinline__ void vel_track(unsigned* slots, double u, double v, double w) {
+// warp maximum of the three magnitudes' codes into the slots, where it exceeds them
+__device__ __forceinline__ void vel_track(unsigned* slots, unsigned u, unsigned v, unsigned w) {
     const unsigned mask = __activemask();
-    const double f[3] = {u, v, w};
+    const unsigned f[3] = {u, v, w};
     const bool first = (threadIdx.x & 31) == __ffs(mask) - 1;
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-        const unsigned h = (unsigned)__double2hiint(f[q]) & 0x7fffffffu;
-        if (!__any_sync(mask, h > __ldcg(slots + q))) continue;
-        const unsigned m = __reduce_max_sync(mask, h);
+        if (!__any_sync(mask, f[q] > __ldcg(slots + q))) continue;
+        const unsigned m = __reduce_max_sync(mask, f[q]);
         if (first) atomicMax(slots + q, m);
     }
 }
@@ -47,21 +47,18 @@ __global__ void __launch_bounds__(256) k_ghost_vel(Geom g, Phys ph, double* u, d
     const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (t >= ghost_count(g)) return;
     const long long c = ghost_vel_cell(g, ph, u, v, w, scal, t);
-    vel_track(vmax, u[c], v[c], w[c]);
+    vel_track(vmax, fx_code(u[c]), fx_code(v[c]), fx_code(w[c]));
 }
 __global__ void __launch_bounds__(256) k_vel_max(Geom g, const double* __restrict__ u, const double* __restrict__ v,
                                                  const double* __restrict__ w, unsigned* vmax) {
     const unsigned n = (unsigned)g.mx * (unsigned)g.my * (unsigned)g.mz, mx = (unsigned)g.mx, my = (unsigned)g.my;
-    double m[3] = {0, 0, 0};
+    unsigned m[3] = {0, 0, 0};
     for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const unsigned jk = t / mx, k = jk / my;
         const long long c = g.at((int)(t - jk * mx), (int)(jk - k * my), (int)k);
-        const double f[3] = {u[c], v[c], w[c]};
-#pragma unroll
-        for (int q = 0; q < 3; q++) {   // the larger magnitude by its bits
-            const unsigned a = (unsigned)__double2hiint(f[q]) & 0x7fffffffu, b = (unsigned)__double2hiint(m[q]);
-            if (a > b) m[q] = __hiloint2double((int)a, 0);
-        }
+        m[0] = max(m[0], fx_code(u[c]));
+        m[1] = max(m[1], fx_code(v[c]));
+        m[2] = max(m[2], fx_code(w[c]));
     }
     vel_track(vmax, m[0], m[1], m[2]);
 }
@@ -85,39 +82,51 @@ __global__ void __launch_bounds__(DG_THREADS, 4) k_dissip(Geom g, Phys ph, const
 #pragma unroll
         for (int n = 0; n < 3; n++) {
             e[n] = fx_exponent(vmax[n]);
-            ok = ok && fx_valid(e[n]);
+            ok = ok && fx_valid(vmax[n]);
         }
         const double b[3] = {g.nonuniform_x ? bx * xp[i] : bx, by, bz};
         const double* F[3] = {q.u, q.v, q.w};
-        for (int k = k0; k < k1; k++) {
-            const long long c = g.at(i, j, k);
-            const long long st[3] = {1, g.P, g.PS};
-            double G[9];   // G[3 d + n] = d u_n / d x_d (derVelX/Y/Z)
+        const auto column = [&](auto fixed) {
+            for (int k = k0; k < k1; k++) {
+                const long long c = g.at(i, j, k);
+                const long long st[3] = {1, g.P, g.PS};
+                double G[9];   // G[3 d + n] = d u_n / d x_d (derVelX/Y/Z)
 #pragma unroll
-            for (int d = 0; d < 3; d++) {
+                for (int d = 0; d < 3; d++) {
 #pragma unroll
-                for (int n = 0; n < 3; n++) {
-                    const double* f = F[n];
-                    FxSum s;
+                    for (int n = 0; n < 3; n++) {
+                        const double* f = F[n];
+                        if constexpr (decltype(fixed)::value) {
+                            FxSum s;
 #pragma unroll
-                    for (int l = 1; l <= V; l++)
-                        s.add(fx_from(f[c + l * st[d]], e[n]) - fx_from(f[c - l * st[d]], e[n]), fxw1(V, l));
-                    G[3 * d + n] = (double)s.value() * (b[d] * fx_pow2(e[n] - 62));
+                            for (int l = 1; l <= V; l++)
+                                s.add(fx_from(f[c + l * st[d]], e[n]) - fx_from(f[c - l * st[d]], e[n]), fxw1(V, l));
+                            G[3 * d + n] = (double)s.value() * (b[d] * fx_pow2(e[n] - 62));
+                        } else {
+                            double s = 0.0;
+#pragma unroll
+                            for (int l = 1; l <= V; l++)
+                                s = fma((double)fxw1(V, l), f[c + l * st[d]] - f[c - l * st[d]], s);
+                            G[3 * d + n] = s * (b[d] * 0x1p-32);
+                        }
+                    }
                 }
+                const double rr = q.r[c], uu = q.u[c], vv = q.v[c], ww = q.w[c], ee = q.e[c];
+                const double en = ee * rcp_nr(rr) - 0.5 * (uu * uu + vv * vv + ww * ww);
+                const double T = ph.cvInv * en;
+                const double mu = (ph.vexp_is_one ? T : pow_visc(T, ph.vexp)) * ph.invRe;
+                const double th = G[0] + G[4] + G[8];
+                const double a = G[1] + G[3], bb = G[2] + G[6], cc = G[5] + G[7];
+                const double wx = G[5] - G[7], wy = G[6] - G[2], wz = G[1] - G[3];
+                double s = fma(2.0, fma(G[0], G[0], fma(G[4], G[4], G[8] * G[8])), fma(a, a, fma(bb, bb, cc * cc)));
+                s = fma(-(2.0 / 3.0) * th, th, s);
+                phi = fma(mu, s, phi);
+                ens += fma(wx, wx, fma(wy, wy, wz * wz));
             }
-            const double rr = q.r[c], uu = q.u[c], vv = q.v[c], ww = q.w[c], ee = q.e[c];
-            const double en = ee * rcp_nr(rr) - 0.5 * (uu * uu + vv * vv + ww * ww);
-            const double T = ph.cvInv * en;
-            const double mu = (ph.vexp_is_one ? T : pow_visc(T, ph.vexp)) * ph.invRe;
-            const double th = G[0] + G[4] + G[8];
-            const double a = G[1] + G[3], bb = G[2] + G[6], cc = G[5] + G[7];
-            const double wx = G[5] - G[7], wy = G[6] - G[2], wz = G[1] - G[3];
-            double s = fma(2.0, fma(G[0], G[0], fma(G[4], G[4], G[8] * G[8])), fma(a, a, fma(bb, bb, cc * cc)));
-            s = fma(-(2.0 / 3.0) * th, th, s);
-            phi = fma(mu, s, phi);
-            ens += fma(wx, wx, fma(wy, wy, wz * wz));
-        }
-        const double wv = ok ? g.wvol[i] : __longlong_as_double(0x7ff8000000000000LL);
+        };
+        if (ok) column(std::true_type());
+        else column(std::false_type());   // out of the format's range (fx_valid): FP64 gradients
+        const double wv = g.wvol[i];
         phi *= wv;
         ens *= wv;
     }

@@ -12,7 +12,8 @@
 //
 // Ranges. |F| < 2^62 (1 - 2^-21) (fx_exponent), so the sum or difference of two fields fits
 // 63 bits and its balanced high half (below) 31 bits; every 64-bit accumulator's bound is
-// noted where it is formed.
+// noted where it is formed. Fields whose range is too wide for this take FP64 sums instead
+// (fx_exponents, kernels_fx.cuh).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -130,15 +131,17 @@ __device__ __forceinline__ void fx_store4(Fx4* p, i64 x, i64 y, i64 z, i64 w) {
 }
 
 // ---- exponents ----
-// e with |f| < 2^e (1 - 2^-21) from the largest high word (sign cleared) of a field's
-// values. Magnitudes below 2^-300 count as 2^-300; above 2^300, infinities and NaN make the
-// state invalid (fx_valid), as they make the FP64 arithmetic overflow.
+// The exponent code E of a value is that of the power of two above it: |f| < 2^(E - 1022) (1 -
+// 2^-21); 0 for values that count as zero. fx_valid: the sums serve fields of zeros and of largest
+// magnitudes from 2^-300 to 2^300; others, infinities and NaN take FP64 sums.
 constexpr int FX_EMAX = 300;
-__device__ __forceinline__ int fx_exponent(unsigned hw) {
-    const int e = (int)(hw >> 20) - 1022 + ((hw & 0xfffffu) == 0xfffffu ? 1 : 0);
-    return e < -FX_EMAX ? -FX_EMAX : e;
+__device__ __forceinline__ unsigned fx_code(double x) {
+    return (((unsigned)__double2hiint(x) & 0x7fffffffu) + 1u) >> 20;
 }
-__device__ __forceinline__ bool fx_valid(int e) { return e <= FX_EMAX; }
+__device__ __forceinline__ int fx_exponent(unsigned code) { return max((int)code - 1022, -FX_EMAX); }
+__device__ __forceinline__ bool fx_valid(unsigned code) {
+    return code == 0 || code - (1022 - FX_EMAX) <= 2 * FX_EMAX;
+}
 
 // x 2^(62 - e), |x| < 2^e, truncated towards zero, on the integer units
 __device__ __forceinline__ i64 fx_from(double x, int e) {
@@ -158,26 +161,68 @@ __device__ __forceinline__ double fx_pow2(int a) {
     return __hiloint2double((min(max(a, -1022), 1023) + 1023) << 20, 0);
 }
 
-// ---- maxima: slots of the eight fields (rho, u, v, w, T, p, H, mu), the largest high words
-// seen. Reads first: a warp issues atomics only while it raises a slot. ----
-__device__ __forceinline__ void fx_track(unsigned* slots, const double (&f)[8]) {
+// ---- ranges of the fields: 16 slots of a state, raised by the kernels that form it. 0..7: the
+// largest codes of rho, u, v, w, T, p, H, mu. 8, 9: of rho and T the largest 2048 minus the exponent
+// field, which gives the smallest magnitude's; the conversion finds these for the next stage (in
+// the recovery of every point they made a 64^3 box 6 % slower), the state kernel for its own state.
+// 0 is an empty slot. Reads first, one request, as the slots are one address for all warps: a warp
+// issues atomics only while it raises a slot, which is rare as codes are exponents alone. ----
+constexpr int FX_SLOTS = 16, FX_LEAST = 8;
+constexpr int FX_SPAN = 3;   // binades of rho and T (fx_exponents, kernels_fx.cuh)
+__device__ __forceinline__ void fx_slots(const unsigned* slots, unsigned (&m)[8]) {
+    i64 r[4];
+    asm volatile("ld.global.cg.v4.b64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(r[0]), "=l"(r[1]), "=l"(r[2]), "=l"(r[3]) : "l"(slots) : "memory");
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        m[2 * q] = (unsigned)r[q];
+        m[2 * q + 1] = (unsigned)(r[q] >> 32);
+    }
+}
+template <int N>
+__device__ __forceinline__ void fx_raise(unsigned* slots, const unsigned (&h)[N]) {
     const unsigned mask = __activemask();
-    const uint4 a = __ldcg((const uint4*)slots), b = __ldcg((const uint4*)slots + 1);
-    const unsigned cur[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    unsigned h[8];
+    unsigned cur[8];
+    fx_slots(slots, cur);
     bool up = false;
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-        h[q] = (unsigned)__double2hiint(f[q]) & 0x7fffffffu;
-        up |= h[q] > cur[q];
-    }
+    for (int q = 0; q < N; q++) up |= h[q] > cur[q];
     if (!__any_sync(mask, up)) return;
     const bool first = (threadIdx.y * blockDim.x + threadIdx.x) % 32 == __ffs(mask) - 1;
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
+    for (int q = 0; q < N; q++) {
         const unsigned m = __reduce_max_sync(mask, h[q]);
         if (first && m > cur[q]) atomicMax(slots + q, m);
     }
 }
+__device__ __forceinline__ void fx_track(unsigned* slots, const double (&f)[8]) {
+    unsigned h[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) h[q] = fx_code(f[q]);
+    fx_raise(slots, h);
+}
+// the smallest magnitudes' high words of rho and T, over any number of points
+struct FxLeast {
+    unsigned r = 0x7fffffffu, t = 0x7fffffffu;
+    __device__ __forceinline__ void add(double rho, double T) {
+        r = min(r, (unsigned)__double2hiint(rho) & 0x7fffffffu);
+        t = min(t, (unsigned)__double2hiint(T) & 0x7fffffffu);
+    }
+    __device__ __forceinline__ void raise(unsigned* slots) const {
+        const unsigned m[2] = {2048u - (r >> 20), 2048u - (t >> 20)};
+        fx_raise(slots + FX_LEAST, m);
+    }
+    // once per block of whole warps, called by all its threads (tid); sh: two words of it; seen: slot
+    // tid as it was some time before (the read would lengthen a small box's kernel by 1 us here)
+    __device__ __forceinline__ void raise_block(unsigned* slots, unsigned* sh, int tid, unsigned seen) const {
+        if (tid < 2) sh[tid] = 0u;
+        __syncthreads();
+        const unsigned mr = __reduce_max_sync(0xffffffffu, 2048u - (r >> 20));
+        const unsigned mt = __reduce_max_sync(0xffffffffu, 2048u - (t >> 20));
+        if (tid % 32 < 2) atomicMax(sh + tid % 32, tid % 32 == 0 ? mr : mt);
+        __syncthreads();
+        if (tid < 2 && sh[tid] > seen) atomicMax(slots + FX_LEAST + tid, sh[tid]);
+    }
+};
 
 }  // namespace cns

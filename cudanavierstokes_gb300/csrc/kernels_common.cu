@@ -54,35 +54,57 @@ __global__ void __launch_bounds__(DIL_TX * DIL_TY) k_dil_march(Geom g, CoefT<flo
 // 256 ghost cells each.
 constexpr int FX_TABLE_BLOCKS = (FXK_COUNT + DIL_TY - 1) / DIL_TY;
 template <int V>
-__global__ void __launch_bounds__(DIL_TX * DIL_TY, 4) k_fx(Geom g, const __grid_constant__ FxBase b,
-                                                           const __grid_constant__ RhsIn<double> in,
-                                                           const double* __restrict__ xp, double lam_mu, int own,
-                                                           int tiles, int nbx, int nby, int nz) {
+__global__ void __launch_bounds__(DIL_TX * DIL_TY, 4) k_fx(const __grid_constant__ Geom g,
+                                                           const __grid_constant__ CoefT<double> cf,
+                                                           const __grid_constant__ RhsIn<double> in, int own, int tiles,
+                                                           int nbx, int nby, int nz) {
     __shared__ i64 su[DIL_TY][DIL_TX + 2 * V];   // u of the tile rows, x halo V on each side
     __shared__ i64 sv[DIL_TY + 2 * V][DIL_TX];   // v of the tile columns, y halo V on each side
+    __shared__ unsigned sl[2];
     const int tid = threadIdx.y * DIL_TX + threadIdx.x;
+    const unsigned seen = tid < 2 ? __ldcg(in.fx.gnext + FX_LEAST + tid) : 0u;
     int e[8];
-    fx_exponents(in.fx.gmax, e);   // out of range: the factors are NaN
+    const bool wide = !fx_exponents(cf.fx, in.fx.gmax, e);
     int t = (int)blockIdx.x - FX_TABLE_BLOCKS;
     if (t < 0) {   // an entry per warp: the entries' branches differ, one warp would take them in turn
         const int q = blockIdx.x * DIL_TY + threadIdx.y;
-        if (threadIdx.x == 0 && q < FXK_COUNT) in.fx.k[q] = fx_table(b, in.fx.gmax, lam_mu, q);
+        if (threadIdx.x == 0 && q < FXK_COUNT) in.fx.k[q] = fx_table(cf.fx, in.fx.gmax, cf.lam_mu, q);
         return;
     }
     if (t >= tiles) {
         t = (t - tiles) * DIL_TX * DIL_TY + tid;
-        if (t < ghost_count(g)) fx_ghost(g, in, e, t);
+        FxLeast least;
+        if (t < ghost_count(g)) fx_ghost(g, in, e, t, wide, least);
+        least.raise_block(in.fx.gnext, sl, tid, seen);
         return;
     }
     const int r = t / nbx, bz = r / nby, k0 = bz * nz;
-    fx_column<V, DIL_TY>(g, b, in, e, xp, (t - r * nbx) * DIL_TX, (r - bz * nby) * DIL_TY, k0, min(k0 + nz, g.mz),
-                         own != 0, (int)threadIdx.x, (int)threadIdx.y, su, sv);
+    const int i0 = (t - r * nbx) * DIL_TX, j0 = (r - bz * nby) * DIL_TY, k1 = min(k0 + nz, g.mz);
+    FxLeast least;
+    if (wide) {
+        const int i = i0 + (int)threadIdx.x, j = j0 + (int)threadIdx.y;
+        if (i < g.mx && j < g.my)
+            for (int k = k0; k < k1; k++) {
+                const int c = (int)g.at(i, j, k);
+                wide_theta<V, true>(g, cf, in, i, j, k, own != 0);
+                least.add(in.r[c], in.t[c]);
+            }
+    } else {
+        fx_column<V, DIL_TY>(g, cf.fx, in, e, cf.xp, i0, j0, k0, k1, own != 0, (int)threadIdx.x, (int)threadIdx.y, su, sv,
+                             least);
+    }
+    least.raise_block(in.fx.gnext, sl, tid, seen);
 }
 
-template <typename R>
-__global__ void __launch_bounds__(256) k_ghost_scalar(Geom g, R* f) {
+__global__ void __launch_bounds__(256) k_ghost_theta(Geom g, float* th) {
     const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (t < ghost_count(g)) ghost_scalar_cell<R>(g, f, t);
+    if (t < ghost_count(g)) ghost_scalar_cell<float>(g, th, t);
+}
+__global__ void __launch_bounds__(256) k_ghost_theta(Geom g, FxFields fx) {
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (t >= ghost_count(g)) return;
+    if (fx.k[FXK_WIDE] == 0) ghost_scalar_cell<i64>(g, fx.th, t);
+    else ghost_scalar_cell<double>(g, (double*)fx.th, t);
 }
 
 // ---------------------------------------------------------------------------------
@@ -263,9 +285,9 @@ void launch_ghost_state(const Geom& g, const Phys& ph, const StencilFields<R>& f
                         double* time_log, long long tcap, cudaStream_t s) {
     k_ghost_state<R><<<ghost_blocks(g), 256, 0, s>>>(g, ph, f, scal, adv, time_log, tcap);
 }
-template <typename R>
-void launch_ghost_scalar(const Geom& g, R* f, cudaStream_t s) {
-    k_ghost_scalar<R><<<ghost_blocks(g), 256, 0, s>>>(g, f);
+void launch_ghost_theta(const Geom& g, float* th, cudaStream_t s) { k_ghost_theta<<<ghost_blocks(g), 256, 0, s>>>(g, th); }
+void launch_ghost_theta(const Geom& g, const FxFields& fx, cudaStream_t s) {
+    k_ghost_theta<<<ghost_blocks(g), 256, 0, s>>>(g, fx);
 }
 void launch_dil_packed(int V, const Geom& g, const CoefT<float>& cf, const float4* qa, float* dil, int own,
                        cudaStream_t s) {
@@ -295,10 +317,10 @@ void launch_fx(int V, const Geom& g, const CoefT<double>& cf, const RhsIn<double
     const unsigned grid = FX_TABLE_BLOCKS + (unsigned)tiles + ghost_blocks(g);
     const dim3 block(DIL_TX, DIL_TY, 1);
     switch (V) {
-    case 1: k_fx<1><<<grid, block, 0, s>>>(g, cf.fx, in, cf.xp, cf.lam_mu, own, tiles, nbx, nby, nz); break;
-    case 2: k_fx<2><<<grid, block, 0, s>>>(g, cf.fx, in, cf.xp, cf.lam_mu, own, tiles, nbx, nby, nz); break;
-    case 3: k_fx<3><<<grid, block, 0, s>>>(g, cf.fx, in, cf.xp, cf.lam_mu, own, tiles, nbx, nby, nz); break;
-    default: k_fx<4><<<grid, block, 0, s>>>(g, cf.fx, in, cf.xp, cf.lam_mu, own, tiles, nbx, nby, nz); break;
+    case 1: k_fx<1><<<grid, block, 0, s>>>(g, cf, in, own, tiles, nbx, nby, nz); break;
+    case 2: k_fx<2><<<grid, block, 0, s>>>(g, cf, in, own, tiles, nbx, nby, nz); break;
+    case 3: k_fx<3><<<grid, block, 0, s>>>(g, cf, in, own, tiles, nbx, nby, nz); break;
+    default: k_fx<4><<<grid, block, 0, s>>>(g, cf, in, own, tiles, nbx, nby, nz); break;
     }
 }
 template <typename R>
@@ -325,13 +347,11 @@ void launch_pack(const Geom& g, const T* src, double* dst, cudaStream_t s) {
                                   double*, long long, cudaStream_t);                                                        \
     template void launch_ghost_state<R>(const Geom&, const Phys&, const StencilFields<R>&, double*, int, double*,  \
                                         long long, cudaStream_t);                                                \
-    template void launch_ghost_scalar<R>(const Geom&, R*, cudaStream_t);                                          \
     template int launch_reduce<R>(const Geom&, const Phys&, const StateIn&, const R*, int, double*, int, double*, \
                                   double*, cudaStream_t);                                                        \
     template void launch_unpack<R>(const Geom&, const double*, R*, cudaStream_t);                                 \
     template void launch_pack<R>(const Geom&, const R*, double*, cudaStream_t);
 CNS_INST(double)
 CNS_INST(float)
-template void launch_ghost_scalar<long long>(const Geom&, long long*, cudaStream_t);
 
 }  // namespace cns

@@ -1,13 +1,15 @@
 // kernels_fx.cuh -- FP64 mode: fixed-point stencil inputs, dilatation and the RHS of one
 // point (fx.cuh explains the number format).
 //
-// Per stage, from the ghosted FP64 fields and their maxima:
+// Per stage, from the ghosted FP64 fields and their ranges:
 //   fx_column   the eight fields of a column of points as integers, and theta from the
 //               integers of u, v, w (fx_point: of one point)
 //   fx_ghost    the same conversion of a ghost cell
 //   fx_table    the stage's scale factors (one thread each)
 //   fx_convective, fx_viscous  the two parts of the RHS of a point on the integer units; each
 //               sum is converted once
+// Where the fields' ranges are too wide for their common exponents (fx_exponents) the stage takes
+// theta from wide_theta and the RHS from rhs_wide, FP64 sums of the FP64 fields.
 #pragma once
 #include "cns_common.cuh"
 #include "cns_internal.h"
@@ -16,17 +18,28 @@
 
 namespace cns {
 
-// exponents of the eight fields from their maxima; false: a field is out of range
-__device__ __forceinline__ bool fx_exponents(const unsigned* gmax, int (&e)[8]) {
-    const uint4 a = __ldcg((const uint4*)gmax), b = __ldcg((const uint4*)gmax + 1);
-    const unsigned m[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+// Exponents of the eight fields from their ranges; false: the stage takes FP64 sums. A value is
+// held to 2^-62 of its field's maximum, so the sums serve
+//   fields within 2^-300 .. 2^300 (fx_valid);
+//   rho and T that vary by at most FX_SPAN binades over the box, ghosts included (a ratio of 8 to
+//   16), T by less where mu's exponent is large: each value of rho, T, p, mu is then held exactly,
+//   and the sums' units, which come from the maxima, are near every point's own (T 1 to 10: a
+//   point's error is up to 5e-15 of the largest value near it, T 1 to 1e3: 7e-13, FP64 1e-15);
+//   rho |u|^2 < 2^8 p: what velocities lose in a region at rest stays below the rounding of its
+//   pressure.
+__device__ __forceinline__ bool fx_exponents(const FxBase& b, const unsigned* slots, int (&e)[8]) {
+    unsigned m[8];
+    fx_slots(slots, m);
+    const uint2 least = __ldcg((const uint2*)(slots + FX_LEAST));
     bool ok = true;
 #pragma unroll
     for (int q = 0; q < 8; q++) {
         e[q] = fx_exponent(m[q]);
-        ok = ok && fx_valid(e[q]);
+        ok = ok && fx_valid(m[q]);
     }
-    return ok;
+    // binades from the smallest magnitude's to the largest's
+    const int sr = (int)(m[0] + least.x) - 2048, st = (int)(m[4] + least.y) - 2048;
+    return ok && sr <= FX_SPAN && st <= b.span_T && e[0] + 2 * max(e[1], max(e[2], e[3])) <= e[5] - sr - st + 8;
 }
 
 // Units. Each sum of the RHS that joins several integer sums has a unit U of its own: the
@@ -83,12 +96,11 @@ __device__ __forceinline__ double fx_factor(const FxBase& b, const int (&e)[8], 
     return fx_scaled(pick(b.b1S), er + (q == FXK_F + 3 ? e[6] : ev(q - FXK_F)) - 61);
 }
 
-// entry t of the stage's table (FXK_*). The factors from the RHS integers to real values are
-// NaN if a field is out of range, so that the state becomes NaN and is reported as every
-// other non-finite state.
+// entry t of the stage's table (FXK_*)
 static __device__ __noinline__ i64 fx_table(const FxBase& b, const unsigned* gmax, double lam_mu, int t) {
     int e[8];
-    if (!fx_exponents(gmax, e)) return 0x7ff8000000000000LL;
+    const bool wide = !fx_exponents(b, gmax, e);
+    if (wide || t == FXK_WIDE) return wide;
     const int xth = fx_unit_theta(b, e);
     const auto K = [&](int d, int q) { return fx_factor(b, e, xth, d, q); };
     const auto ev = [&](int q) { return q == 1 ? e[1] : q == 2 ? e[2] : q == 3 ? e[3] : e[6]; };   // u, v, w, H
@@ -137,22 +149,30 @@ __device__ __forceinline__ i64 fx_mul2(i64 a0, i64 b0, i64 a1, i64 b1) {
     return (fx_mad(a0h, b0h, fx_mad(a1h, b1h, 0)) << 2) + (m >> 30);
 }
 
-// the eight fields of element c as integers; u and v given if the caller has them
-__device__ __forceinline__ void fx_store(const FxFields& o, const RhsIn<double>& in, const int (&e)[8], int c, i64 u,
-                                         i64 v, i64 w) {
-    fx_store4(o.v + c, u, v, w, fx_from(in.p[c], e[5]));
-    o.t[c] = make_longlong2(fx_from(in.t[c], e[4]), fx_from(in.m[c], e[7]));
-    o.r[c] = make_longlong2(fx_from(in.r[c], e[0]), fx_from(in.h[c], e[6]));
+// the eight fields of element c as integers, the velocities given
+__device__ __forceinline__ void fx_store(const FxFields& o, const int (&e)[8], int c, i64 u, i64 v, i64 w,
+                                         const double (&q)[5]) {   // q: rho, T, p, H, mu
+    fx_store4(o.v + c, u, v, w, fx_from(q[2], e[5]));
+    o.t[c] = make_longlong2(fx_from(q[1], e[4]), fx_from(q[4], e[7]));
+    o.r[c] = make_longlong2(fx_from(q[0], e[0]), fx_from(q[3], e[6]));
+}
+// rho, T, p, H, mu of element c
+__device__ __forceinline__ void fx_scan(const RhsIn<double>& in, int c, double (&q)[5]) {
+    q[0] = in.r[c]; q[1] = in.t[c]; q[2] = in.p[c]; q[3] = in.h[c]; q[4] = in.m[c];
 }
 
-// the conversion of ghost cell t
-__device__ __forceinline__ void fx_ghost(const Geom& g, const RhsIn<double>& in, const int (&e)[8], int t) {
+// the conversion of ghost cell t (wide: its ranges alone)
+__device__ __forceinline__ void fx_ghost(const Geom& g, const RhsIn<double>& in, const int (&e)[8], int t, bool wide,
+                                         FxLeast& least) {
     const GhostCell gc = ghost_cell_of(g, t);
     const int off = gc.side == 0 ? -gc.m : gc.m - 1;
     const int c = (int)(gc.face == 0   ? g.at(gc.side == 0 ? off : g.mx + off, gc.j, gc.k)
                         : gc.face == 1 ? g.at(gc.i, gc.side == 0 ? off : g.my + off, gc.k)
                                        : g.at(gc.i, gc.j, gc.side == 0 ? off : g.mz + off));
-    fx_store(in.fx, in, e, c, fx_from(in.u[c], e[1]), fx_from(in.v[c], e[2]), fx_from(in.w[c], e[3]));
+    double q[5];
+    fx_scan(in, c, q);
+    least.add(q[0], q[1]);
+    if (!wide) fx_store(in.fx, e, c, fx_from(in.u[c], e[1]), fx_from(in.v[c], e[2]), fx_from(in.w[c], e[3]), q);
 }
 
 // Conversion of a column of points and its theta. The threads (tx, ty), tx < 32, ty < TY, own
@@ -166,7 +186,7 @@ __device__ __forceinline__ void fx_ghost(const Geom& g, const RhsIn<double>& in,
 template <int V, int TY>
 __device__ __forceinline__ void fx_column(const Geom& g, const FxBase& b, const RhsIn<double>& in, const int (&e)[8],
                                           const double* __restrict__ xp, int i0, int j0, int k0, int k1, bool own,
-                                          int tx, int ty, i64 (*su)[32 + 2 * V], i64 (*sv)[32]) {
+                                          int tx, int ty, i64 (*su)[32 + 2 * V], i64 (*sv)[32], FxLeast& least) {
     static_assert(V <= TY, "the y halo rows are loaded by the first and last V tile rows");
     const int i = i0 + tx, j = j0 + ty;
     const bool inside = i < g.mx && j < g.my;
@@ -198,7 +218,9 @@ __device__ __forceinline__ void fx_column(const Geom& g, const FxBase& b, const 
     for (int k = k0; k < k1; k++) {
         const int ck = c0 + k * PS;
         double q[5] = {0, 0, 0, 0, 0};
-        if (inside) { q[0] = __ldg(in.p + ck); q[1] = __ldg(in.t + ck); q[2] = __ldg(in.m + ck); q[3] = __ldg(in.r + ck); q[4] = __ldg(in.h + ck); }
+        if (inside) {
+            q[0] = __ldg(in.r + ck); q[1] = __ldg(in.t + ck); q[2] = __ldg(in.p + ck); q[3] = __ldg(in.h + ck); q[4] = __ldg(in.m + ck);
+        }
         const i64 cu = fx_from(nu, e[1]), cv = fx_from(nv, e[2]);
         ring[2 * V] = fx_from(nw, e[3]);
         const i64 cx = xl || xr ? fx_from(hx, e[1]) : 0, cy = yl || yr ? fx_from(hy, e[2]) : 0;
@@ -223,9 +245,8 @@ __device__ __forceinline__ void fx_column(const Geom& g, const FxBase& b, const 
             const i64 th = fx_mul(sx.value(), kx) + fx_mul(sy.value(), ky) + fx_mul(sz.value(), kz);
             in.fx.th[ck] = th;
             if (own) dil_ghost_owner<i64>(g, in.fx.th, ck, i, j, k, th);
-            fx_store4(in.fx.v + ck, cu, cv, ring[V], fx_from(q[0], e[5]));
-            in.fx.t[ck] = make_longlong2(fx_from(q[1], e[4]), fx_from(q[2], e[7]));
-            in.fx.r[ck] = make_longlong2(fx_from(q[3], e[0]), fx_from(q[4], e[6]));
+            fx_store(in.fx, e, ck, cu, cv, ring[V], q);
+            least.add(q[0], q[1]);
         }
 #pragma unroll
         for (int l = 0; l < 2 * V; l++) ring[l] = ring[l + 1];
@@ -236,7 +257,7 @@ __device__ __forceinline__ void fx_column(const Geom& g, const FxBase& b, const 
 // stage kernel's form; the same integers)
 template <int V>
 __device__ __forceinline__ void fx_point(const Geom& g, const FxBase& b, const RhsIn<double>& in, const int (&e)[8],
-                                         const double* __restrict__ xp, int i, int j, int k) {
+                                         const double* __restrict__ xp, int i, int j, int k, FxLeast& least) {
     const int c = (int)g.at(i, j, k), P = (int)g.P, PS = (int)g.PS;
     i64 kx, ky, kz;
     fx_theta_factors(b, e, g.nonuniform_x, xp[i], kx, ky, kz);
@@ -249,7 +270,10 @@ __device__ __forceinline__ void fx_point(const Geom& g, const FxBase& b, const R
     }
     const i64 th = fx_mul(sx.value(), kx) + fx_mul(sy.value(), ky) + fx_mul(sz.value(), kz);
     in.fx.th[c] = th;
-    fx_store(in.fx, in, e, c, fx_from(in.u[c], e[1]), fx_from(in.v[c], e[2]), fx_from(in.w[c], e[3]));
+    double q[5];
+    fx_scan(in, c, q);
+    least.add(q[0], q[1]);
+    fx_store(in.fx, e, c, fx_from(in.u[c], e[1]), fx_from(in.v[c], e[2]), fx_from(in.w[c], e[3]), q);
 }
 
 // The sums of one direction at a point, in two passes over the neighbour pairs (-l, l), each of
@@ -454,6 +478,113 @@ __device__ __forceinline__ void fx_viscous(const Geom& g, const FxBase& b, const
     en = fma((double)fx_dot3(dT[0], dmu[0], dT[1], dmu[1], dT[2], dmu[2]), fx_unit<RO>(K, FXK_UC, sm), en);
     en = fma(in.m[c], (double)diss * fx_unit<RO>(K, FXK_UE, 2 * st), en);
     out[3] = fma(u0, out[0], fma(v0, out[1], fma(w0, out[2], en)));
+}
+
+// ---- FP64 sums ----
+// theta at element c and its ghost images
+template <int V, bool RO>
+__device__ __noinline__ void wide_theta(const Geom& g, const CoefT<double>& cf, const RhsIn<double>& in, int i, int j,
+                                        int k, bool own) {
+    const int c = (int)g.at(i, j, k), P = (int)g.P, PS = (int)g.PS;
+    const auto d1 = [&](const double* f, int st, const double* co) {
+        double s = co[1] * (ld<RO>(f + c + st) - ld<RO>(f + c - st));
+#pragma unroll
+        for (int l = 2; l <= V; l++) s = fma(co[l], ld<RO>(f + c + l * st) - ld<RO>(f + c - l * st), s);
+        return s;
+    };
+    double x = d1(in.u, 1, cf.c1V[0]);
+    if (g.nonuniform_x) x *= cf.xp[i];
+    const double th = x + d1(in.v, P, cf.c1V[1]) + d1(in.w, PS, cf.c1V[2]);
+    double* o = (double*)in.fx.th;
+    o[c] = th;
+    if (own) dil_ghost_owner<double>(g, o, c, i, j, k, th);
+}
+
+// RHS of the point at element c (without body force and sponge), with the sums of fx_convective
+// and fx_viscous in FP64 from the FP64 fields and theta
+template <int S, int V, bool RO>
+__device__ __forceinline__ void rhs_wide(const Geom& g, const CoefT<double>& cf, const RhsIn<double>& in, int quirk,
+                                         int i, int c, double (&acc)[5]) {
+    const double* th = (const double*)in.fx.th;
+    const auto at = [&](const double* f, int o) { return ld<RO>(f + c + o); };
+    const bool nux = g.nonuniform_x;
+    const double xp = nux ? cf.xp[i] : 1.0;
+    const double u0 = at(in.u, 0), v0 = at(in.v, 0), w0 = at(in.w, 0), r0 = at(in.r, 0), h0 = at(in.h, 0),
+                 m0 = at(in.m, 0), th23 = (2. / 3.) * at(th, 0);
+    const auto d1 = [&](const double* f, int st, const double* co) {
+        double s = co[1] * (at(f, st) - at(f, -st));
+#pragma unroll
+        for (int l = 2; l <= V; l++) s = fma(co[l], at(f, l * st) - at(f, -l * st), s);
+        return s;
+    };
+    double G[9];   // G[3 a + b] = d u_b / d x_a
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const int st = d == 0 ? 1 : (int)(d == 1 ? g.P : g.PS);
+        const double x = d == 0 ? xp : 1.0;
+        G[3 * d] = d1(in.u, st, cf.c1V[d]) * x;
+        G[3 * d + 1] = d1(in.v, st, cf.c1V[d]) * x;
+        G[3 * d + 2] = d1(in.w, st, cf.c1V[d]) * x;
+    }
+    const double t[6] = {fma(2.0, G[0], -th23), fma(2.0, G[4], -th23), fma(2.0, G[8], -th23),
+                         G[1] + G[3], G[2] + G[6], G[5] + G[7]};
+    // y-z dissipation with the quirk: tau_yz dv/dz in the y sum as in the z sum (src/cuda_rhs.cu:175)
+    const double q12 = quirk ? G[7] + G[7] : t[5];
+    const double diss = fma(t[0], G[0], fma(t[1], G[4], fma(t[2], G[8], fma(t[3], t[3], fma(t[4], t[4], t[5] * q12)))));
+#pragma unroll
+    for (int q = 0; q < 5; q++) acc[q] = 0.0;
+    double W[3] = {0, 0, 0}, L[4] = {0, 0, 0, 0}, cond = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const int st = d == 0 ? 1 : (int)(d == 1 ? g.P : g.PS);
+        const bool sx = d == 0 && nux;
+        const double x = sx ? xp : 1.0;
+        const double* F[4] = {in.u, in.v, in.w, in.t};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (sx) {
+#pragma unroll
+                for (int l = -V; l <= V; l++) L[q] = fma(__ldg(cf.cvsx + (l + V) * g.mx + i), at(F[q], l), L[q]);
+            } else {
+                L[q] = fma(cf.c2V[d][0], at(F[q], 0), L[q]);
+#pragma unroll
+                for (int l = 1; l <= V; l++) L[q] = fma(cf.c2V[d][l], at(F[q], l * st) + at(F[q], -l * st), L[q]);
+            }
+        }
+        const double dmu = d1(in.m, st, cf.c1V[d]) * x;
+        W[0] = fma(d == 0 ? t[0] : d == 1 ? t[3] : t[4], dmu, W[0]);
+        W[1] = fma(d == 0 ? t[3] : d == 1 ? t[1] : t[5], dmu, W[1]);
+        W[2] = fma(d == 0 ? t[4] : d == 1 ? t[5] : t[2], dmu, W[2]);
+        cond = fma(d1(in.t, st, cf.c1V[d]) * x, dmu, cond);
+        W[d] = fma(m0 * (1.0 / 3.0), d1(th, st, cf.c1V[d]) * x, W[d]);
+        // fluxes (fx_conv's) and the pressure gradient; fc = c1S / 4, the mass flux's weight twice that
+        const double* gf = d == 0 ? in.u : d == 1 ? in.v : in.w;
+        const double g0 = d == 0 ? u0 : d == 1 ? v0 : w0;
+        double f[5] = {0, 0, 0, 0, 0}, dp = 0.0;
+#pragma unroll
+        for (int l = 1; l <= S; l++) {
+            const double am = cf.fc[d][l] * (at(in.r, -l * st) + r0) * (at(gf, -l * st) + g0);
+            const double ap = cf.fc[d][l] * (r0 + at(in.r, l * st)) * (g0 + at(gf, l * st));
+            f[0] += am - ap;
+            f[1] = fma(am, at(in.u, -l * st), fma(-ap, at(in.u, l * st), f[1]));
+            f[2] = fma(am, at(in.v, -l * st), fma(-ap, at(in.v, l * st), f[2]));
+            f[3] = fma(am, at(in.w, -l * st), fma(-ap, at(in.w, l * st), f[3]));
+            f[4] = fma(am, at(in.h, -l * st), fma(-ap, at(in.h, l * st), f[4]));
+            dp = fma(cf.c1S[d][l], at(in.p, l * st) - at(in.p, -l * st), dp);
+        }
+        acc[0] = fma(2.0 * x, f[0], acc[0]);
+#pragma unroll
+        for (int q = 1; q < 5; q++) acc[q] = fma(x, f[q], acc[q]);
+        acc[1 + d] = fma(-x, dp, acc[1 + d]);
+    }
+    const double half = 0.5 * acc[0];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        W[q] = fma(m0, L[q], W[q]);
+        acc[1 + q] = fma(q == 0 ? u0 : q == 1 ? v0 : w0, half, acc[1 + q]) + W[q];
+    }
+    cond = fma(m0, L[3], cond);
+    acc[4] = fma(h0, half, acc[4]) + fma(m0, diss, cf.lam_mu * cond) + fma(u0, W[0], fma(v0, W[1], w0 * W[2]));
 }
 
 }  // namespace cns

@@ -15,8 +15,8 @@ namespace cns {
 // roundings and mu is evaluated in FP32 from the FP64 T rounded to FP32.
 // ---------------------------------------------------------------------------------
 // T, p, H, mu (and the FP32 copies) of one point from its FP64 state and 1/rho; the state
-// kernel and the fused epilogue of the RHS kernel share it
-template <typename R>
+// kernel and the fused epilogue of the RHS kernel share it. LEAST: and the smallest magnitudes
+template <typename R, bool LEAST = false>
 __device__ __forceinline__ void state_store(const Phys& ph, const DerivedOut<R>& o, double* scal, long long c,
                                             double rr, double inv, double uu, double vv, double ww, double ee) {
     if constexpr (sizeof(R) == 4) {
@@ -48,6 +48,11 @@ __device__ __forceinline__ void state_store(const Phys& ph, const DerivedOut<R>&
         o.h[c] = hh;
         o.m[c] = suth * ph.invRe;
         fx_track(o.gmax, {rr, uu, vv, ww, T, pr, hh, suth * ph.invRe});
+        if constexpr (LEAST) {
+            FxLeast least;
+            least.add(rr, T);
+            least.raise(o.gmax);
+        }
         if (!positive_bits(T) || !positive_bits(rr)) scal[SC_NONFINITE] = 1.0;   // racy flag write, any writer is fine
     }
 }
@@ -57,7 +62,7 @@ __device__ __forceinline__ void state_point(const Geom& g, const Phys& ph, const
                                             double* scal, int i, int j, int k) {
     const long long c = g.at(i, j, k);
     const double rr = q.r[c], uu = q.u[c], vv = q.v[c], ww = q.w[c], ee = q.e[c];
-    state_store<R>(ph, o, scal, c, rr, rcp_nr(rr), uu, vv, ww, ee);
+    state_store<R, true>(ph, o, scal, c, rr, rcp_nr(rr), uu, vv, ww, ee);
 }
 
 // Stage 0 of a step advances the simulation time by dt (deviceAdvanceTime) and, with a
@@ -199,10 +204,10 @@ __device__ __forceinline__ void ghost_state_cell(const Geom& g, const Phys& ph, 
         return;
     }
     R* F[8] = {f.r, f.u, f.v, f.w, f.t, f.p, f.h, f.m};
-    // ghosts that are no copies of interior values join the maxima; the next state's slots
+    // ghosts that are no copies of interior values join the ranges; the next state's slots
     // start at zero (its writer runs after this phase)
     constexpr bool FX = sizeof(R) == 8;
-    if (FX && t < 8) f.gnext[t] = 0u;
+    if (FX && t < FX_SLOTS) f.gnext[t] = 0u;
     const GhostCell gc = ghost_cell_of(g, t);
     const int m = gc.m, side = gc.side;
     long long cg, cs;

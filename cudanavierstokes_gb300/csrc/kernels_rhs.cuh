@@ -316,6 +316,17 @@ __device__ __forceinline__ void rhs_point_packed(const Geom& g, const CoefT<floa
     stage_tail<float>(g, up, scal, i, k, c, acc, u0, v0, w0, r0);
 }
 
+// The FP64 mode's point of a stage with FP64 sums (a call of its own: the other path keeps its
+// registers)
+template <int S, int V, bool RO>
+__device__ __noinline__ void wide_point(const Geom& g, const CoefT<double>& cf, const RhsIn<double>& in,
+                                        const Update<double>& up, double* scal, int quirk, int i, int j, int k) {
+    const int c = (int)g.at(i, j, k);
+    double acc[5];
+    rhs_wide<S, V, RO>(g, cf, in, quirk, i, c, acc);
+    stage_tail<double>(g, up, scal, i, k, c, acc, up.qin.u[c], up.qin.v[c], up.qin.w[c], up.qin.r[c]);
+}
+
 // RHS + stage update of one interior point (i, j, k), every neighbour from global memory
 // (CW: the FP32 body with compile-time weights, see rhs_dir_packed)
 template <typename R, int S, int V, bool CW = false>
@@ -324,9 +335,14 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
     if constexpr (sizeof(R) == 4) {
         rhs_point_packed<S, V, CW>(g, cf, in, up, scal, quirk, i, j, k);
     } else {
+        if (ld<!CW>(in.fx.k + FXK_WIDE) != 0) {
+            wide_point<S, V, !CW>(g, cf, in, up, scal, quirk, i, j, k);
+            return;
+        }
         const int c = (int)g.at(i, j, k);
         const double u0 = up.qin.u[c], v0 = up.qin.v[c], w0 = up.qin.w[c];
-        double acc[5], vis[4];
+        double acc[5];
+        double vis[4];
         fx_convective<S, CW>(g, cf.fx, in.fx, i, c, acc);
         fx_viscous<V, CW>(g, cf.fx, in, quirk, i, c, u0, v0, w0, vis);
 #pragma unroll
@@ -346,8 +362,10 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
 // (128 registers), bound by latency: issue 38 %, FP64 pipe 44 %, ~3,700 instructions per point;
 // on the channel 128x160x192 0.93 ms, with 3 blocks (168 registers) 1.11, 5 (96, spilling) 0.98.
 template <typename R, int S, int V>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 4) k_rhs(Geom g, const __grid_constant__ CoefT<R> cf,
-                                                                     const __grid_constant__ RhsIn<R> in, Update<R> up,
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 4) k_rhs(const __grid_constant__ Geom g,
+                                                                     const __grid_constant__ CoefT<R> cf,
+                                                                     const __grid_constant__ RhsIn<R> in,
+                                                                     const __grid_constant__ Update<R> up,
                                                                      double* __restrict__ scal, int quirk, int row0) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = row0 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
@@ -363,15 +381,21 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 4) k_rhs(Geom g, con
 // 0.93 ms against 1.12.
 constexpr int SPLIT_POINTS = 64;
 template <int S, int V>
-__global__ void __launch_bounds__(2 * SPLIT_POINTS, 4) k_rhs_split(Geom g, const __grid_constant__ CoefT<double> cf,
+__global__ void __launch_bounds__(2 * SPLIT_POINTS, 4) k_rhs_split(const __grid_constant__ Geom g,
+                                                                  const __grid_constant__ CoefT<double> cf,
                                                                   const __grid_constant__ RhsIn<double> in,
-                                                                  Update<double> up, double* __restrict__ scal,
+                                                                  const __grid_constant__ Update<double> up,
+                                                                  double* __restrict__ scal,
                                                                   int quirk) {
     __shared__ double sv[4][SPLIT_POINTS];
     const int bh = (int)blockDim.y / 2, row = (int)threadIdx.y % bh, s = row * (int)blockDim.x + (int)threadIdx.x;
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = (int)blockIdx.y * bh + row, k = (int)blockIdx.z;
     const bool inside = i < g.mx && j < g.my, first = (int)threadIdx.y < bh;
     const int c = (int)g.at(i, j, k);
+    if (ld<true>(in.fx.k + FXK_WIDE) != 0) {
+        if (inside && first) wide_point<S, V, true>(g, cf, in, up, scal, quirk, i, j, k);
+        return;
+    }
     double acc[5];
     if (inside) {
         if (first) {

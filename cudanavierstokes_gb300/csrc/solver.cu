@@ -144,7 +144,7 @@ DerivedOut<R> derived_out(cns_solver* h, int b) {
 // calcState of the current state (when the RHS kernel has not recovered it already)
 template <typename R>
 int state_phase(cns_solver* h) {
-    if (h->gmax[0]) CK(cudaMemsetAsync(h->gmax[h->cur], 0, 8 * sizeof(unsigned), h->stream));
+    if (h->gmax[0]) CK(cudaMemsetAsync(h->gmax[h->cur], 0, FX_SLOTS * sizeof(unsigned), h->stream));
     launch_state<R>(h->geom, h->phys, state_in(h, h->cur), derived_out<R>(h, h->cur), h->scal, 0, nullptr, 0,
                     h->stream);
     h->launches += 1;
@@ -187,8 +187,8 @@ int grad_phase(cns_solver* h) {
     }
     h->launches += 1;
     if (!own) {
-        if constexpr (std::is_same<R, double>::value) launch_ghost_scalar<long long>(h->geom, h->fx.th, h->stream);
-        else launch_ghost_scalar<R>(h->geom, (R*)h->dil, h->stream);
+        if constexpr (std::is_same<R, double>::value) launch_ghost_theta(h->geom, h->fx, h->stream);
+        else launch_ghost_theta(h->geom, (float*)h->dil, h->stream);
         h->launches += 1;
     }
     CKL();
@@ -397,6 +397,8 @@ int set_fx_base(cns_solver* h) {
         for (int d = 0; d < 3; d++) b.b1V3[d] = b.b1V[d] / 3.0;
     };
     for (int d = 0; d < 3; d++) b.th[d] = b.b1V[d];
+    // mu = T^viscexp / Re within 8 binades, where every value is exact
+    b.span_T = (int)(FX_SPAN / std::max(1.0, 0.5 * fabs(h->p.viscexp)));
     b.thmax = b.th[0];
     b.xx = nullptr;
     b.xpk = nullptr;
@@ -576,7 +578,7 @@ int cns_create(const cns_params* pin, int device, cns_solver** out) {
         if (!rc) rc = h->alloc_field((void**)&h->fx.r, sizeof(longlong2));
         h->fx.th = (long long*)h->dil;
         if (!rc) rc = h->alloc(&h->fx.k, FXK_COUNT);
-        for (int b = 0; b < 2 && !rc; b++) rc = h->alloc(&h->gmax[b], 8);
+        for (int b = 0; b < 2 && !rc; b++) rc = h->alloc(&h->gmax[b], FX_SLOTS);
         if (!rc) rc = set_fx_base(h);
     }
     if (!rc) rc = h->alloc_fields(h->rb, 5, rs);

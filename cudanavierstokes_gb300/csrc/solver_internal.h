@@ -41,7 +41,7 @@ struct cns_solver {
     // q[cur] and writes those of the new state q[1 - cur] (fused state recovery).
     void* der[2][4] = {};
     // FP64 mode: fixed-point stencil inputs of the current stage (kernels_fx.cuh), the
-    // stage's scale factors, and the maxima of the fields of each state buffer
+    // stage's scale factors, and the ranges of the fields of each state buffer
     cns::FxFields fx{};
     unsigned* gmax[2] = {};
     longlong2* xx = nullptr;     // integer metrics of a stretched x
