@@ -96,8 +96,8 @@ struct cns_batch {
     int* d_err = nullptr;
     int *d_status = nullptr, *h_status = nullptr;   // k_batch_status; h_status page-locked
     // full residency unless a shape is set or tuned (choose_shape clamps it): 20 steps of 8
-    // FP32 boxes 32..128 take 42 ms with 7 blocks per SM, 115 ms with 1
-    int threads = 128, blocks_per_sm = 32, nsm = 152;
+    // FP32 boxes 32..128 and their fields take 30 ms with 7 blocks per SM, 115 ms with 1
+    int threads = 128, blocks_per_sm = 32, nsm = GB300_SMS;
     long long units = 0;                 // point units of all members
     bool tuned = false;
     cudaGraphExec_t exec[2] = {nullptr, nullptr};

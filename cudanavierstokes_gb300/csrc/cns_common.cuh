@@ -16,6 +16,9 @@
 
 namespace cns {
 
+// SMs of a GB300: the grids of the single solver's kernels are fitted to them
+constexpr int GB300_SMS = 152;
+
 enum XBC { XBC_PER = 0, XBC_WALL = 1, XBC_BL = 2 };
 
 // indices into the device scalar block
@@ -72,21 +75,24 @@ struct FxBase {
     const long long* xpk;   // [mx] 1/x' as a factor (low word, balanced high half), the largest 2^63 (1 - 2^-20)
 };
 template <typename R>
-struct CoefFx {};
+struct CoefOf;
 template <>
-struct CoefFx<double> {
+struct CoefOf<double> {
     FxBase fx;
 };
+template <>
+struct CoefOf<float> {
+    float fq[3][5];   // 0.5 * c1S: split-form quadratic flux (rho u) weights
+    float inv[3];     // inverse grid spacing of each direction (d_dx, d_dy, d_dz)
+    float inv2[3];    // their squares
+};
 template <typename R>
-struct CoefT : CoefFx<R> {
+struct CoefT : CoefOf<R> {
     R c1S[3][5];
     R c1V[3][5];
     R c2V[3][5];
-    R fq[3][5];      // 0.5  * c1S: split-form quadratic flux (rho u) weights
     R fc[3][5];      // 0.25 * c1S: split-form cubic flux (rho u phi) weights
     R lam_mu;        // lambda / mu = 1 / (Pr Ec)
-    R inv[3];        // inverse grid spacing of each direction (d_dx, d_dy, d_dz)
-    R inv2[3];       // their squares
     const R* xp;     // [mx]
     const R* cvsx;   // [(2V+1)*mx], index it*mx + i
 };

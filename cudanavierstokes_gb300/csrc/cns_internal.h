@@ -64,7 +64,8 @@ struct FxFields {
 // packed records qa, qb and theta)
 template <typename R>
 struct RhsIn {
-    const R *r, *u, *v, *w, *t, *p, *h, *m, *dil;
+    const R *r, *u, *v, *w, *t, *p, *h, *m;
+    const R* dil;   // FP32-RHS mode, with qa and qb
     const float4 *qa, *qb;
     FxFields fx;   // FP64 mode
 };

@@ -41,7 +41,7 @@ __device__ __forceinline__ void vel_track(unsigned* slots, unsigned u, unsigned 
 }
 
 // the velocity ghost layer of the FP64 state (in FP32-RHS mode the ghost kernel fills the
-// FP32 stencil copies, not the state), and the maxima of the three components with it
+// FP32 stencil copies, not the state), and the largest codes of the three components with it
 __global__ void __launch_bounds__(256) k_ghost_vel(Geom g, Phys ph, double* u, double* v, double* w,
                                                    const double* scal, unsigned* vmax) {
     const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
@@ -63,11 +63,12 @@ __global__ void __launch_bounds__(256) k_vel_max(Geom g, const double* __restric
     vel_track(vmax, m[0], m[1], m[2]);
 }
 
-// The nine gradients as fixed-point sums (fx.cuh; vmax: the components' maxima, ghosts
+// The nine gradients as fixed-point sums (fx.cuh; vmax: the components' largest codes, ghosts
 // included; b: inverse spacings over the weights' denominator), the rest in FP64. With theta
 // the trace, sum tau_ab G_ab = 2 sum G_aa^2 + sum_{a<b} (G_ab + G_ba)^2 - 2/3 theta^2.
 // (Channel 128x160x192: 72 FP64 instructions of the gradients and 27 + 28 of the contraction
-// and the viscosity power per point made the call 1.38 ms, this form 0.56 ms.)
+// and the viscosity power per point made the call 1.38 ms, this form 0.56 ms; what it spends now
+// is 72 conversions to fixed point a point, every neighbour's anew, and the contraction in FP64.)
 template <int V>
 __global__ void __launch_bounds__(DG_THREADS, 4) k_dissip(Geom g, Phys ph, const double* __restrict__ xp, double bx,
                                                        double by, double bz, const unsigned* __restrict__ vmax,
@@ -192,14 +193,14 @@ int cns_dissipation(cns_solver* h, double* out) {
     const StateIn q{h->q[c][0], h->q[c][1], h->q[c][2], h->q[c][3], h->q[c][4]};
     const dim3 grid((g.mx + 31) / 32, (g.my + 3) / 4, (g.mz + DG_NZ - 1) / DG_NZ);
     const long long nb = (long long)grid.x * grid.y * grid.z;
-    double* buf = nullptr;   // partials, the two means, the maxima
+    double* buf = nullptr;   // partials, the two means, the largest codes
     if (cns::solver_scratch(h, 2 * (size_t)nb + 4, &buf)) return CNS_ERR_OOM;
     unsigned* vmax = (unsigned*)(buf + 2 * nb + 2);
     e = cudaMemsetAsync(vmax, 0, 4 * sizeof(unsigned), h->stream);
     if (e != cudaSuccess) return diag_error(e);
     const unsigned gb = (unsigned)((ghost_count(g) + 255) / 256);
     k_ghost_vel<<<gb, 256, 0, h->stream>>>(g, h->phys, h->q[c][1], h->q[c][2], h->q[c][3], h->scal, vmax);
-    k_vel_max<<<4 * 152, 256, 0, h->stream>>>(g, h->q[c][1], h->q[c][2], h->q[c][3], vmax);
+    k_vel_max<<<4 * GB300_SMS, 256, 0, h->stream>>>(g, h->q[c][1], h->q[c][2], h->q[c][3], vmax);
     const int V = h->p.stencil_visc;
     const double s = ldexp(1.0, 32 - fxs1(V)) / fxn1(V), bx = g.dx * s, by = g.dy * s, bz = g.dz * s;
 #define CNS_DISSIP(VV) k_dissip<VV><<<grid, DG_THREADS, 0, h->stream>>>(g, h->phys, h->xp_d, bx, by, bz, vmax, q, buf)

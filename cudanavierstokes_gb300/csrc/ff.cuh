@@ -186,23 +186,10 @@ struct ffacc2 {
     }
 };
 
-template <typename R>
-inline constexpr bool is_ff = false;
-template <>
-inline constexpr bool is_ff<ff> = true;
-
-// FP64 <-> pair: (double)h + (double)l rounds once in FP64 (2^-53, below the pair's own
-// precision); the split rounds h, then the remainder x - h (exact in FP64)
-__device__ __forceinline__ double ff_to_d(ff x) { return (double)x.h + (double)x.l; }
+// FP64 to pair: the split rounds h, then the remainder x - h (exact in FP64)
 __device__ __forceinline__ ff d_to_ff(double x) {
     const float h = __double2float_rn(x);
     return ff(h, __double2float_rn(x - (double)h));
 }
 
 }  // namespace cns
-
-// read-only cached load of a pair (one 8-byte load)
-__device__ __forceinline__ cns::ff __ldg(const cns::ff* p) {
-    const float2 v = __ldg(reinterpret_cast<const float2*>(p));
-    return cns::ff(v.x, v.y);
-}

@@ -297,7 +297,7 @@ void launch_dil_packed(int V, const Geom& g, const CoefT<float>& cf, const float
     // line at four blocks per SM was slower (64^3 9.3 us, 75 x 53 x 91 11.7 against 9.8: more z halos), at
     // one the same (64^3 7.9, 75 x 53 x 91 10.9).
     int nz = DIL_NZ;
-    while (nz > 1 && (long long)nbx * nby * ((g.mz + nz - 1) / nz) < 2 * 152) nz /= 2;
+    while (nz > 1 && (long long)nbx * nby * ((g.mz + nz - 1) / nz) < 2 * GB300_SMS) nz /= 2;
     const dim3 grid(nbx, nby, (g.mz + nz - 1) / nz);
     const dim3 block(DIL_TX, DIL_TY, 1);
     switch (V) {
@@ -312,7 +312,7 @@ void launch_dil_packed(int V, const Geom& g, const CoefT<float>& cf, const float
 void launch_fx(int V, const Geom& g, const CoefT<double>& cf, const RhsIn<double>& in, int own, cudaStream_t s) {
     const int nbx = (g.mx + DIL_TX - 1) / DIL_TX, nby = (g.my + DIL_TY - 1) / DIL_TY;
     int nz = DIL_NZ;
-    while (nz > 1 && (long long)nbx * nby * ((g.mz + nz - 1) / nz) < 4 * 152) nz /= 2;
+    while (nz > 1 && (long long)nbx * nby * ((g.mz + nz - 1) / nz) < 4 * GB300_SMS) nz /= 2;
     const int tiles = nbx * nby * ((g.mz + nz - 1) / nz);
     const unsigned grid = FX_TABLE_BLOCKS + (unsigned)tiles + ghost_blocks(g);
     const dim3 block(DIL_TX, DIL_TY, 1);

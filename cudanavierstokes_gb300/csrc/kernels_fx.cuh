@@ -187,7 +187,7 @@ template <int V, int TY>
 __device__ __forceinline__ void fx_column(const Geom& g, const FxBase& b, const RhsIn<double>& in, const int (&e)[8],
                                           const double* __restrict__ xp, int i0, int j0, int k0, int k1, bool own,
                                           int tx, int ty, i64 (*su)[32 + 2 * V], i64 (*sv)[32], FxLeast& least) {
-    static_assert(V <= TY, "the y halo rows are loaded by the first and last V tile rows");
+    static_assert(2 * V <= TY, "the y halo rows are loaded by the first and last V tile rows");
     const int i = i0 + tx, j = j0 + ty;
     const bool inside = i < g.mx && j < g.my;
     const bool ghosted = i < g.mx + V && j < g.my + V;   // own slot of the tiles is read by someone
@@ -207,12 +207,11 @@ __device__ __forceinline__ void fx_column(const Geom& g, const FxBase& b, const 
             nu = __ldg(in.u + ck);
             nv = __ldg(in.v + ck);
         }
-        // the halos: a thread fills at most one of the two x halos (V <= 16); with V > TY / 2
-        // the rows of the two y halos overlap, the upper one is then fetched at the store
+        // the halos: a thread fills at most one of the two x halos and one of the two y halos
         if (xl && j < g.my) hx = __ldg(in.u + ck - V);
         if (xr && i < g.mx && j < g.my) hx = __ldg(in.u + ck + V);
         if (yl && i < g.mx) hy = __ldg(in.v + ck - V * P);
-        if (yr && j < g.my && i < g.mx && !yl) hy = __ldg(in.v + ck + V * P);
+        if (yr && j < g.my && i < g.mx) hy = __ldg(in.v + ck + V * P);
     };
     if (k0 < k1) fetch(k0);
     for (int k = k0; k < k1; k++) {
@@ -231,8 +230,7 @@ __device__ __forceinline__ void fx_column(const Geom& g, const FxBase& b, const 
         if (xl) su[ty][tx] = cx;
         if (xr) su[ty][tx + 2 * V] = cx;
         if (yl) sv[ty][tx] = cy;
-        if (yr && !yl) sv[ty + 2 * V][tx] = cy;
-        if (2 * V > TY && yr && yl && j < g.my && i < g.mx) sv[ty + 2 * V][tx] = fx_from(__ldg(in.v + ck + V * P), e[2]);
+        if (yr) sv[ty + 2 * V][tx] = cy;
         __syncthreads();
         if (inside) {
             FxSum sx, sy, sz;
@@ -279,7 +277,7 @@ __device__ __forceinline__ void fx_point(const Geom& g, const FxBase& b, const R
 // The sums of one direction at a point, in two passes over the neighbour pairs (-l, l), each of
 // which loads a pair once and feeds every sum that needs it (one pass for all of them needs 150
 // registers: 640 bytes spilled and 1.28 against 1.23 ms on the channel; with the four values
-// both passes read as one 32-byte load and both loops unrolled 0.93 ms):
+// both passes read as one 32-byte load and both loops unrolled 0.88 ms):
 //   fx_visc  first derivatives of u, v, w, mu, T, theta and second ones of u, v, w, T (viscous
 //            order)
 //   fx_conv  first derivative of p and the telescoped split-form fluxes (advective order)

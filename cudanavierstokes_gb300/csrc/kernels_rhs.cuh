@@ -144,8 +144,8 @@ __device__ __forceinline__ void stage_tail(const Geom& g, const Update<R>& up, d
 // every sum that needs them -- the first derivatives of u, v, w, mu, T, theta at the
 // viscous order and of p at the advective order, the second derivatives of u, v, w, T, and
 // the telescoped split-form fluxes -- so no stencil is held in registers. Each sum is
-// accumulated in the order of the FP64-mode body (centre term, then l ascending) with the
-// same expressions; the non-uniform x second derivative adds the pair (l, -l) per l.
+// accumulated from the centre term with l ascending; the non-uniform x second derivative adds
+// the pair (l, -l) per l.
 // ---------------------------------------------------------------------------------
 //
 // CW (compile-time weights): the sums use the central-difference weights as immediates and
@@ -214,7 +214,7 @@ __device__ __forceinline__ void rhs_dir_packed(const Geom& g, const CoefT<float>
             }
         }
         dp = l == 1 ? w1S(1) * (Bp.y - Bm.y) : fma(w1S(l), Bp.y - Bm.y, dp);
-        // telescoped split-form fluxes (rhs_direction: a_l Q+- shared by the cubic fluxes)
+        // telescoped split-form fluxes, a_l Q+- shared by the cubic ones
         const float gm = DIR == 0 ? Am.y : (DIR == 1 ? Am.z : Am.w);
         const float gp = DIR == 0 ? Ap.y : (DIR == 1 ? Ap.z : Ap.w);
         const float Qm = (Am.x + r0) * (gm + un);

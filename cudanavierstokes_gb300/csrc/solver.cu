@@ -111,13 +111,13 @@ RhsIn<R> rhs_in(cns_solver* h, int c) {
     if (h->fp32) {   // packed records (rho, u, v, w) and (T, p, H, mu)
         in.qa = (const float4*)h->der[c][0];
         in.qb = (const float4*)h->der[c][1];
+        in.dil = (const R*)h->dil;
     } else {
         in.r = (const R*)h->q[c][0]; in.u = (const R*)h->q[c][1]; in.v = (const R*)h->q[c][2];
         in.w = (const R*)h->q[c][3];
         in.h = (const R*)h->der[c][0]; in.t = (const R*)h->der[c][1]; in.p = (const R*)h->der[c][2];
         in.m = (const R*)h->der[c][3];
     }
-    in.dil = (const R*)h->dil;
     in.fx = h->fx;
     in.fx.gmax = h->gmax[c]; in.fx.gnext = h->gmax[1 - c];
     return in;
@@ -547,7 +547,7 @@ int cns_create(const cns_params* pin, int device, cns_solver** out) {
             h->cf64.c1S[d][k] = h->hg.c1S[d][k]; h->cf64.c1V[d][k] = h->hg.c1V[d][k]; h->cf64.c2V[d][k] = h->hg.c2V[d][k];
             h->cf32.c1S[d][k] = (float)h->hg.c1S[d][k]; h->cf32.c1V[d][k] = (float)h->hg.c1V[d][k];
             h->cf32.c2V[d][k] = (float)h->hg.c2V[d][k];
-            h->cf64.fq[d][k] = h->hg.fq[d][k]; h->cf64.fc[d][k] = h->hg.fc[d][k];
+            h->cf64.fc[d][k] = h->hg.fc[d][k];
             h->cf32.fq[d][k] = (float)h->hg.fq[d][k]; h->cf32.fc[d][k] = (float)h->hg.fc[d][k];
         }
     // lambda = mu / (Pr Ec)  (calcState, src/cuda_main.cu:218-242)
@@ -555,7 +555,6 @@ int cns_create(const cns_params* pin, int device, cns_solver** out) {
     h->cf32.lam_mu = (float)h->cf64.lam_mu;
     const double inv[3] = {h->hg.dx, h->hg.dy, h->hg.dz}, inv2[3] = {h->hg.d2x, h->hg.d2y, h->hg.d2z};
     for (int d = 0; d < 3; d++) {
-        h->cf64.inv[d] = inv[d]; h->cf64.inv2[d] = inv2[d];
         h->cf32.inv[d] = (float)inv[d]; h->cf32.inv2[d] = (float)inv2[d];
     }
     CK(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));

@@ -17,7 +17,7 @@ using namespace cns;
 namespace {
 
 constexpr int ST_X = 32, ST_R = 8;   // x-indices and row lanes of a block
-constexpr int ST_BLOCKS = 4 * 152;    // blocks of a plane sum (a few per SM: a row is a dependent step)
+constexpr int ST_BLOCKS = 4 * GB300_SMS;    // blocks of a plane sum (a few per SM: a row is a dependent step)
 
 // fixed-order sum of the row lanes' five values, valid in lane 0
 __device__ __forceinline__ void lane_sum(double (&s)[5]) {
