@@ -17,8 +17,8 @@
 // which is the same value with 2 instead of l(l+1) pair products per l. The product
 // (rho_a+rho_b)(g_a+g_b) is shared by the mass flux and the four cubic fluxes.
 //
-// FP64 and pair mode: the sums over the neighbours in 64-bit fixed point (kernels_fx.cuh), the
-// stage update and the recovery in FP64. FP32-RHS mode: rhs_point_packed on FP32 records.
+// FP64 and pair mode: the sums over the neighbours in 64-bit fixed point, or in FP64 where the
+// fields' ranges ask for it (kernels_fx.cuh), the stage update and the recovery in FP64. FP32-RHS mode: rhs_point_packed on FP32 records.
 #pragma once
 #include <algorithm>
 #include <cstdlib>
@@ -359,8 +359,9 @@ __device__ __forceinline__ void rhs_point(const Geom& g, const CoefT<R>& cf, con
 //
 // FP32: 7 blocks of 128 per SM (72 registers) measured fastest (6: 80 registers, +13 %
 // time; 5: 96 registers, and stages that read the RK register ran 3.5x slower). FP64: 4 blocks
-// (128 registers), bound by latency: issue 38 %, FP64 pipe 44 %, ~3,700 instructions per point;
-// on the channel 128x160x192 0.93 ms, with 3 blocks (168 registers) 1.11, 5 (96, spilling) 0.98.
+// (128 registers), bound by latency: issue 37 %, FP64 pipe 50 %, ~3,890 instructions per point,
+// 0.995 ms on the channel 128x160x192 (when that was 0.93 ms, before grad p and grad theta left the
+// integer sums, 3 blocks of 168 registers took 1.11, 5 of 96, spilling, 0.98).
 template <typename R, int S, int V>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 4) k_rhs(const __grid_constant__ Geom g,
                                                                      const __grid_constant__ CoefT<R> cf,
@@ -378,7 +379,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 4) k_rhs(const __gri
 // convective part of its 64 points (32 x 2, or 16 x 4 on a narrow box) and, with the viscous part that the other warps hand over
 // in shared memory, the stage update. 14^3 .. 28^3 boxes 14.3 .. 16.4 us against 16.4 .. 18.4; from
 // 32^3 (18.8 us against 18.4) on one thread per point is the faster, on the channel 128x160x192
-// 0.93 ms against 1.12.
+// 0.93 ms against 1.12 (measured before grad p and grad theta left the integer sums; a 16x20x24
+// box's kernel still takes 14.3 us).
 constexpr int SPLIT_POINTS = 64;
 template <int S, int V>
 __global__ void __launch_bounds__(2 * SPLIT_POINTS, 4) k_rhs_split(const __grid_constant__ Geom g,

@@ -64,7 +64,19 @@ extern "C" {
 #define CNS_RK4_CLASSIC    2   /* classic 4-stage RK4: no counterpart in the reference   */
 
 /* RHS arithmetic */
-#define CNS_PREC_FP64      0   /* plain FP64 everywhere, as the reference                */
+/*
+ * CNS_PREC_FP64: state, Runge-Kutta update, T/p recovery and reductions in FP64. The RHS's
+ * stencil sums run in 64-bit fixed point: a value is held to 2^-62 of the largest magnitude
+ * of its field in the box, ghosts included. Values of at least 2^-9 of it are exact; a velocity
+ * component below that loses bits, by less than what the rounding of the pressure there does.
+ * A stage whose fields do not suit this forms its sums in FP64, as the reference, at about a
+ * quarter of the speed: rho or T varying by more than three binades (a ratio of 8 to 16; T by
+ * less for viscexp above 2), rho |u|^2 above about 2^8 p, a field's largest magnitude outside
+ * 2^-300 .. 2^300, infinities, NaN. The kernels decide that from the fields; the
+ * relative error of the RHS is the plain FP64 sums' or less (relative to each equation's
+ * maximum; see the velocities above for regions almost at rest).
+ */
+#define CNS_PREC_FP64      0
 #define CNS_PREC_FP32_RHS  1   /* RHS in FP32; state, RK accumulation, T/p recovery and
                                   reductions in FP64                                     */
 #define CNS_PREC_PAIR_RHS  2   /* at least ~48-bit RHS arithmetic (FP32 pairs): served by the
