@@ -218,7 +218,8 @@ __device__ __forceinline__ void fx_column(const Geom& g, const FxBase& b, const 
         const int ck = c0 + k * PS;
         double q[5] = {0, 0, 0, 0, 0};
         if (inside) {
-            q[0] = __ldg(in.r + ck); q[1] = __ldg(in.t + ck); q[2] = __ldg(in.p + ck); q[3] = __ldg(in.h + ck); q[4] = __ldg(in.m + ck);
+            q[0] = __ldg(in.r + ck); q[1] = __ldg(in.t + ck); q[2] = __ldg(in.p + ck);
+            q[3] = __ldg(in.h + ck); q[4] = __ldg(in.m + ck);
         }
         const i64 cu = fx_from(nu, e[1]), cv = fx_from(nv, e[2]);
         ring[2 * V] = fx_from(nw, e[3]);

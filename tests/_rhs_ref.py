@@ -27,7 +27,8 @@ def rhs(p, f, T=np.longdouble):
     c1S, (c1V, c2V) = _weights(S, T)[0], _weights(V, T)
     at = lambda a, d, l: np.roll(a, -l, axis=2 - d)  # noqa: E731
     d1 = lambda a, d, c: sum(c[k] * (at(a, d, k) - at(a, d, -k)) for k in range(1, len(c))) * inv[d]  # noqa: E731
-    d2 = lambda a, d: (c2V[0] * a + sum(c2V[k] * (at(a, d, k) + at(a, d, -k)) for k in range(1, V + 1))) * inv[d] ** 2  # noqa: E731
+    d2 = lambda a, d: (c2V[0] * a + sum(c2V[k] * (at(a, d, k) + at(a, d, -k))  # noqa: E731
+                                        for k in range(1, V + 1))) * inv[d] ** 2
     U = [u, v, w]
     G = [[d1(U[c], d, c1V) for c in range(3)] for d in range(3)]
     th = G[0][0] + G[1][1] + G[2][2]
